@@ -14,6 +14,8 @@
 #include "hlbl_gb300.h"
 #include "hlbl_gb300_rng.h"
 #include "hlbl_internal.h"
+#include "p1_f64.h"
+#include "p2_f64.h"
 #include "p2_tc.h"
 #include "pieces_2p2.h"
 #include "qed_provider.cuh"
@@ -138,20 +140,20 @@ __global__ void f32_tile_copy_kernel(const double* __restrict__ blk, Geometry ge
 }
 
 // ---- launch plumbing -------------------------------------------------------
-template <typename T, int NF, int TS>
+template <int NF, int TS>
 struct P1Launch {
   static constexpr int threads = NF * 144;
-  static constexpr size_t smem = p1_smem_bytes<T, NF, TS>();
+  static constexpr size_t smem = p1_smem_bytes<NF, TS>();
   static int init(int nsm, int& grid) {
-    cudaError_t e = cudaFuncSetAttribute(p1_kernel<T, NF, TS>,
+    cudaError_t e = cudaFuncSetAttribute(p1_kernel<NF, TS>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     // all of the unified L1/shared storage as shared memory: two FP32 CTAs per SM
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(p1_kernel<T, NF, TS>, cudaFuncAttributePreferredSharedMemoryCarveout,
+      e = cudaFuncSetAttribute(p1_kernel<NF, TS>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return cuda_fail(e, "p1 smem attribute");
     int nb = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, p1_kernel<T, NF, TS>, threads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, p1_kernel<NF, TS>, threads, smem);
     if (e != cudaSuccess) return cuda_fail(e, "p1 occupancy");
     if (nb < 1) return fail(HLBL_ECUDA, "p1 kernel cannot be resident (smem %zu)", smem);
     grid = nb * nsm;
@@ -159,7 +161,7 @@ struct P1Launch {
   }
   static void launch(int grid, cudaStream_t st, const double* y, const PairBatch& b,
                      const Geometry& geo, int f0, double* partials, int* err, float* y32 = nullptr) {
-    p1_kernel<T, NF, TS><<<dim3(grid, b.n), threads, smem, st>>>(y, b, geo, f0, partials, err, y32);
+    p1_kernel<NF, TS><<<dim3(grid, b.n), threads, smem, st>>>(y, b, geo, f0, partials, err, y32);
   }
   static long long tiles(long long V) { return (V + TS - 1) / TS; }
 };
@@ -180,20 +182,18 @@ struct P2Launch {
     return HLBL_OK;
   }
   static void launch(int grid, cudaStream_t st, const double* y, const PairBatch& b,
-                     const Geometry& geo, const P2Args& a, const T* bt, double* partials, int* err) {
-    p2_kernel<T, NF, TS><<<dim3(grid, b.n), threads, smem, st>>>(y, b, geo, a, bt, partials, err);
+                     const Geometry& geo, const P2Args& a, const T* bt, double* partials, int* err,
+                     const int* only_if = nullptr) {
+    p2_kernel<T, NF, TS><<<dim3(grid, b.n), threads, smem, st>>>(y, b, geo, a, bt, partials, err, only_if);
   }
   static long long tiles(long long V) { return (V + TS - 1) / TS; }
 };
 
 // tile sizes per precision (the FP32 two-flavour kernels have a second tile
 // size each, which the autotuner may choose)
-using P1D2 = P1Launch<double, 2, 8>;
-using P1D1 = P1Launch<double, 1, 8>;
-using P1F2 = P1Launch<float, 2, 8>;
-using P1F2s = P1Launch<float, 2, 4>;
-using P1F1 = P1Launch<float, 1, 8>;
-using P2D2 = P2Launch<double, 2, 4>;
+using P1F2 = P1Launch<2, 8>;
+using P1F2s = P1Launch<2, 4>;
+using P1F1 = P1Launch<1, 8>;
 using P2D1 = P2Launch<double, 1, 4>;
 using P2F2 = P2Launch<float, 2, 4>;
 using P2F2s = P2Launch<float, 2, 2>;
@@ -229,8 +229,10 @@ struct hlbl_ctx {
   cudaStream_t stream = nullptr;
   Geometry geo{};
   hlbl_qed_params qp{};
-  int grid_p1d2 = 0, grid_p1d1 = 0, grid_p1f2 = 0, grid_p1f1 = 0, grid_p1f2s = 0;
-  int grid_p2d2 = 0, grid_p2d1 = 0, grid_p2f2 = 0, grid_p2f1 = 0, grid_p2f2s = 0;
+  int grid_p1d[2] = {};       // FP64 pass 1 (p1_f64.cu) for one and two flavours
+  int grid_p1f2 = 0, grid_p1f1 = 0, grid_p1f2s = 0;
+  int grid_p2d[2] = {};       // FP64 pass 2 (p2_f64.cu) for one and two flavours
+  int grid_p2d1 = 0, grid_p2f2 = 0, grid_p2f1 = 0, grid_p2f2s = 0;
   int p1_small = 0, p2_small = 0;  // FP32 tile variants chosen (autotuner)
   // FP32 two-flavour pass 2 on the tensor cores (p2_tc.cu); off: CUDA cores
   int tc = 1;
@@ -255,6 +257,8 @@ struct hlbl_ctx {
   double* d_dz = nullptr;     // [2][2880]
   double* d_g = nullptr;      // [2][11520]
   void* d_bt = nullptr;       // [2][288*160] of double (float uses half of it)
+  double* d_dzq = nullptr;    // FP64 pass 2: dz in block-diagonal form, [kMaxBatch][2][p2f64_dzq_len]
+  int* d_bad = nullptr;       // hlbl_cu_4pt_contraction: sums that are not the gamma images of one dz
   double* d_w = nullptr;      // QED weights [V][3][6]
   long long w_cap = 0;        // sites d_w holds
   // the QED kernel (hlbl_ctx_set_qed_kernel): the stand-in's closed form, or
@@ -345,7 +349,8 @@ float* x32_block(hlbl_ctx* c, const Geometry& geo, int slot) { return c->d_x32 +
 
 // Pass 1 + reduction + gamma insertion + Bt for the batch's pairs, flavours
 // [f0, f0+nf). Pair i, flavour fl: dz at d_dz + (i*nf + fl)*kDzLen, g at
-// d_g + (i*nf + fl)*kGLen, Bt at d_bt + (i*nf + fl)*kBtK*kBtN.
+// d_g + (i*nf + fl)*kGLen, Bt at d_bt + (i*nf + fl)*kBtK*kBtN. The FP64 pass 2
+// takes dz itself, as dzq (quat_basis.cuh), instead of g and Bt.
 int run_pass1(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch& b, int f0,
               int nf, int precision, double* add_dzu, double* add_dzsu, bool build_bt) {
   if (c->stage_pending) {  // blocks staged on the side stream must have landed
@@ -364,8 +369,8 @@ int run_pass1(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch
   }
   prof_begin(c, 0);
   if (precision == HLBL_FP64) {
-    if (nf == 2) { grid = per_pair_grid(c->grid_p1d2, b.n, P1D2::tiles(geo.V)); P1D2::launch(grid, c->stream, y, b, geo, f0, c->d_part1, c->d_err); }
-    else { grid = per_pair_grid(c->grid_p1d1, b.n, P1D1::tiles(geo.V)); P1D1::launch(grid, c->stream, y, b, geo, f0, c->d_part1, c->d_err); }
+    grid = per_pair_grid(c->grid_p1d[nf - 1], b.n, p1f64_tiles(geo.V));
+    p1f64_launch(nf, grid, c->stream, y, b, geo, f0, c->d_part1, c->d_err);
   } else {
     if (nf == 2 && c->p1_small) { grid = per_pair_grid(c->grid_p1f2s, b.n, P1F2s::tiles(geo.V)); P1F2s::launch(grid, c->stream, y, bb, geo, f0, c->d_part1, c->d_err, y32); }
     else if (nf == 2) { grid = per_pair_grid(c->grid_p1f2, b.n, P1F2::tiles(geo.V)); P1F2::launch(grid, c->stream, y, bb, geo, f0, c->d_part1, c->d_err, y32); }
@@ -375,13 +380,14 @@ int run_pass1(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch
   p1_reduce_kernel<<<dim3((kDzLen + kRedOut - 1) / kRedOut, nf, b.n), kRedOut * kRedGrp, 0, c->stream>>>(
       c->d_part1, grid, nf, c->d_dz, add_dzu, add_dzsu);
   if (!build_bt) return HLBL_OK;
+  if (precision == HLBL_FP64) {
+    p2f64_launch_dzq(c->d_dz, nullptr, nullptr, nf, b.n, c->d_dzq, nullptr, c->stream);
+    return HLBL_OK;
+  }
   g_build_kernel<<<dim3((kGLen / 2 + 255) / 256, nf, b.n), 256, 0, c->stream>>>(c->d_dz, nf, c->d_g);
   dim3 const gb((kBtK * kBtN + 255) / 256, nf, b.n);
   if (tcp)
     tc_launch_btu(c->d_g, b.n, c->d_btu, false, nullptr, c->stream);
-  else if (precision == HLBL_FP64)
-    bt_build_kernel<double><<<gb, 256, 0, c->stream>>>(c->d_g, c->d_g + kGDzuLen, kGLen,
-                                                       (size_t)nf * kGLen, nf, static_cast<double*>(c->d_bt));
   else
     bt_build_kernel<float><<<gb, 256, 0, c->stream>>>(c->d_g, c->d_g + kGDzuLen, kGLen,
                                                       (size_t)nf * kGLen, nf, static_cast<float*>(c->d_bt));
@@ -471,10 +477,11 @@ int run_qed(hlbl_ctx* c, const Geometry& geo, const PairBatch& b, double xunit, 
   return HLBL_OK;
 }
 
-// Pass 2 for the batch's pairs with Bt already built; pair i's sums go to
-// b.p[i].out[0..nf) (added if add).
+// Pass 2 for the batch's pairs with Bt (or dzq) already built; pair i's sums go to
+// b.p[i].out[0..nf) (added if add). bad: an FP64 flag on the device; where it is
+// set, the sums come from the general kernel with Bt instead of dzq.
 int run_pass2(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch& b, double xunit,
-              int f0, int nf, int precision, int add) {
+              int f0, int nf, int precision, int add, const int* bad = nullptr) {
   P2Args a{};
   if (int rc = run_qed(c, geo, b, xunit, precision, a)) return rc;
   a.xunit = xunit;
@@ -482,9 +489,10 @@ int run_pass2(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch
   int grid;
   prof_begin(c, 1);
   if (precision == HLBL_FP64) {
-    const double* bt = static_cast<const double*>(c->d_bt);
-    if (nf == 2) { grid = per_pair_grid(c->grid_p2d2, b.n, P2D2::tiles(geo.V)); P2D2::launch(grid, c->stream, y, b, geo, a, bt, c->d_part2, c->d_err); }
-    else { grid = per_pair_grid(c->grid_p2d1, b.n, P2D1::tiles(geo.V)); P2D1::launch(grid, c->stream, y, b, geo, a, bt, c->d_part2, c->d_err); }
+    grid = per_pair_grid(c->grid_p2d[nf - 1], b.n, p2f64_tiles(geo.V));
+    p2f64_launch(nf, grid, c->stream, y, b, geo, a, c->d_dzq, c->d_part2, c->d_err, bad);
+    if (bad != nullptr)  // the same partials, from the other kernel
+      P2D1::launch(grid, c->stream, y, b, geo, a, static_cast<const double*>(c->d_bt), c->d_part2, c->d_err, bad);
   } else if (use_tc(c, precision, nf)) {
     TcBatch tb{};
     tb.y32 = x32_block(c, geo, 0);
@@ -583,16 +591,16 @@ int hlbl_ctx_create(hlbl_ctx** out, const int global[4], const int local[4],
   e = cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return bail(cuda_fail(e, "SM count"));
   int rc;
-  if ((rc = P1D2::init(c->nsm, c->grid_p1d2)) || (rc = P1D1::init(c->nsm, c->grid_p1d1)) ||
+  if ((rc = p1f64_init(2, c->nsm, c->grid_p1d[1])) || (rc = p1f64_init(1, c->nsm, c->grid_p1d[0])) ||
       (rc = P1F2::init(c->nsm, c->grid_p1f2)) || (rc = P1F1::init(c->nsm, c->grid_p1f1)) ||
-      (rc = P2D2::init(c->nsm, c->grid_p2d2)) || (rc = P2D1::init(c->nsm, c->grid_p2d1)) ||
+      (rc = p2f64_init(c->nsm, c->grid_p2d)) || (rc = P2D1::init(c->nsm, c->grid_p2d1)) ||
       (rc = P2F2::init(c->nsm, c->grid_p2f2)) || (rc = P2F1::init(c->nsm, c->grid_p2f1)) ||
       (rc = P1F2s::init(c->nsm, c->grid_p1f2s)) || (rc = P2F2s::init(c->nsm, c->grid_p2f2s)) ||
       (rc = tc_init(c->nsm, c->grid_tc)) || (rc = p1f32_init(c->nsm, c->grid_p1f)) ||
       (rc = coef_init(c->nsm)))
     return bail(rc);
-  c->max_grid = std::max({c->grid_p1d2, c->grid_p1d1, c->grid_p1f2, c->grid_p1f1, c->grid_p2d2,
-                          c->grid_p2d1, c->grid_p2f2, c->grid_p2f1, c->grid_p1f2s, c->grid_p2f2s,
+  c->max_grid = std::max({c->grid_p1d[0], c->grid_p1d[1], c->grid_p1f2, c->grid_p1f1, c->grid_p2d[0],
+                          c->grid_p2d[1], c->grid_p2f2, c->grid_p2f1, c->grid_p1f2s, c->grid_p2f2s,
                           c->grid_tc, c->grid_p1f[0], c->grid_p1f[1], c->grid_p1f[2], c->grid_p1f[3]});
   e = cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->stage_ev, cudaEventDisableTiming);
@@ -610,6 +618,8 @@ int hlbl_ctx_create(hlbl_ctx** out, const int global[4], const int local[4],
       {(void**)&c->d_dz, sizeof(double) * kMaxBatch * 2 * kDzLen},
       {(void**)&c->d_g, sizeof(double) * kMaxBatch * 2 * kGLen},
       {(void**)&c->d_bt, sizeof(double) * kMaxBatch * 2 * kBtK * kBtN},
+      {(void**)&c->d_dzq, sizeof(double) * kMaxBatch * 2 * p2f64_dzq_len()},
+      {(void**)&c->d_bad, sizeof(int)},
       {(void**)&c->d_btu, sizeof(float) * kMaxBatch * tc_btu_floats_per_pair()},
       {(void**)&c->d_bscale, sizeof(float) * kMaxBatch * 2},
       {(void**)&c->d_out, sizeof(double) * 2},
@@ -635,6 +645,8 @@ void hlbl_ctx_destroy(hlbl_ctx* c) {
   cudaFree(c->d_dz);
   cudaFree(c->d_g);
   cudaFree(c->d_bt);
+  cudaFree(c->d_dzq);
+  cudaFree(c->d_bad);
   cudaFree(c->d_btu);
   cudaFree(c->d_bscale);
   cudaFree(c->d_x32);
@@ -908,10 +920,16 @@ int hlbl_cu_4pt_contraction(hlbl_ctx* c, double* d_ks, const double* d_g_dzu,
   if (!aligned16(src) || !aligned16(y)) return fail(HLBL_EINVAL, "hlbl_cu_4pt_contraction: blocks must be 16-byte aligned");
   Geometry geo{};
   if (int rc = make_geometry(global, local, pc, geo)) return rc;
+  // the sums are four gamma images of one dz (contract.cpp:58-77), from which
+  // the block-diagonal form is built; a caller may pass other numbers, which
+  // the build finds, and then the general form's kernel does the work
+  cudaError_t e = cudaMemsetAsync(c->d_bad, 0, sizeof(int), c->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "hlbl_cu_4pt_contraction");
+  p2f64_launch_dzq(nullptr, d_g_dzu, d_g_dzsu, 1, 1, c->d_dzq, c->d_bad, c->stream);
   bt_build_kernel<double><<<dim3((kBtK * kBtN + 255) / 256, 1, 1), 256, 0, c->stream>>>(
       d_g_dzu, d_g_dzsu, 0, 0, 1, static_cast<double*>(c->d_bt));
   PairBatch const b = one_pair(src, d_ks, gsx, yv);
-  if (int rc = run_pass2(c, geo, y, b, xunit, iflavor, 1, HLBL_FP64, 1)) return rc;
+  if (int rc = run_pass2(c, geo, y, b, xunit, iflavor, 1, HLBL_FP64, 1, c->d_bad)) return rc;
   return check_launch("hlbl_cu_4pt_contraction launch");
 }
 

@@ -114,13 +114,6 @@ __device__ __forceinline__ void load_row(const float* __restrict__ p, float r[24
     r[4 * i] = v.x; r[4 * i + 1] = v.y; r[4 * i + 2] = v.z; r[4 * i + 3] = v.w;
   }
 }
-__device__ __forceinline__ void load_row(const double* __restrict__ p, double r[24]) {
-#pragma unroll
-  for (int i = 0; i < 12; ++i) {
-    double2 const v = reinterpret_cast<const double2*>(p)[i];
-    r[2 * i] = v.x; r[2 * i + 1] = v.y;
-  }
-}
 
 
 // Pass 1's FP32 path: convert a landed FP64 stage into the FP32 compute copy
@@ -161,23 +154,24 @@ __device__ __forceinline__ void convert_and_copy(const double* __restrict__ st, 
 //   dzsu[s] += X_s,   dzu[k] += zh_rho(z) X_sigma - zh_sigma(z) X_rho.
 // X_s is assembled from the eight spin-block products
 //   P[s1][s2] = sum_c conj(B[s1][c]) A[s2][c],  s2 = src(s, s1),
-// which is all of g5 g_s's support. Per-site products in T, accumulated per
-// tile in T, then into FP64 per tile.
-// FP32 path: as it converts a tile, pass 1 also writes it into the FP32
-// tile copies the tensor-core pass 2 reads (y32 by pair 0's CTAs, each
+// which is all of g5 g_s's support. On FP64 blocks with FP32 products (the FP64
+// products are p1_f64.cu's), accumulated per tile in FP32, then into
+// compensated FP32 sums. As it converts a tile, pass 1 also writes it into the
+// FP32 tile copies the tensor-core pass 2 reads (y32 by pair 0's CTAs, each
 // partner's by its own; null pointers: no copy).
-template <typename T, int NF, int TS>
-__global__ void __launch_bounds__(NF * 144, sizeof(T) == sizeof(float) ? 2 : 1)
+template <int NF, int TS>
+__global__ void __launch_bounds__(NF * 144, 2)
 p1_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0,
           double* __restrict__ partials, int* __restrict__ err, float* __restrict__ y32) {
   constexpr int kRows = 2 * NF * 12;
-  constexpr size_t kStage = (size_t)kRows * TS * 24;  // doubles per stage
+  using T = float;
+  constexpr size_t kStage = (size_t)kRows * TS * 24;  // doubles of the stage
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  double* s_stage = reinterpret_cast<double*>(smem_raw);         // [2][kRows][TS][24]
+  double* s_stage = reinterpret_cast<double*>(smem_raw);         // [kRows][TS][24]
   // zerohalf weights of the tile's sites, converted once (a per-thread
   // int -> float conversion issues on GB300's slow FP64/conversion pipe)
   T* s_zh = reinterpret_cast<T*>(smem_raw + stage_bytes<T, NF, TS>());  // [TS][4]
-  __shared__ __align__(8) uint64_t s_bar[2];
+  __shared__ __align__(8) uint64_t s_bar;
   __shared__ int s_fail;
 
   int const pi = blockIdx.y;
@@ -187,11 +181,8 @@ p1_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0,
   int const fl = t / 144, ia = (t % 144) / 12, ib = t % 12;
 
   // Per-thread sums over this CTA's tiles, each tile's sum added in:
-  // compensated FP64 on the FP64 path, compensated FP32 (Kahan) on the FP32
-  // path, converted to FP64 at the end.
-  constexpr bool kComp = sizeof(T) == sizeof(double);
-  using Acc = typename std::conditional<kComp, Neu, KahanF>::type;
-  Acc acc_u[6][2], acc_s[4][2];
+  // compensated FP32 (Kahan), converted to FP64 at the end.
+  KahanF acc_u[6][2], acc_s[4][2];
   T tu[6][2], ts[4][2];
 #pragma unroll
   for (int k = 0; k < 6; ++k) tu[k][0] = tu[k][1] = T(0);
@@ -214,11 +205,9 @@ p1_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0,
       }
   };
 
-  constexpr bool kDB = sizeof(T) == sizeof(double);  // double-buffered FP64 stages
-  float* s_copy = reinterpret_cast<float*>(s_stage + kStage);  // FP32 mode: the converted tile
+  float* s_copy = reinterpret_cast<float*>(s_stage + kStage);  // the converted tile
   if (t == 0) {
-    mbar_init(&s_bar[0], 1);
-    mbar_init(&s_bar[1], 1);
+    mbar_init(&s_bar, 1);
     fence_mbar_init();
     s_fail = 0;
   }
@@ -226,61 +215,38 @@ p1_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0,
   long long const ntiles = (geo.V + TS - 1) / TS;
   long long tile = blockIdx.x;
   // src flavour f0+fl, y flavour 1-(f0+fl)
-  if (t == 0 && tile < ntiles) issue_tile<NF, TS>(s_stage, &s_bar[0], src, y, f0, 1, 1 - f0, -1, geo.V, tile * TS);
-  bool next_in_flight = false;
-  int i = 0;
-  for (; tile < ntiles; ++i, tile += gridDim.x) {
-    int const st = kDB ? (i & 1) : 0;
+  if (t == 0 && tile < ntiles) issue_tile<NF, TS>(s_stage, &s_bar, src, y, f0, 1, 1 - f0, -1, geo.V, tile * TS);
+  uint32_t parity = 0;
+  for (; tile < ntiles; parity ^= 1u, tile += gridDim.x) {
     long long const s0 = tile * TS;
     int const nvalid = (int)min((long long)TS, geo.V - s0);
-    next_in_flight = tile + gridDim.x < ntiles;
-    // FP64: prefetch into the other stage (its readers passed the last barrier)
-    if (kDB && t == 0 && next_in_flight) {
-      fence_proxy_async_smem();
-      issue_tile<NF, TS>(s_stage + (st ^ 1) * kStage, &s_bar[st ^ 1], src, y, f0, 1, 1 - f0, -1,
-                         geo.V, (tile + gridDim.x) * TS);
-    }
     for (int s = t; s < TS; s += blockDim.x) {
       int rel[4];
       rel_coords_fast(geo, gsx, min(s0 + s, geo.V - 1), rel);
 #pragma unroll
       for (int r = 0; r < 4; ++r) s_zh[s * 4 + r] = (T)coord_map_zerohalf(rel[r], geo.global[r]);
     }
-    uint32_t const parity = kDB ? (uint32_t)((i >> 1) & 1) : (uint32_t)(i & 1);
-    if (!mbar_wait(&s_bar[st], parity)) s_fail = 1;
+    if (!mbar_wait(&s_bar, parity)) s_fail = 1;
     __syncthreads();
     if (s_fail) break;
-    const T* tile_data;
-    if constexpr (kDB) {
-      tile_data = reinterpret_cast<const T*>(s_stage + st * kStage);
-    } else {
-      // FP32: convert once, then the stage takes the next tile while we compute
-      convert_and_copy<NF, TS>(s_stage, s_copy, batch.p[pi].src32, pi == 0 ? y32 : nullptr, f0, geo.V, s0,
-                               nvalid);
-      __syncthreads();
-      if (t == 0 && next_in_flight) {
-        fence_proxy_async_smem();
-        issue_tile<NF, TS>(s_stage, &s_bar[0], src, y, f0, 1, 1 - f0, -1, geo.V, (tile + gridDim.x) * TS);
-      }
-      tile_data = reinterpret_cast<const T*>(s_copy);
+    // convert once, then the stage takes the next tile while we compute
+    convert_and_copy<NF, TS>(s_stage, s_copy, batch.p[pi].src32, pi == 0 ? y32 : nullptr, f0, geo.V, s0, nvalid);
+    __syncthreads();
+    if (t == 0 && tile + gridDim.x < ntiles) {
+      fence_proxy_async_smem();
+      issue_tile<NF, TS>(s_stage, &s_bar, src, y, f0, 1, 1 - f0, -1, geo.V, (tile + gridDim.x) * TS);
     }
+    const T* tile_data = s_copy;
 
     constexpr int RS = row_stride<T, TS>();
     const T* A_base = tile_data + ((size_t)(0 * NF + fl) * 12 + ia) * RS;
     const T* B_base = tile_data + ((size_t)(1 * NF + fl) * 12 + ib) * RS;
 #pragma unroll 1
     for (int s = 0; s < nvalid; ++s) {
-      // FP32: the site's rows into registers with 16-byte loads; FP64: read
-      // in place (two rows of doubles would crowd the registers)
-      T Ar[24], Br[24];
-      const T* A = A_base + s * 24;
-      const T* B = B_base + s * 24;
-      if constexpr (sizeof(T) == sizeof(float)) {
-        load_row(A, Ar);
-        load_row(B, Br);
-        A = Ar;
-        B = Br;
-      }
+      // the site's rows into registers with 16-byte loads
+      T A[24], B[24];
+      load_row(A_base + s * 24, A);
+      load_row(B_base + s * 24, B);
       // P[s1][s2] for s2 = s1^2 (gamma_0, gamma_3) and s2 = 3-s1 (gamma_1, gamma_2)
       T pa[4][2], pb[4][2];
 #pragma unroll
@@ -326,12 +292,8 @@ p1_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0,
   }
   flush();
   if (s_fail) {
-    // a wait gave up: report it, and let no copy into this CTA's shared
-    // memory outlive it (bounded, as everything else)
-    if (t == 0) {
-      if (err) atomicExch(err, kErrWaitTimeout);
-      if (kDB && next_in_flight) mbar_wait(&s_bar[(i + 1) & 1], (uint32_t)(((i + 1) >> 1) & 1));
-    }
+    // a wait gave up: report it
+    if (t == 0 && err) atomicExch(err, kErrWaitTimeout);
     return;
   }
 
@@ -682,23 +644,18 @@ constexpr size_t p2_smem_bytes() {
          + sizeof(T) * (size_t)(TS * 3 * kQ);                            // tensor inputs
 }
 
-template <typename T, int NF, int TS>
+template <int NF, int TS>
 constexpr size_t p1_smem_bytes() {
-  return stage_bytes<T, NF, TS>() + sizeof(T) * TS * 4;
+  return stage_bytes<float, NF, TS>() + sizeof(float) * TS * 4;
 }
 
-// The pass-1 variant of hlbl_cu_dzu_dzsu_noalloc: one flavour, FP64, the
-// same tile as the context's FP64 pass 1.
-struct P1NoAllocTraits {
-  static constexpr int kTS = 8;
-  static constexpr int kThreads = 144;
-  static constexpr size_t kSmem = p1_smem_bytes<double, 1, kTS>();
-};
-
+// only_if: return at once unless *only_if is set (null: run).
 template <typename T, int NF, int TS>
 __global__ void __launch_bounds__(NF * 160)
 p2_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, P2Args args,
-          const T* __restrict__ bt_all, double* __restrict__ partials, int* __restrict__ err) {
+          const T* __restrict__ bt_all, double* __restrict__ partials, int* __restrict__ err,
+          const int* __restrict__ only_if) {
+  if (only_if != nullptr && *only_if == 0) return;
   constexpr int kRows = 2 * NF * 12;
   constexpr size_t kStage = (size_t)kRows * TS * 24;  // doubles per input stage
   extern __shared__ __align__(128) unsigned char smem_raw[];

@@ -16,10 +16,9 @@
 #include "contract_kernels.cuh"
 #include "hlbl_gb300.h"
 #include "hlbl_internal.h"
+#include "p1_f64.h"
 
 namespace {
-
-using Kernel = hg::P1NoAllocTraits;
 
 // One 2,880-double slot of partial sums per thread block, for at most
 // HLBL_NOALLOC_MAX_BLOCKS blocks: 512 x 2880 x 8 B = 11.8 MB. Pass 1 strides
@@ -65,22 +64,12 @@ int setup(int dev, double** addr, int** err, int* resident) {
     if (e != cudaSuccess) return hg::cuda_fail(e, "noalloc: cudaGetSymbolAddress(partials)");
     e = cudaGetSymbolAddress(&q, g_err);
     if (e != cudaSuccess) return hg::cuda_fail(e, "noalloc: cudaGetSymbolAddress(error word)");
-    e = cudaFuncSetAttribute(hg::p1_kernel<double, 1, Kernel::kTS>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Kernel::kSmem);
-    // the same carveout as the context's pass 1, so the occupancy is the same
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(hg::p1_kernel<double, 1, Kernel::kTS>,
-                               cudaFuncAttributePreferredSharedMemoryCarveout,
-                               cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return hg::cuda_fail(e, "noalloc: smem attribute");
-    int nb = 0, nsm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, hg::p1_kernel<double, 1, Kernel::kTS>,
-                                                      Kernel::kThreads, Kernel::kSmem);
-    if (e != cudaSuccess) return hg::cuda_fail(e, "noalloc: occupancy");
-    if (nb < 1) return hg::fail(HLBL_ECUDA, "noalloc: pass 1 cannot be resident (smem %zu)", Kernel::kSmem);
+    // the context's pass 1 of one flavour, at its occupancy
+    int nsm = 0, resident_blocks = 0;
     e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return hg::cuda_fail(e, "noalloc: SM count");
-    g_resident[dev] = nb * nsm;
+    if (int rc = hg::p1f64_init(1, nsm, resident_blocks)) return rc;
+    g_resident[dev] = resident_blocks;
     g_err_addr[dev] = static_cast<int*>(q);
     g_partials_addr[dev] = static_cast<double*>(p);
   }
@@ -123,7 +112,7 @@ extern "C" int hlbl_cu_dzu_dzsu_noalloc(double* d_dzu, double* d_dzsu, const dou
   if (int rc = setup(dev, &partials, &err, &resident)) return rc;
   // pass 1 strides over the tiles: any grid of at least one block gives the
   // same sums, so the grid is capped at the scratch's slots
-  long long const tiles = (V + Kernel::kTS - 1) / Kernel::kTS;
+  long long const tiles = hg::p1f64_tiles(V);
   long long nb = tiles < resident ? tiles : resident;
   if (nb > HLBL_NOALLOC_MAX_BLOCKS) nb = HLBL_NOALLOC_MAX_BLOCKS;
   int const nblocks = (int)nb;
@@ -136,8 +125,7 @@ extern "C" int hlbl_cu_dzu_dzsu_noalloc(double* d_dzu, double* d_dzsu, const dou
   b.n = 1;
   b.p[0].src = fwd_src;
   for (int r = 0; r < 4; ++r) b.p[0].gsx[r] = gsx[r];
-  hg::p1_kernel<double, 1, Kernel::kTS><<<dim3(nblocks, 1), Kernel::kThreads, Kernel::kSmem, st>>>(
-      fwd_y, b, geo, iflavor, partials, err, nullptr);
+  hg::p1f64_launch(1, nblocks, st, fwd_y, b, geo, iflavor, partials, err);
   noalloc_reduce_kernel<<<(hg::kDzLen + 255) / 256, 256, 0, st>>>(partials, nblocks, err, d_dzu, d_dzsu);
   e = cudaGetLastError();
   if (e != cudaSuccess) return hg::cuda_fail(e, "hlbl_cu_dzu_dzsu_noalloc launch");
