@@ -261,6 +261,8 @@ struct hlbl_ctx {
   int* d_bad = nullptr;       // hlbl_cu_4pt_contraction: sums that are not the gamma images of one dz
   double* d_w = nullptr;      // QED weights [V][3][6]
   long long w_cap = 0;        // sites d_w holds
+  unsigned* d_near = nullptr;    // evaluations near the origin (qed_weights_near_kernel), 3 per site of w_cap
+  unsigned* d_near_n = nullptr;  // their counts per pair, and the CTAs done [kMaxBatch + 1]
   // the QED kernel (hlbl_ctx_set_qed_kernel): the stand-in's closed form, or
   // a provider through the generic coefficient path
   int qed_kind = kQedStandInClosed;
@@ -384,28 +386,37 @@ int run_pass1(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch
     p2f64_launch_dzq(c->d_dz, nullptr, nullptr, nf, b.n, c->d_dzq, nullptr, c->stream);
     return HLBL_OK;
   }
+  if (tcp) {
+    tc_launch_btu(c->d_dz, b.n, c->d_btu, false, nullptr, c->stream);
+    return HLBL_OK;
+  }
   g_build_kernel<<<dim3((kGLen / 2 + 255) / 256, nf, b.n), 256, 0, c->stream>>>(c->d_dz, nf, c->d_g);
   dim3 const gb((kBtK * kBtN + 255) / 256, nf, b.n);
-  if (tcp)
-    tc_launch_btu(c->d_g, b.n, c->d_btu, false, nullptr, c->stream);
-  else
-    bt_build_kernel<float><<<gb, 256, 0, c->stream>>>(c->d_g, c->d_g + kGDzuLen, kGLen,
-                                                      (size_t)nf * kGLen, nf, static_cast<float*>(c->d_bt));
+  bt_build_kernel<float><<<gb, 256, 0, c->stream>>>(c->d_g, c->d_g + kGDzuLen, kGLen,
+                                                (size_t)nf * kGLen, nf, static_cast<float*>(c->d_bt));
+  return HLBL_OK;
+}
+
+// The QED weight buffers for `need` sites over all pairs of a launch.
+int ensure_weights(hlbl_ctx* c, long long need) {
+  if (need <= c->w_cap) return HLBL_OK;
+  if (c->capturing) return fail(HLBL_ESTATE, "QED weight buffer too small during graph capture");
+  cudaStreamSynchronize(c->stream);
+  cudaFree(c->d_w);
+  cudaFree(c->d_near);
+  c->d_w = nullptr;
+  c->d_near = nullptr;
+  c->w_cap = 0;
+  cudaError_t e = cudaMalloc(&c->d_w, sizeof(double) * 3 * HLBL_QED_NW * (size_t)need);
+  if (e == cudaSuccess) e = cudaMalloc(&c->d_near, sizeof(unsigned) * 3 * (size_t)need);
+  if (e != cudaSuccess) return fail(HLBL_ENOMEM, "QED weight buffer: %s", cudaGetErrorString(e));
+  c->w_cap = need;
   return HLBL_OK;
 }
 
 // The QED weights of the batch's pairs into d_w ([pair][V][3][6]).
 int run_weights(hlbl_ctx* c, const Geometry& geo, const PairBatch& b, double xunit, int precision) {
-  long long const need = geo.V * b.n;
-  if (need > c->w_cap) {
-    if (c->capturing) return fail(HLBL_ESTATE, "QED weight buffer too small during graph capture");
-    cudaFree(c->d_w);
-    c->d_w = nullptr;
-    c->w_cap = 0;
-    cudaError_t e = cudaMalloc(&c->d_w, sizeof(double) * 3 * HLBL_QED_NW * (size_t)need);
-    if (e != cudaSuccess) return fail(HLBL_ENOMEM, "QED weight buffer: %s", cudaGetErrorString(e));
-    c->w_cap = need;
-  }
+  if (int rc = ensure_weights(c, geo.V * b.n)) return rc;
   WArgs wa{};
   wa.batch = b;
   wa.xunit = xunit;
@@ -417,10 +428,13 @@ int run_weights(hlbl_ctx* c, const Geometry& geo, const PairBatch& b, double xun
   int const blocks = (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, (long long)c->nsm * 16 / b.n));
   if (precision == HLBL_FP32 && c->qed_fp32) {
     // one thread per site (its three evaluations)
-    int const bs = (int)std::max<long long>(1, std::min<long long>((geo.V + 255) / 256, (long long)c->nsm * 16 / b.n));
-    qed_weights_fp32_kernel<<<dim3(bs, b.n), 256, 0, c->stream>>>(geo, wa, c->qed_r64, c->qf, c->d_w);
+    int const bs = (int)std::max<long long>(
+        1, std::min<long long>((geo.V + kWThreads - 1) / kWThreads, (long long)c->nsm * 32 / b.n));
+    qed_weights_fp32_kernel<<<dim3(bs, b.n), kWThreads, 0, c->stream>>>(geo, wa, c->qed_r64, c->qf, c->d_w, c->d_near, c->d_near_n);
+    int const bn = std::min(bs, std::max(1, c->nsm / b.n));  // a CTA per SM: eight evaluations at once each
+    qed_weights_near_kernel<<<dim3(bn, b.n), kWThreads, 0, c->stream>>>(geo, wa, c->qf, c->d_w, c->d_near, c->d_near_n);
   } else {
-    qed_weights_exact_kernel<<<dim3(blocks, b.n), 256, 0, c->stream>>>(geo, wa, c->d_w);
+    qed_weights_exact_kernel<<<dim3(blocks, b.n), 256, 0, c->stream>>>(geo, wa, c->qf, c->d_w);
   }
   return HLBL_OK;
 }
@@ -530,8 +544,7 @@ int run_group_f32(hlbl_ctx* c, const PairBatch& b, const TcBatch& tb, double xun
   prof_end(c, 0);
   p1_reduce_kernel<<<dim3((kDzLen + kRedOut - 1) / kRedOut, 2, b.n), kRedOut * kRedGrp, 0, c->stream>>>(c->d_part1, g1, 2, c->d_dz,
                                                                              nullptr, nullptr);
-  g_build_kernel<<<dim3((kGLen / 2 + 255) / 256, 2, b.n), 256, 0, c->stream>>>(c->d_dz, 2, c->d_g);
-  tc_launch_btu(c->d_g, b.n, c->d_btu, c->tc16 != 0, c->d_bscale, c->stream);
+  tc_launch_btu(c->d_dz, b.n, c->d_btu, c->tc16 != 0, c->d_bscale, c->stream);
   P2Args a{};
   if (int rc = run_qed(c, geo, b, xunit, HLBL_FP32, a)) return rc;
   a.xunit = xunit;
@@ -620,6 +633,7 @@ int hlbl_ctx_create(hlbl_ctx** out, const int global[4], const int local[4],
       {(void**)&c->d_bt, sizeof(double) * kMaxBatch * 2 * kBtK * kBtN},
       {(void**)&c->d_dzq, sizeof(double) * kMaxBatch * 2 * p2f64_dzq_len()},
       {(void**)&c->d_bad, sizeof(int)},
+      {(void**)&c->d_near_n, sizeof(unsigned) * (kMaxBatch + 1)},
       {(void**)&c->d_btu, sizeof(float) * kMaxBatch * tc_btu_floats_per_pair()},
       {(void**)&c->d_bscale, sizeof(float) * kMaxBatch * 2},
       {(void**)&c->d_out, sizeof(double) * 2},
@@ -629,6 +643,7 @@ int hlbl_ctx_create(hlbl_ctx** out, const int global[4], const int local[4],
     if (e != cudaSuccess) return bail(fail(HLBL_ENOMEM, "cudaMalloc %zu bytes: %s", b.n, cudaGetErrorString(e)));
   }
   e = cudaMemset(c->d_err, 0, sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(c->d_near_n, 0, sizeof(unsigned) * (kMaxBatch + 1));
   if (e != cudaSuccess) return bail(cuda_fail(e, "error flag"));
   e = cudaMallocHost(reinterpret_cast<void**>(&c->h_out), sizeof(double) * 2);
   if (e != cudaSuccess) return bail(fail(HLBL_ENOMEM, "cudaMallocHost: %s", cudaGetErrorString(e)));
@@ -653,6 +668,8 @@ void hlbl_ctx_destroy(hlbl_ctx* c) {
   cudaFree(c->d_out);
   cudaFree(c->d_err);
   cudaFree(c->d_w);
+  cudaFree(c->d_near);
+  cudaFree(c->d_near_n);
   cudaFree(c->d_coef);
   cudaFree(c->d_dense64);
   cudaFree(c->d_dense32);
@@ -1086,16 +1103,7 @@ int hlbl_ctx_reserve(hlbl_ctx* c, int max_pairs) {
     return ensure_coef(c, std::max(coef_bytes(c->geo, std::min(max_pairs, g64), false),
                                    coef_bytes(c->geo, std::min(max_pairs, g32), true)));
   }
-  long long const need = c->geo.V * std::min(max_pairs, kMaxBatch);
-  if (need <= c->w_cap) return HLBL_OK;
-  cudaStreamSynchronize(c->stream);
-  cudaFree(c->d_w);
-  c->d_w = nullptr;
-  c->w_cap = 0;
-  cudaError_t e = cudaMalloc(&c->d_w, sizeof(double) * 3 * HLBL_QED_NW * (size_t)need);
-  if (e != cudaSuccess) return fail(HLBL_ENOMEM, "QED weight buffer: %s", cudaGetErrorString(e));
-  c->w_cap = need;
-  return HLBL_OK;
+  return ensure_weights(c, c->geo.V * std::min(max_pairs, kMaxBatch));
 }
 
 int hlbl_stage_async(hlbl_ctx* c, void* d_dst, const void* h_src, size_t bytes, int after_compute) {

@@ -41,12 +41,17 @@ struct PairBatch {
   PairDesc p[kMaxBatch];
 };
 
-// Neumaier's compensated FP64 sum: the site-block and volume sums.
+// Neumaier's compensated FP64 sum: the site-block and volume sums. The larger
+// of the two in magnitude is chosen by comparing their bits as integers (as
+// numbers, on the FP64 pipe, the comparison and both forms of the error cost
+// seven of that pipe's instructions instead of four).
 struct Neu {
   double s = 0.0, c = 0.0;
   __device__ __forceinline__ void add(double v) {
-    double const t = s + v;
-    c += fabs(s) >= fabs(v) ? (s - t) + v : (v - t) + s;
+    unsigned long long const m = 0x7FFFFFFFFFFFFFFFull;
+    bool const big = ((unsigned long long)__double_as_longlong(s) & m) >= ((unsigned long long)__double_as_longlong(v) & m);
+    double const t = s + v, a = big ? s : v, b = big ? v : s;
+    c += (a - t) + b;
     s = t;
   }
   __device__ __forceinline__ double get() const { return s + c; }
@@ -313,10 +318,11 @@ p1_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0,
 // Fixed-order, compensated (Neumaier) FP64 sum over the CTAs' partials.
 // dz[fl][i] = sum_cta partials[cta][fl][i]; if add_to != null also
 // add_to[fl][i] += dz (the reference's accumulate-into-caller semantics).
-// A CTA takes 32 outputs; its 8 warps each sum every 8th CTA's partials
-// (compensated), then one warp adds the 8 partial sums in order: 8x the
-// warps of one thread per output, each with an eighth of the chain.
-constexpr int kRedOut = 32, kRedGrp = 8;
+// A CTA takes 16 outputs (180 CTAs per flavour and pair, so that they spread
+// evenly over the SMs: the kernel is bound by the FP64 pipe, 5760 compensated
+// additions per partial); its 16 half warps each sum every 16th CTA's partials
+// (four loads in flight), then a tree adds the 16 sums.
+constexpr int kRedOut = 16, kRedGrp = 16;
 static __global__ void __launch_bounds__(kRedOut * kRedGrp)
     p1_reduce_kernel(const double* __restrict__ partials, int ncta, int nf, double* __restrict__ dz,
                      double* add_dzu, double* add_dzsu) {
@@ -325,29 +331,34 @@ static __global__ void __launch_bounds__(kRedOut * kRedGrp)
   int const i = blockIdx.x * kRedOut + o;
   __shared__ double rs[kRedGrp][kRedOut], rc[kRedGrp][kRedOut];
   partials += (size_t)pi * ncta * nf * kDzLen;
-  double s = 0.0, c = 0.0;
+  Neu a;
   if (i < kDzLen && fl < nf) {
-    for (int b = grp; b < ncta; b += kRedGrp) {
-      double const v = partials[((size_t)b * nf + fl) * kDzLen + i];
-      double const tt = s + v;
-      c += fabs(s) >= fabs(v) ? (s - tt) + v : (v - tt) + s;
-      s = tt;
+    const double* p = partials + (size_t)fl * kDzLen + i;
+    size_t const step = (size_t)nf * kDzLen;
+    int b = grp;
+    for (; b + 3 * kRedGrp < ncta; b += 4 * kRedGrp) {
+      double v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = p[(size_t)(b + u * kRedGrp) * step];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) a.add(v[u]);
+    }
+    for (; b < ncta; b += kRedGrp) a.add(p[(size_t)b * step]);
+  }
+#pragma unroll
+  for (int h = kRedGrp / 2; h > 0; h >>= 1) {
+    if (grp >= h && grp < 2 * h) {
+      rs[grp][o] = a.s;
+      rc[grp][o] = a.c;
+    }
+    __syncthreads();
+    if (grp < h) {
+      a.add(rs[grp + h][o]);
+      a.c += rc[grp + h][o];
     }
   }
-  rs[grp][o] = s;
-  rc[grp][o] = c;
-  __syncthreads();
   if (grp != 0 || i >= kDzLen || fl >= nf) return;
-  s = 0.0;
-  c = 0.0;
-  for (int g = 0; g < kRedGrp; ++g) {
-    c += rc[g][o];
-    double const v = rs[g][o];
-    double const tt = s + v;
-    c += fabs(s) >= fabs(v) ? (s - tt) + v : (v - tt) + s;
-    s = tt;
-  }
-  s += c;
+  double const s = a.get();
   dz += (size_t)pi * nf * kDzLen;
   dz[fl * kDzLen + i] = s;
   if (add_dzu != nullptr) {
@@ -501,7 +512,7 @@ __device__ __forceinline__ void qed_args(const Geometry& geo, const int gsx[4], 
   }
 }
 
-static __global__ void qed_weights_exact_kernel(Geometry geo, WArgs args, double* __restrict__ w) {
+static __global__ void qed_weights_exact_kernel(Geometry geo, WArgs args, QedF32 qf, double* __restrict__ w) {
   long long const n = geo.V * 3;
   int const pi = blockIdx.y;
   int const gsx[4] = {args.batch.p[pi].gsx[0], args.batch.p[pi].gsx[1], args.batch.p[pi].gsx[2], args.batch.p[pi].gsx[3]};
@@ -512,7 +523,7 @@ static __global__ void qed_weights_exact_kernel(Geometry geo, WArgs args, double
     double a[4], b[4], X, c, Y, ww[HLBL_QED_NW];
     qed_args(geo, gsx, yv, args.xunit, i / 3, (int)(i % 3), a, b);
     hlbl_qed_invariants(a, b, &X, &c, &Y);
-    hlbl_qed_weights(&args.qp, X, c, Y, ww);
+    qed_weights_fp64(args.qp, qf, X, c, Y, ww);
 #pragma unroll
     for (int j = 0; j < HLBL_QED_NW; ++j) w[i * HLBL_QED_NW + j] = ww[j];
   }
@@ -523,15 +534,52 @@ static __global__ void qed_weights_exact_kernel(Geometry geo, WArgs args, double
 // FP32 keeps a few 1e-7 relative accuracy; qed_f32.cuh), in FP64 inside that
 // radius (near the origin) -- the FP64 QED evaluation is kept only there.
 // One thread per site: its three evaluations share the site's coordinates
-// (32-bit integer arithmetic, V < 2^31); the quadrature is FP32; the FP64
-// evaluations near the origin are shared by the warp (one node per lane)
-// instead of run by single lanes.
-static __global__ void qed_weights_fp32_kernel(Geometry geo, WArgs args, double r64, QedF32 qf,
-                                               double* __restrict__ w) {
+// (32-bit integer arithmetic, 3 V < 2^32); the quadrature is FP32. The FP64
+// evaluations near the origin are only listed (near: 3 V places per pair, the
+// pair's count in near_n), and qed_weights_near_kernel takes the list, half a
+// warp per evaluation, over all SMs: the sites near the origin are a few
+// neighbours (65 within 0.1/m_mu at a = 0.1 fm), whose FP64 chains held a
+// handful of warps, and with them the kernel, for 185 us (8192 sites x 4 pairs;
+// 56 us with a CTA's warps sharing its sites). Measured, both kernels: 185 -> 37
+// us there, 131 -> 104 us per pair at 663,552 sites.
+constexpr int kWThreads = 128;
+struct SiteArgs {  // the integer vectors of one site's three evaluations, as sums
+  int nx, nxy, dxy, dxx;
+};
+__device__ __forceinline__ SiteArgs site_args(const Geometry& geo, const int gsx[4], const int yv[4], const int iy[4],
+                                              unsigned site) {
+  unsigned s = site;
+  int c[4];
+  c[3] = (int)(s % (unsigned)geo.local[3]); s /= (unsigned)geo.local[3];
+  c[2] = (int)(s % (unsigned)geo.local[2]); s /= (unsigned)geo.local[2];
+  c[1] = (int)(s % (unsigned)geo.local[1]); s /= (unsigned)geo.local[1];
+  c[0] = (int)s;
+  // the arguments are small integer vectors times xunit: |a|^2, |b|^2 and
+  // a.b are exact integer sums (times xunit^2), so |a|, |b| and cos(a, b)
+  // come out of correctly rounded FP32 square roots and one division
+  // (within 1.5 ulp; the FP64 weight gets the same invariants in FP64)
+  SiteArgs q{0, 0, 0, 0};
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    int const G = geo.global[r];
+    int const rel = (c[r] + geo.pc[r] * geo.local[r] - gsx[r] + G) % G;
+    int const ix = coord_map(rel, G), ixy = coord_map_diff(rel, yv[r], G);
+    q.nx += ix * ix;
+    q.nxy += ixy * ixy;
+    q.dxy += ix * iy[r];
+    q.dxx += ix * ixy;
+  }
+  return q;
+}
+
+static __global__ void __launch_bounds__(kWThreads)
+qed_weights_fp32_kernel(Geometry geo, WArgs args, double r64, QedF32 qf, double* __restrict__ w,
+                        unsigned* __restrict__ near, unsigned* __restrict__ near_n) {
   int const pi = blockIdx.y;
   int const gsx[4] = {args.batch.p[pi].gsx[0], args.batch.p[pi].gsx[1], args.batch.p[pi].gsx[2], args.batch.p[pi].gsx[3]};
   int const yv[4] = {args.batch.p[pi].yv[0], args.batch.p[pi].yv[1], args.batch.p[pi].yv[2], args.batch.p[pi].yv[3]};
   w += (size_t)pi * geo.V * 3 * HLBL_QED_NW;
+  near += (size_t)pi * geo.V * 3;
   unsigned const V = (unsigned)geo.V, stride = gridDim.x * blockDim.x;
   float const xuf = (float)args.xunit, r64f = (float)r64;
   int iy[4], ny = 0;
@@ -540,69 +588,75 @@ static __global__ void qed_weights_fp32_kernel(Geometry geo, WArgs args, double 
     iy[r] = coord_map(mod_pos(yv[r], geo.global[r]), geo.global[r]);
     ny += iy[r] * iy[r];
   }
-  // every lane runs every iteration (the near-origin evaluations are shared
-  // by the warp); lanes past the end compute on the last site and store nothing
-  for (unsigned base = blockIdx.x * blockDim.x; base < V; base += stride) {
-    unsigned const site = min(base + threadIdx.x, V - 1);
-    bool const valid = base + threadIdx.x < V;
-    unsigned s = site;
-    int c[4];
-    c[3] = (int)(s % (unsigned)geo.local[3]); s /= (unsigned)geo.local[3];
-    c[2] = (int)(s % (unsigned)geo.local[2]); s /= (unsigned)geo.local[2];
-    c[1] = (int)(s % (unsigned)geo.local[1]); s /= (unsigned)geo.local[1];
-    c[0] = (int)s;
-    // the arguments are small integer vectors times xunit: |a|^2, |b|^2 and
-    // a.b are exact integer sums (times xunit^2), so |a|, |b| and cos(a, b)
-    // come out of correctly rounded FP32 square roots and one division
-    // (within 1.5 ulp; the FP64 weight gets the same invariants in FP64)
-    int ix[4], ixy[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      int const G = geo.global[r];
-      int const rel = (c[r] + geo.pc[r] * geo.local[r] - gsx[r] + G) % G;
-      ix[r] = coord_map(rel, G);
-      ixy[r] = coord_map_diff(rel, yv[r], G);
-    }
-    int nx = 0, nxy = 0, dxy = 0, dxx = 0;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      nx += ix[r] * ix[r];
-      nxy += ixy[r] * ixy[r];
-      dxy += ix[r] * iy[r];
-      dxx += ix[r] * ixy[r];
-    }
+  for (unsigned site = blockIdx.x * blockDim.x + threadIdx.x; site < V; site += stride) {
+    SiteArgs const q = site_args(geo, gsx, yv, iy, site);
 #pragma unroll
     for (int e = 0; e < 3; ++e) {
       // e = 0: K(xm, ym), e = 1: K(ym, xm), e = 2: K(xm, x - y)
-      int const na = e == 1 ? ny : nx, nb = e == 0 ? ny : (e == 1 ? nx : nxy), nab = e == 2 ? dxx : dxy;
+      int const na = e == 1 ? ny : q.nx, nb = e == 0 ? ny : (e == 1 ? q.nx : q.nxy), nab = e == 2 ? q.dxx : q.dxy;
       float const ra = sqrtf((float)na), rb = sqrtf((float)nb);
       float const X = xuf * ra, Y = xuf * rb;
+      if (fminf(X, Y) < r64f) {
+        near[atomicAdd(near_n + pi, 1u)] = 3 * site + e;
+        continue;
+      }
       float cc = (na > 0 && nb > 0) ? (float)nab / (ra * rb) : 0.f;
       cc = fminf(1.f, fmaxf(-1.f, cc));
-      bool const near = fminf(X, Y) < r64f;
-      double ww[HLBL_QED_NW];
-      {
-        float wf[HLBL_QED_NW];
-        if (qf.geometric) weights_f32<true, false>(qf, X, cc, Y, wf);
-        else weights_f32<false, false>(qf, X, cc, Y, wf);
+      float wf[HLBL_QED_NW];
+      if (qf.geometric) weights_f32<true, false>(qf, X, cc, Y, wf);
+      else weights_f32<false, false>(qf, X, cc, Y, wf);
 #pragma unroll
-        for (int j = 0; j < HLBL_QED_NW; ++j) ww[j] = (double)wf[j];
-      }
-      double Xd = 0, cd = 0, Yd = 0;
-      if (near) {
-        Xd = args.xunit * sqrt((double)na);
-        Yd = args.xunit * sqrt((double)nb);
-        cd = (na > 0 && nb > 0) ? (double)nab / sqrt((double)na * (double)nb) : 0.0;
-        cd = cd > 1.0 ? 1.0 : (cd < -1.0 ? -1.0 : cd);
-      }
-      // near the origin: the FP64 weight of the FP64 arguments, the warp
-      // sharing each such evaluation (one quadrature node per lane)
-      unsigned const m = __ballot_sync(0xffffffffu, near);
-      if (m) qed_weights_fp64_warp(args.qp, m, Xd, cd, Yd, ww);
-      if (valid) {
+      for (int j = 0; j < HLBL_QED_NW; ++j) w[((size_t)site * 3 + e) * HLBL_QED_NW + j] = (double)wf[j];
+    }
+  }
+}
+
+// The listed evaluations in FP64, from the FP64 arguments: a half warp each,
+// lane = quadrature node. The order of the list does not matter (each
+// evaluation stands alone). The last CTA zeroes the counts for the next call:
+// near_n[0..kMaxBatch) the pairs' counts, near_n[kMaxBatch] the CTAs done.
+static __global__ void __launch_bounds__(kWThreads)
+qed_weights_near_kernel(Geometry geo, WArgs args, QedF32 qf, double* __restrict__ w,
+                        const unsigned* __restrict__ near, unsigned* __restrict__ near_n) {
+  static_assert(HLBL_QED_NQ == 16, "one node per lane of a half warp");
+  int const pi = blockIdx.y;
+  int const gsx[4] = {args.batch.p[pi].gsx[0], args.batch.p[pi].gsx[1], args.batch.p[pi].gsx[2], args.batch.p[pi].gsx[3]};
+  int const yv[4] = {args.batch.p[pi].yv[0], args.batch.p[pi].yv[1], args.batch.p[pi].yv[2], args.batch.p[pi].yv[3]};
+  w += (size_t)pi * geo.V * 3 * HLBL_QED_NW;
+  near += (size_t)pi * geo.V * 3;
+  int iy[4], ny = 0;
 #pragma unroll
-        for (int j = 0; j < HLBL_QED_NW; ++j) w[((size_t)site * 3 + e) * HLBL_QED_NW + j] = ww[j];
-      }
+  for (int r = 0; r < 4; ++r) {
+    iy[r] = coord_map(mod_pos(yv[r], geo.global[r]), geo.global[r]);
+    ny += iy[r] * iy[r];
+  }
+  unsigned const n = near_n[pi], halves = gridDim.x * (kWThreads / 16);
+  unsigned const half = blockIdx.x * (kWThreads / 16) + (threadIdx.x >> 4);
+  int const node = threadIdx.x & 15;
+  // a warp's two halves stay together: the one past the end repeats the last
+  for (unsigned i0 = half & ~1u; i0 < n; i0 += halves) {
+    unsigned const i = i0 + (half & 1u), dst = near[min(i, n - 1)];
+    int const e = (int)(dst % 3u);
+    SiteArgs const q = site_args(geo, gsx, yv, iy, dst / 3u);
+    int const na = e == 1 ? ny : q.nx, nb = e == 0 ? ny : (e == 1 ? q.nx : q.nxy), nab = e == 2 ? q.dxx : q.dxy;
+    double cd = (na > 0 && nb > 0) ? (double)nab / sqrt((double)na * (double)nb) : 0.0;
+    cd = cd > 1.0 ? 1.0 : (cd < -1.0 ? -1.0 : cd);
+    double t[HLBL_QED_NW];
+#pragma unroll
+    for (int j = 0; j < HLBL_QED_NW; ++j) t[j] = 0.0;
+    qed_node_fp64(args.qp, qf, node, args.xunit * sqrt((double)na), cd, args.xunit * sqrt((double)nb), t);
+#pragma unroll
+    for (int j = 0; j < HLBL_QED_NW; ++j) {
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) t[j] += __shfl_xor_sync(0xffffffffu, t[j], o);
+      if (node == j && i < n) w[(size_t)dst * HLBL_QED_NW + j] = t[j];
+    }
+  }
+  __syncthreads();  // every thread has read the count
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(near_n + kMaxBatch, 1u) == gridDim.x * gridDim.y - 1) {
+      for (int i = 0; i <= kMaxBatch; ++i) near_n[i] = 0u;
     }
   }
 }
@@ -924,34 +978,23 @@ p2_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, P2Args ar
 // out[fl] = sum_cta partials[cta][fl] (fixed order, compensated); if add
 // is set, out[fl] is added to rather than written.
 // One warp per flavour: lane l sums every 32nd CTA's partial (compensated),
-// lane 0 adds the 32 lane sums in order (fixed order, deterministic).
+// a shuffle tree adds the lanes' (fixed order, deterministic; five dependent
+// additions where lane 0 alone added 32).
 static __global__ void __launch_bounds__(64) p2_reduce_kernel(const double* __restrict__ partials, int ncta,
                                                               int nf, PairBatch batch, int add) {
   int const fl = threadIdx.x >> 5, lane = threadIdx.x & 31, pi = blockIdx.x;
-  __shared__ double rs[2][32], rc[2][32];
   if (fl >= nf) return;
   partials += (size_t)pi * ncta * nf;
-  double s = 0.0, c = 0.0;
-  for (int b = lane; b < ncta; b += 32) {
-    double const v = partials[(size_t)b * nf + fl];
-    double const tt = s + v;
-    c += fabs(s) >= fabs(v) ? (s - tt) + v : (v - tt) + s;
-    s = tt;
+  Neu a;
+  for (int b = lane; b < ncta; b += 32) a.add(partials[(size_t)b * nf + fl]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    double const os = __shfl_down_sync(0xffffffffu, a.s, o), oc = __shfl_down_sync(0xffffffffu, a.c, o);
+    a.add(os);
+    a.c += oc;
   }
-  rs[fl][lane] = s;
-  rc[fl][lane] = c;
-  __syncwarp();
   if (lane != 0) return;
-  s = 0.0;
-  c = 0.0;
-  for (int l = 0; l < 32; ++l) {
-    c += rc[fl][l];
-    double const v = rs[fl][l];
-    double const tt = s + v;
-    c += fabs(s) >= fabs(v) ? (s - tt) + v : (v - tt) + s;
-    s = tt;
-  }
-  s += c;
+  double const s = a.get();
   double* __restrict__ out = batch.p[pi].out;
   if (add) out[fl] += s;
   else out[fl] = s;

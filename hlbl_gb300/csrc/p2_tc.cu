@@ -149,14 +149,18 @@ __device__ __forceinline__ void f16_split2(float a, float b, uint32_t& hi, uint3
   hi = *reinterpret_cast<const uint32_t*>(&h);
   lo = *reinterpret_cast<const uint32_t*>(&l);
 }
+// 2^(15 - e), as far as FP32 has it
+__host__ __device__ __forceinline__ float f16_scale_exp(int e) {
+  int const k = 15 - e;
+  return ldexpf(1.f, k < -126 ? -126 : (k > 127 ? 127 : k));
+}
 // 2^(15 - e) for the smallest e with bound < 2^e: scales values bounded by
 // `bound` into FP16's range with a factor of two to spare (1 for bound 0)
 __host__ __device__ __forceinline__ float f16_scale(float bound) {
   if (!(bound > 0.f) || !(bound <= 3.0e38f)) return 1.f;  // zero, NaN or infinite inputs
   int e;
   frexpf(bound, &e);  // bound = m 2^e, m in [0.5, 1)
-  int const k = 15 - e;
-  return ldexpf(1.f, k < -126 ? -126 : (k > 127 ? 127 : k));
+  return f16_scale_exp(e);
 }
 
 // ---- tcgen05 / TMA helpers ---------------------------------------------------
@@ -834,98 +838,78 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
-// B operand of the tensor-core pass 2, from the gamma-inserted pass-1 sums:
-// per (pair, flavour) and chunk of 16 k, the 160 x 16 block of Bt^T as TF32
-// hi and lo parts in the K-major core-matrix layout (core (kg, n/8) at
-// (kg*20 + n/8)*128 bytes, row n%8 at 16 bytes, k%4 at 4 bytes). The values
-// are bt_build_kernel's.
-__global__ void btu_build_kernel(const double* __restrict__ g, int nf, float* __restrict__ btu) {
+// B operand of the tensor-core pass 2, from pass 1's sums dz with the gammas of
+// both sides written out (bt_build_kernel's values of g_build_kernel's g). Per
+// (pair, flavour) and chunk of 16 k, the 160 x 16 block of Bt^T in the K-major
+// core-matrix layout. TF32 operands: hi and lo parts (core (kg, n/8) at
+// (kg*20 + n/8)*128 bytes, row n%8 at 16 bytes, k%4 at 4 bytes). FP16 operands:
+// the values times bscale as hi, lo and lo2 parts, each the rounding of the
+// rest of the FP64 value (core (k/8, n/8) at (k/8*20 + n/8)*128 bytes, row n%8
+// at 16 bytes, k%8 at 2 bytes); bscale per (pair, flavour) is 2^(15 - e) with
+// 2^e above max |dz| (every Bt entry is a component of dz times a power of i),
+// which every CTA finds for itself from the 2880 sums: one launch, where g, its
+// maximum and the operand took three (8,192 sites,
+// four pairs: 27 -> 16 us).
+template <bool kF16>
+__global__ void __launch_bounds__(256) btu_build_kernel(const double* __restrict__ dz, float* __restrict__ bscale,
+                                                        void* __restrict__ btu) {
   int const fl = blockIdx.y, pi = blockIdx.z;
-  int const i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kBtK * kBtN || fl >= nf) return;
-  const double* g_dzu = g + ((size_t)pi * nf + fl) * kGLen;
-  const double* g_dzsu = g_dzu + kGDzuLen;
+  int const i = blockIdx.x * 256 + threadIdx.x;
+  dz += ((size_t)pi * 2 + fl) * kDzLen;
+  double scale = 1.0;
+  if constexpr (kF16) {
+    // the largest magnitude by the high words' bits: the exponent is all that
+    // the scale needs, and the integer pipe is 64 times the FP64 pipe
+    __shared__ unsigned red[8];
+    unsigned m = 0;
+    for (int q = threadIdx.x; q < kDzLen; q += 256) m = max(m, (unsigned)__double2hiint(dz[q]) & 0x7FFFFFFFu);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) m = max(m, red[w]);
+    int const e2 = (int)(m >> 20) - 1022;  // the largest is below 2^e2 (zero, infinite, NaN, beyond FP32: no scale)
+    float const sc = m == 0 || e2 > 127 ? 1.f : f16_scale_exp(e2);
+    if (blockIdx.x == 0 && threadIdx.x == 0) bscale[pi * 2 + fl] = sc;
+    scale = (double)sc;  // a power of two: exact
+  }
+  if (i >= kBtK * kBtN) return;
   int const k = i / kBtN, n = i % kBtN;
   // k within chunk c: 4 jj + 2 hh + e for the pair (p, q) the D formation
   // puts there (block b = c/2 of 4 p x 4 q, half c & 1)
-  int const cc = k / kKc, kl = k % kKc, jj = kl >> 2, hh = (kl >> 1) & 1, e = kl & 1;
-  int const bb = cc >> 1, bbp = bb / kBlocksQ, bbq = bb - bbp * kBlocksQ;
-  int const p = 4 * bbp + 2 * (cc & 1) + (jj >> 1), q = 4 * bbq + 2 * (jj & 1) + hh;
+  int const c = k / kKc, kl = k % kKc, jj = kl >> 2, hh = (kl >> 1) & 1, e = kl & 1;
+  int const bb = c >> 1, bbp = bb / kBlocksQ, bbq = bb - bbp * kBlocksQ;
+  int const p = 4 * bbp + 2 * (c & 1) + (jj >> 1), q = 4 * bbq + 2 * (jj & 1) + hh;
   int const lam = n & 3, nu = (n >> 2) & 3, j = n >> 4;
-  int const sq = q / 3, cq = q % 3;
-  int sq2 = 0;
-#pragma unroll
-  for (int s = 0; s < 4; ++s)
-    if (gg5_src(lam, s) == sq) sq2 = s;
-  int const ph = gg5_ph(lam, sq2);
-  const double* v = j < 6 ? g_dzu + ((((j * 4 + nu) * 12) + (3 * sq2 + cq)) * 12 + p) * 2
-                          : g_dzsu + (((((j - 6) * 4 + nu) * 12) + (3 * sq2 + cq)) * 12 + p) * 2;
+  // M[q][p] = i^(phases) dz[j][(s, c_q)][(gg5_src(nu, s_p), c_p)], s the spin
+  // that gamma_lam gamma_5 takes s_q from (an involution)
+  int const s2 = gg5_src(lam, q / 3), sp = p / 3;
+  int const ph = (gg5_ph(lam, s2) + gg5_ph(nu, sp)) & 3;
+  const double* v = dz + ((j * 12 + 3 * s2 + q % 3) * 12 + 3 * gg5_src(nu, sp) + p % 3) * 2;
   double re, im;
   mul_iph(ph, v[0], v[1], re, im);
-  double const x = e == 0 ? re : -im;
-  float const hi = __uint_as_float(tf32_rna((float)x));
-  float const lo = __uint_as_float(tf32_rna((float)(x - (double)hi)));
-  int const c = k / kKc, kk = k % kKc;
-  size_t const base = (((size_t)pi * 2 + fl) * kChunks + c) * 2 * kBPart;
-  int const off = ((kk >> 2) * (kBtN / 8) + (n >> 3)) * 32 + (n & 7) * 4 + (kk & 3);
-  btu[base + off] = hi;
-  btu[base + kBPart + off] = lo;
-}
-
-// FP16 operands: the B scale per (pair, flavour), 2^(15 - e) with 2^e above
-// max |g| (every Bt entry is a component of g times a power of i)
-__global__ void bscale_kernel(const double* __restrict__ g, int nf, float* __restrict__ bscale) {
-  __shared__ float red[8];
-  int const fl = blockIdx.x, pi = blockIdx.y;
-  const double* gp = g + ((size_t)pi * nf + fl) * kGLen;
-  float m = 0.f;
-  for (int i = threadIdx.x; i < kGLen; i += blockDim.x) m = fmaxf(m, fabsf((float)gp[i]));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmaxf(m, red[w]);
-    bscale[pi * 2 + fl] = f16_scale(m);
+  double const x = (e == 0 ? re : -im) * scale;
+  if constexpr (kF16) {
+    // x = f + g to 48 bits in FP32 (f64_to_f32: on the integer pipe), then the
+    // parts from f and g in FP32 (f - hi and r - lo are exact)
+    float const f = f64_to_f32(x), g = f64_to_f32(x - (double)f);
+    __half const hi = __float2half_rn(f);
+    float const r = f - __half2float(hi);
+    __half const lo = __float2half_rn(r + g);
+    __half const lo2 = __float2half_rn((r - __half2float(lo)) + g);
+    int const off = ((kl >> 3) * (kBtN / 8) + (n >> 3)) * 64 + (n & 7) * 8 + (kl & 7);
+    __half* out = static_cast<__half*>(btu) + (((size_t)pi * 2 + fl) * kChunks + c) * 3 * kBPart + off;
+    out[0] = hi;
+    out[kBPart] = lo;
+    out[2 * kBPart] = lo2;
+  } else {
+    float const hi = __uint_as_float(tf32_rna((float)x));
+    float const lo = __uint_as_float(tf32_rna((float)(x - (double)hi)));
+    int const off = ((kl >> 2) * (kBtN / 8) + (n >> 3)) * 32 + (n & 7) * 4 + (kl & 3);
+    float* out = static_cast<float*>(btu) + (((size_t)pi * 2 + fl) * kChunks + c) * 2 * kBPart + off;
+    out[0] = hi;
+    out[kBPart] = lo;
   }
-}
-
-// btu_build_kernel's values scaled by bscale, as FP16 hi, lo and lo2 parts
-// (each the rounding of the rest of the FP64 value) in the K-major
-// core-matrix layout of 8 k (core (k/8, n/8) at (k/8*20 + n/8)*128
-// bytes, row n%8 at 16 bytes, k%8 at 2 bytes)
-__global__ void btu16_build_kernel(const double* __restrict__ g, int nf, const float* __restrict__ bscale,
-                                   __half* __restrict__ btu) {
-  int const fl = blockIdx.y, pi = blockIdx.z;
-  int const i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kBtK * kBtN || fl >= nf) return;
-  const double* g_dzu = g + ((size_t)pi * nf + fl) * kGLen;
-  const double* g_dzsu = g_dzu + kGDzuLen;
-  int const k = i / kBtN, n = i % kBtN;
-  int const cc = k / kKc, kl = k % kKc, jj = kl >> 2, hh = (kl >> 1) & 1, e = kl & 1;
-  int const bb = cc >> 1, bbp = bb / kBlocksQ, bbq = bb - bbp * kBlocksQ;
-  int const p = 4 * bbp + 2 * (cc & 1) + (jj >> 1), q = 4 * bbq + 2 * (jj & 1) + hh;
-  int const lam = n & 3, nu = (n >> 2) & 3, j = n >> 4;
-  int const sq = q / 3, cq = q % 3;
-  int sq2 = 0;
-#pragma unroll
-  for (int s = 0; s < 4; ++s)
-    if (gg5_src(lam, s) == sq) sq2 = s;
-  int const ph = gg5_ph(lam, sq2);
-  const double* v = j < 6 ? g_dzu + ((((j * 4 + nu) * 12) + (3 * sq2 + cq)) * 12 + p) * 2
-                          : g_dzsu + (((((j - 6) * 4 + nu) * 12) + (3 * sq2 + cq)) * 12 + p) * 2;
-  double re, im;
-  mul_iph(ph, v[0], v[1], re, im);
-  double const x = (e == 0 ? re : -im) * (double)bscale[pi * 2 + fl];  // a power of two: exact
-  __half const hi = __double2half(x);
-  double const r1 = x - (double)__half2float(hi);
-  __half const lo = __double2half(r1);
-  __half const lo2 = __double2half(r1 - (double)__half2float(lo));
-  int const off = ((kl >> 3) * (kBtN / 8) + (n >> 3)) * 64 + (n & 7) * 8 + (kl & 7);
-  size_t const base = (((size_t)pi * 2 + fl) * kChunks + cc) * 3 * kBPart;
-  btu[base + off] = hi;
-  btu[base + kBPart + off] = lo;
-  btu[base + 2 * kBPart + off] = lo2;
 }
 
 }  // namespace tc
@@ -956,14 +940,10 @@ int tc_init(int nsm, int& grid) {
   return HLBL_OK;
 }
 
-void tc_launch_btu(const double* d_g, int npairs, void* d_btu, bool f16, float* d_bscale, cudaStream_t st) {
+void tc_launch_btu(const double* d_dz, int npairs, void* d_btu, bool f16, float* d_bscale, cudaStream_t st) {
   dim3 const gb((kBtK * kBtN + 255) / 256, 2, npairs);
-  if (f16) {
-    tc::bscale_kernel<<<dim3(2, npairs), 256, 0, st>>>(d_g, 2, d_bscale);
-    tc::btu16_build_kernel<<<gb, 256, 0, st>>>(d_g, 2, d_bscale, static_cast<__half*>(d_btu));
-  } else {
-    tc::btu_build_kernel<<<gb, 256, 0, st>>>(d_g, 2, static_cast<float*>(d_btu));
-  }
+  if (f16) tc::btu_build_kernel<true><<<gb, 256, 0, st>>>(d_dz, d_bscale, d_btu);
+  else tc::btu_build_kernel<false><<<gb, 256, 0, st>>>(d_dz, d_bscale, d_btu);
 }
 
 void tc_launch_p2(int grid, int npairs, cudaStream_t st, const TcBatch& tb, const Geometry& geo,

@@ -39,7 +39,7 @@ size_t tc_btu_floats_per_pair();
 int tc_init(int nsm, int& grid);
 // f16: FP16 operands (B built with a per-(pair, flavour) scale into
 // d_bscale[2 * pair + flavour]; the copies' trailers give A's scale)
-void tc_launch_btu(const double* d_g, int npairs, void* d_btu, bool f16, float* d_bscale, cudaStream_t st);
+void tc_launch_btu(const double* d_dz, int npairs, void* d_btu, bool f16, float* d_bscale, cudaStream_t st);
 void tc_launch_p2(int grid, int npairs, cudaStream_t st, const TcBatch& tb, const Geometry& geo,
                   const P2Args& a, const void* d_btu, bool f16, const float* d_bscale, double* partials, int* err);
 long long tc_tiles(long long V);

@@ -326,7 +326,7 @@ __device__ __forceinline__ void weights(const P234Args& p, const T* a, const T* 
   if constexpr (sizeof(T) == 8) {
     double X, c, Y;
     hlbl_qed_invariants(a, b, &X, &c, &Y);
-    hlbl_qed_weights(&p.qp, X, c, Y, w);
+    qed_weights_fp64(p.qp, p.qf, X, c, Y, w);
   } else {
     float xx = 0.f, yy = 0.f, xy = 0.f;
 #pragma unroll
@@ -345,7 +345,7 @@ __device__ __forceinline__ void weights(const P234Args& p, const T* a, const T* 
         bd[r] = (double)b[r];
       }
       hlbl_qed_invariants(ad, bd, &Xd, &cd, &Yd);
-      hlbl_qed_weights(&p.qp, Xd, cd, Yd, wd);
+      qed_weights_fp64(p.qp, p.qf, Xd, cd, Yd, wd);
 #pragma unroll
       for (int j = 0; j < 6; ++j) w[j] = (float)wd[j];
     } else {

@@ -73,7 +73,7 @@ struct QedStandIn {
 #pragma unroll
       for (int j = 0; j < HLBL_QED_NW; ++j) w[j] = wf[j];
     } else {
-      hlbl_qed_weights(&qp, X, c, Y, w);
+      qed_weights_fp64(qp, qf, X, c, Y, w);
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {

@@ -518,7 +518,7 @@ qed_weights_surrogate_kernel(Geometry geo, WArgs args, const float* __restrict__
         cd = cd > 1.0 ? 1.0 : (cd < -1.0 ? -1.0 : cd);
       }
       unsigned const m = __ballot_sync(0xffffffffu, near);
-      if (m) qed_weights_fp64_warp(args.qp, m, Xd, cd, Yd, ww);
+      if (m) qed_weights_fp64_warp(args.qp, qf, m, Xd, cd, Yd, ww);
       if (valid) {
         fb += outside ? 1 : 0;
 #pragma unroll
