@@ -10,17 +10,17 @@
 // are FP32 in the 3xTF32 form A_hi B_hi + A_hi B_lo + A_lo B_hi (hi = the
 // TF32 rounding, lo = the TF32 rounding of the rest), accumulated in TMEM.
 //
-// Warp roles (15 warps):
+// Warp roles (19 warps):
 //   0      TMA producer of the FP32 input rows (S = x[1-f] rows q, Y = y[f]
 //          rows p: 3 KB per (flavour, ia, tile)) -- one thread
 //   1      TMA producer of the B chunks (16 k x 160 n, hi and lo, 20 KB) -- one thread
 //   2      TMEM allocation; tcgen05.mma issue and commits -- one thread
-//   3-10   D formation, two groups of four warps on alternate chunks of
+//   3-14   D formation, three groups of four warps on every third chunk of
 //          16 k (8 (p, q): half of a block of 4 p x 4 q): warp j of a group
 //          forms the chunk's j-th pair of (p, q) (one Y row, two S rows) for
 //          its lane's site: O = Y conj(S) spin blocks -> D_mu -> hi/lo ->
 //          shared memory in the K-major no-swizzle core-matrix layout
-//   11-14  epilogue: one TMEM lane quadrant each (warp % 4 = mu); per phase,
+//   15-18  epilogue: one TMEM lane quadrant each (warp % 4 = mu); per phase,
 //          the F rows from TMEM dotted with the QED coefficients of the
 //          row's site, into a compensated FP64 sum
 // The tensor cores accumulate in FP32 with truncation (biased toward zero),
@@ -71,8 +71,8 @@ constexpr int kChunks = kBtK / kKc;        // 18
 // sets stream through small rings instead of one being held for a whole
 // phase: the S rows 4 bq..4 bq+3 of a block (a ring of two blocks; fetched
 // again, from L2, for each p-block) and the Y rows of a p-block by halves,
-// half h (rows 4 bp + 2h, 4 bp + 2h + 1) read only by D group h (a ring of
-// three halves). This leaves room for five A and B stages.
+// half h (rows 4 bp + 2h, 4 bp + 2h + 1) read by each D group in one of its
+// three chunks (a ring of three halves). This leaves room for five A and B stages.
 constexpr int kRowsPerGroup = 4, kBlocksQ = 3;
 constexpr int kYRows = 2;
 constexpr int kBlocks = 9;  // per phase: 3 p-blocks x 3 q-blocks
@@ -80,8 +80,9 @@ constexpr int kHalf = kChunks / 2;               // chunks per main-accumulator 
 constexpr uint32_t kCorrCol = 2 * kBtN;          // the correction accumulator's first column
 constexpr int kAPart = kM * kKc;           // floats per A part (hi or lo)
 constexpr int kBPart = kBtN * kKc;         // floats per B part
-constexpr int kWarpRows = 0, kWarpB = 1, kWarpMma = 2, kWarpD0 = 3, kDWarps = 8;
-constexpr int kDGroup = 4;  // D warps per chunk (a group); kDWarps / kDGroup chunks in flight
+constexpr int kWarpRows = 0, kWarpB = 1, kWarpMma = 2, kWarpD0 = 3, kDWarps = 12;
+constexpr int kDGroup = 4;  // D warps per chunk (a group); kDGroups chunks in flight
+constexpr int kDGroups = kDWarps / kDGroup;
 constexpr int kWarpE0 = kWarpD0 + kDWarps, kEWarps = 4;
 constexpr int kThreads = 32 * (kWarpE0 + kEWarps);
 constexpr uint32_t kTmemCols = 512;
@@ -200,6 +201,12 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                    smem_u32(bar))
                : "memory");
 }
+// true in one lane of the converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -229,7 +236,12 @@ __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.
 
 // A wait that gives up when the CTA has failed or after kWaitLimit polls
 // (then it marks the CTA failed). Returns false on give-up.
+// The first poll stands before the loop: it succeeds nearly always (try_wait
+// itself waits for a while), and its path is then short (60 cycles where the
+// loop alone took 240, twice per chunk in the MMA warp).
 __device__ __forceinline__ bool wait_or_fail(uint64_t* bar, uint32_t parity, volatile int* fail) {
+  if (mbar_try_wait(bar, parity)) return true;
+#pragma unroll 1
   for (uint32_t i = 0; i < kWaitLimit; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 63) == 63 && *fail) return false;
@@ -435,8 +447,8 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
   };
 
   if (t == 0) {
-    for (int i = 0; i < kSGroups; ++i) { mbar_init(&sm.s_full[i], 1); mbar_init(&sm.s_empty[i], kDWarps); }
-    for (int i = 0; i < kYSlots; ++i) { mbar_init(&sm.y_full[i], 1); mbar_init(&sm.y_empty[i], kDGroup); }
+    for (int i = 0; i < kSGroups; ++i) { mbar_init(&sm.s_full[i], 1); mbar_init(&sm.s_empty[i], 2 * kDGroup); }
+    for (int i = 0; i < kYSlots; ++i) { mbar_init(&sm.y_full[i], 1); mbar_init(&sm.y_empty[i], kDGroups * kDGroup); }
     for (int i = 0; i < kSt; ++i) { mbar_init(&sm.a_full[i], kDGroup); mbar_init(&sm.a_empty[i], 1); }
     for (int i = 0; i < kSt; ++i) { mbar_init(&sm.b_full[i], 1); mbar_init(&sm.b_empty[i], 1); }
     mbar_init(&sm.acc_full, 1);
@@ -478,10 +490,13 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
     // issued before it.
     if (lane == 0 && nph > 0) {
       bool ok = true;
+#pragma unroll 1
       for (int P = 0; ok && P < nph; ++P) {
         int const f = P & 1;
         long long const tile = blockIdx.x + (long long)(P >> 1) * gridDim.x;
+#pragma unroll 1
         for (int bp = 0; ok && bp < 3; ++bp) {
+#pragma unroll 1
           for (int h = 0; ok && h < 2; ++h) {
             int const uy = (P * 3 + bp) * 2 + h, ys = uy % kYSlots;
             if (!wait_or_fail(&sm.y_empty[ys], (uint32_t)(((uy / kYSlots) & 1) ^ 1), fail)) { ok = false; break; }
@@ -491,6 +506,7 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
               bulk_g2s(sm.Y[ys][r], row_ptr(y32, f, 4 * bp + 2 * h + r, tile), kRowBytes, &sm.y_full[ys]);
             rows_issued_y = uy;
           }
+#pragma unroll 1
           for (int bq = 0; ok && bq < kBlocksQ; ++bq) {
             int const us = P * kBlocks + bp * kBlocksQ + bq, ss = us % kSGroups;
             if (!wait_or_fail(&sm.s_empty[ss], (uint32_t)(((us / kSGroups) & 1) ^ 1), fail)) { ok = false; break; }
@@ -508,10 +524,12 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
     if (lane == 0) {
       int bc = 0;
       bool ok = true;
+#pragma unroll 1
       for (int P = 0; ok && P < nph; ++P) {
         constexpr int kBP = OpT<kF16>::kBParts;
         const unsigned char* src =
             static_cast<const unsigned char*>(btu) + ((size_t)pi * 2 + (P & 1)) * kChunks * kBP * Sm::kBPartB;
+#pragma unroll 1
         for (int c = 0; c < kChunks; ++c, ++bc) {
           int const st = bc % kSt;
           if (!wait_or_fail(&sm.a_empty[st], (uint32_t)(((bc / kSt) & 1) ^ 1), fail)) { ok = false; break; }
@@ -524,12 +542,14 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
     }
   } else if (warp == kWarpMma) {
     // ---- MMA issue ----------------------------------------------------------------
-    // The tensor pipe runs the six MMAs of a chunk in about 500 cycles, so the
-    // issuing thread's own per-chunk work has to stay well below that: the
-    // stage descriptors differ only in their start address (bits 0-13, in
-    // 16-byte units, no carry below 256 KB), so they are formed once and
-    // advanced by constants; ring positions and phases are counters.
-    if (lane == 0) {
+    // The tensor pipe runs the four FP16 MMAs of a chunk in about 330 cycles,
+    // so the issuing warp's own per-chunk work has to stay well below that: the
+    // whole warp walks the loop and waits, so that its control flow and the
+    // descriptors are uniform, and one elected lane issues; the stage
+    // descriptors differ only in their start address (bits 0-13, in 16-byte
+    // units, no carry below 256 KB), so they are formed once and advanced by
+    // constants; ring positions and phases are counters.
+    {
       uint64_t const a_desc0 = sdesc(smem_u32(sm.A[0][0]), (kM / 8) * 128, 128);
       uint64_t const b_desc0 = sdesc(smem_u32(sm.B[0][0]), (kBtN / 8) * 128, 128);
       // in 16-byte units: stage to stage, hi to lo part, and (TF32, two
@@ -543,12 +563,14 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
       uint32_t aph = 0, bph = 0;
       uint32_t const dc = tmem + kCorrCol;
       bool ok = true;
+#pragma unroll 1
       for (int P = 0; ok && P < nph; ++P) {
         // first half into main buffer P&1 (phase P-1's second half, free once
         // folded), second half into buffer (P+1)&1 (free once dotted)
         if (!wait_or_fail(&sm.folded, (uint32_t)((P & 1) ^ 1), fail)) break;
         tc_fence_after();
         uint32_t const d0 = tmem + (uint32_t)((P & 1) * kBtN), d1 = tmem + (uint32_t)(((P + 1) & 1) * kBtN);
+#pragma unroll 1
         for (int c = 0; c < kChunks; ++c) {
           if (c == kHalf) {
             if (!wait_or_fail(&sm.dotted, (uint32_t)((P & 1) ^ 1), fail)) { ok = false; break; }
@@ -563,6 +585,7 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
           uint64_t const ahi = a_desc0 + (uint64_t)as * kAStage16, bhi = b_desc0 + (uint64_t)bs * kBStage16;
           // hi.hi into the main buffer, hi.lo and lo.hi into the correction
           // accumulator
+          if (elect_one()) {
           if constexpr (kF16) {
             mma_f16(d, ahi, bhi, (c != 0 && c != kHalf) ? 1u : 0u);
             mma_f16(dc, ahi, bhi + kBLo16, c ? 1u : 0u);
@@ -576,13 +599,16 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
             mma_tf32(dc, ahi + kAK16, bhi + kBK16 + kBLo16, 1u);
             mma_tf32(dc, ahi + kAK16 + kALo16, bhi + kBK16, 1u);
           }
-          mma_any = true;
           mma_commit(&sm.a_empty[as]);  // also frees B stage bs (= as)
+          }
+          __syncwarp();
+          mma_any = true;
           if (++as == kSt) { as = 0; aph ^= 1u; }
           if (++bs == kSt) { bs = 0; bph ^= 1u; }
         }
         if (!ok) break;
-        mma_commit(&sm.acc_full);
+        if (elect_one()) mma_commit(&sm.acc_full);
+        __syncwarp();
       }
     }
   } else if (warp < kWarpE0) {
@@ -591,18 +617,19 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
     int const j = (warp - kWarpD0) % kDGroup;    // the chunk's j-th pair of (p, q)
     int const s = lane;
     bool ok = true;
-    float y[24];  // this lane's Y row p: loaded at a p-block's first chunk, kept for its three
+#pragma unroll 1
     for (int P = 0; ok && P < nph; ++P) {
       long long const tile = blockIdx.x + (long long)(P >> 1) * gridDim.x;
       int const nvalid = (int)min((long long)kSites, geo.V - tile * kSites);
-      for (int c = grp; c < kChunks; c += kDWarps / kDGroup) {
-        // chunk c is half c & 1 (= grp) of block b = (bp, bq): this warp's
-        // pair is p = 4 bp + 2 grp + j/2 (row p_in of the Y group) and
+#pragma unroll 1
+      for (int c = grp; c < kChunks; c += kDGroups) {
+        // chunk c is half c & 1 of block b = (bp, bq): this warp's
+        // pair is p = 4 bp + 2 (c & 1) + j/2 (row p_in of the Y half) and
         // q = 4 bq + q_in, q_in + 1 (rows of the S group), q_in = 2 (j & 1)
         int const b = c >> 1, bp = b / kBlocksQ, bq = b - bp * kBlocksQ;
-        int const uy = (P * 3 + bp) * 2 + grp, ys = uy % kYSlots;  // this group's half
+        int const uy = (P * 3 + bp) * 2 + (c & 1), ys = uy % kYSlots;
         int const us = P * kBlocks + b, ss = us % kSGroups;
-        if (bq == 0) ok = ok && wait_or_fail(&sm.y_full[ys], (uint32_t)((uy / kYSlots) & 1), fail);
+        ok = ok && wait_or_fail(&sm.y_full[ys], (uint32_t)((uy / kYSlots) & 1), fail);
         ok = ok && wait_or_fail(&sm.s_full[ss], (uint32_t)((us / kSGroups) & 1), fail);
         int const ac = P * kChunks + c, as = ac % kSt;
         if (!ok || !wait_or_fail(&sm.a_empty[as], (uint32_t)(((ac / kSt) & 1) ^ 1), fail)) { ok = false; break; }
@@ -612,7 +639,8 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
         unsigned char* Ahi = sm.A[as][0] + (kF16 ? (j >> 1) * 2048 + s * 16 + 8 * (j & 1) : j * 2048 + s * 16);
         unsigned char* Alo = sm.A[as][1] + (kF16 ? (j >> 1) * 2048 + s * 16 + 8 * (j & 1) : j * 2048 + s * 16);
         if (s < nvalid) {
-          if (bq == 0) {
+          float y[24];
+          {
             const float* Yr = sm.Y[ys][p_in] + f32_tile_off(s, 0);
             float const sc = kF16 ? ((P & 1) ? ascale1 : ascale0) : 1.f;  // FP16: D scaled through Y
 #pragma unroll
@@ -705,10 +733,10 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
         __syncwarp();
         if (lane == 0) {
           mbar_arrive(&sm.a_full[as]);
-          // every D warp reads each S block in one chunk; a group reads its
-          // Y half in three (bq = 0..2)
+          // two groups read each S block, in one chunk each; every group
+          // reads each Y half, in one of its three chunks (bq = 0..2)
           mbar_arrive(&sm.s_empty[ss]);
-          if (bq == kBlocksQ - 1) mbar_arrive(&sm.y_empty[ys]);
+          mbar_arrive(&sm.y_empty[ys]);
         }
       }
     }
@@ -727,6 +755,7 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
 #pragma unroll
     for (int r = 0; r < 4; ++r) q.ym[r] = (float)(coord_map(mod_pos(yv[r], geo.global[r]), geo.global[r]) * xu);
     Neu run0, run1;
+#pragma unroll 1
     for (int P = 0; P < nph; ++P) {
       long long const tile = blockIdx.x + (long long)(P >> 1) * gridDim.x;
       long long const v = tile * kSites + s;
