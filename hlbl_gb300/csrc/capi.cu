@@ -244,6 +244,10 @@ struct hlbl_ctx {
   size_t x32_floats = 0;
   float* d_btu = nullptr;     // tensor-core B operand [kMaxBatch][tc_btu_floats_per_pair]
   float* d_bscale = nullptr;  // FP16 operands: B scale [kMaxBatch][2]
+  double* d_tsum = nullptr;   // tensor-core pass 2: per-tile sums (tc_tsum_len)
+  size_t tsum_cap = 0;        // doubles
+  double* d_tred = nullptr;   // its reduction's parts [kTcRedPart]
+  unsigned* d_tcnt = nullptr;  // its tile counter and the reduction's [1 + kMaxBatch]
   int tc16 = 1;               // FP16 operands in the FP32-copy path's pass 2 (hlbl_ctx_set_tc_fp16)
   // staging of host blocks on a side stream (hlbl_stage_async)
   cudaStream_t copy_stream = nullptr;
@@ -397,6 +401,21 @@ int run_pass1(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch
   return HLBL_OK;
 }
 
+// The per-tile sums of the tensor-core pass 2 for npairs pairs.
+int ensure_tsum(hlbl_ctx* c, const Geometry& geo, int npairs) {
+  size_t const need = tc_tsum_len(geo.V, npairs);
+  if (need <= c->tsum_cap) return HLBL_OK;
+  if (c->capturing) return fail(HLBL_ESTATE, "tile sum buffer too small during graph capture");
+  cudaStreamSynchronize(c->stream);
+  cudaFree(c->d_tsum);
+  c->d_tsum = nullptr;
+  c->tsum_cap = 0;
+  cudaError_t e = cudaMalloc(&c->d_tsum, sizeof(double) * need);
+  if (e != cudaSuccess) return fail(HLBL_ENOMEM, "tile sum buffer: %s", cudaGetErrorString(e));
+  c->tsum_cap = need;
+  return HLBL_OK;
+}
+
 // The QED weight buffers for `need` sites over all pairs of a launch.
 int ensure_weights(hlbl_ctx* c, long long need) {
   if (need <= c->w_cap) return HLBL_OK;
@@ -501,6 +520,8 @@ int run_pass2(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch
   a.xunit = xunit;
   a.f0 = f0;
   int grid;
+  if (use_tc(c, precision, nf))
+    if (int rc = ensure_tsum(c, geo, b.n)) return rc;
   prof_begin(c, 1);
   if (precision == HLBL_FP64) {
     grid = per_pair_grid(c->grid_p2d[nf - 1], b.n, p2f64_tiles(geo.V));
@@ -514,8 +535,10 @@ int run_pass2(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch
       tb.x32[i] = x32_block(c, geo, 1 + i);
       for (int r = 0; r < 4; ++r) { tb.gsx[i][r] = b.p[i].gsx[r]; tb.yv[i][r] = b.p[i].yv[r]; }
     }
-    grid = per_pair_grid(c->grid_tc, b.n, tc_tiles(geo.V));
-    tc_launch_p2(grid, b.n, c->stream, tb, geo, a, c->d_btu, false, nullptr, c->d_part2, c->d_err);
+    tc_launch_p2(c->grid_tc, b.n, c->stream, tb, geo, a, c->d_btu, false, nullptr, c->d_tsum, c->d_tcnt, c->d_err);
+    prof_end(c, 1);
+    tc_launch_reduce(b.n, c->stream, geo, c->d_tsum, c->d_tred, c->d_tcnt, c->d_tcnt + 1, b, add);
+    return HLBL_OK;
   } else {
     const float* bt = static_cast<const float*>(c->d_bt);
     if (nf == 2 && c->p2_small) { grid = per_pair_grid(c->grid_p2f2s, b.n, P2F2s::tiles(geo.V)); P2F2s::launch(grid, c->stream, y, b, geo, a, bt, c->d_part2, c->d_err); }
@@ -549,11 +572,11 @@ int run_group_f32(hlbl_ctx* c, const PairBatch& b, const TcBatch& tb, double xun
   if (int rc = run_qed(c, geo, b, xunit, HLBL_FP32, a)) return rc;
   a.xunit = xunit;
   a.f0 = 0;
-  int const g2 = per_pair_grid(c->grid_tc, b.n, tc_tiles(geo.V));
+  if (int rc = ensure_tsum(c, geo, b.n)) return rc;
   prof_begin(c, 1);
-  tc_launch_p2(g2, b.n, c->stream, tb, geo, a, c->d_btu, c->tc16 != 0, c->d_bscale, c->d_part2, c->d_err);
+  tc_launch_p2(c->grid_tc, b.n, c->stream, tb, geo, a, c->d_btu, c->tc16 != 0, c->d_bscale, c->d_tsum, c->d_tcnt, c->d_err);
   prof_end(c, 1);
-  p2_reduce_kernel<<<b.n, 64, 0, c->stream>>>(c->d_part2, g2, 2, b, 0);
+  tc_launch_reduce(b.n, c->stream, geo, c->d_tsum, c->d_tred, c->d_tcnt, c->d_tcnt + 1, b, 0);
   return HLBL_OK;
 }
 
@@ -633,6 +656,8 @@ int hlbl_ctx_create(hlbl_ctx** out, const int global[4], const int local[4],
       {(void**)&c->d_bt, sizeof(double) * kMaxBatch * 2 * kBtK * kBtN},
       {(void**)&c->d_dzq, sizeof(double) * kMaxBatch * 2 * p2f64_dzq_len()},
       {(void**)&c->d_bad, sizeof(int)},
+      {(void**)&c->d_tred, sizeof(double) * kTcRedPart},
+      {(void**)&c->d_tcnt, sizeof(unsigned) * (1 + kMaxBatch)},
       {(void**)&c->d_near_n, sizeof(unsigned) * (kMaxBatch + 1)},
       {(void**)&c->d_btu, sizeof(float) * kMaxBatch * tc_btu_floats_per_pair()},
       {(void**)&c->d_bscale, sizeof(float) * kMaxBatch * 2},
@@ -643,6 +668,7 @@ int hlbl_ctx_create(hlbl_ctx** out, const int global[4], const int local[4],
     if (e != cudaSuccess) return bail(fail(HLBL_ENOMEM, "cudaMalloc %zu bytes: %s", b.n, cudaGetErrorString(e)));
   }
   e = cudaMemset(c->d_err, 0, sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(c->d_tcnt, 0, sizeof(unsigned) * (1 + kMaxBatch));
   if (e == cudaSuccess) e = cudaMemset(c->d_near_n, 0, sizeof(unsigned) * (kMaxBatch + 1));
   if (e != cudaSuccess) return bail(cuda_fail(e, "error flag"));
   e = cudaMallocHost(reinterpret_cast<void**>(&c->h_out), sizeof(double) * 2);
@@ -670,6 +696,9 @@ void hlbl_ctx_destroy(hlbl_ctx* c) {
   cudaFree(c->d_w);
   cudaFree(c->d_near);
   cudaFree(c->d_near_n);
+  cudaFree(c->d_tsum);
+  cudaFree(c->d_tred);
+  cudaFree(c->d_tcnt);
   cudaFree(c->d_coef);
   cudaFree(c->d_dense64);
   cudaFree(c->d_dense32);
@@ -1095,6 +1124,7 @@ int hlbl_ctx_reserve(hlbl_ctx* c, int max_pairs) {
     int const group = c->batch_group > 0 ? std::min(c->batch_group, kMaxBatch) : kMaxBatch;
     if (int rc = ensure_x32(c, c->geo, std::min(max_pairs, group))) return rc;
   }
+  if (int rc = ensure_tsum(c, c->geo, std::min(max_pairs, kMaxBatch))) return rc;
   if (c->qed_kind != kQedStandInClosed) {
     // the generic path's coefficients: FP64 layout for the pair groups of the
     // FP64-block calls, FP32 layout for those of the FP32-copy path

@@ -4,8 +4,8 @@
 // (ker_4pt_contraction, cuda_lattice.cu:277-484, restructured as in
 // contract_kernels.cuh).
 //
-// Per CTA (one per SM, persistent over tiles of 32 sites) and per phase
-// (tile, flavour f): the 128 x 160 product F = A . B^T, A = Dr with rows
+// Per CTA (one per SM, persistent; tiles of 32 sites of all pairs from a common
+// queue) and per phase (tile, flavour f): the 128 x 160 product F = A . B^T, A = Dr with rows
 // (mu, site) = mu*32 + site and K = 288 = (p, q, re/im), B = Bt^T. Products
 // are FP32 in the 3xTF32 form A_hi B_hi + A_hi B_lo + A_lo B_hi (hi = the
 // TF32 rounding, lo = the TF32 rounding of the rest), accumulated in TMEM.
@@ -22,7 +22,9 @@
 //          shared memory in the K-major no-swizzle core-matrix layout
 //   15-18  epilogue: one TMEM lane quadrant each (warp % 4 = mu); per phase,
 //          the F rows from TMEM dotted with the QED coefficients of the
-//          row's site, into a compensated FP64 sum
+//          row's site; the quadrant's sum is stored per (tile, flavour), and
+//          the tiles' sums are added in a fixed order afterwards, whichever
+//          CTA took them
 // The tensor cores accumulate in FP32 with truncation (biased toward zero),
 // so the error grows with the number of MMAs added into one accumulator and
 // the small hi.lo and lo.hi products lose most of their bits if added into
@@ -46,6 +48,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
@@ -85,6 +88,13 @@ constexpr int kDGroup = 4;  // D warps per chunk (a group); kDGroups chunks in f
 constexpr int kDGroups = kDWarps / kDGroup;
 constexpr int kWarpE0 = kWarpD0 + kDWarps, kEWarps = 4;
 constexpr int kThreads = 32 * (kWarpE0 + kEWarps);
+// The CTAs take their units (pair, tile) from a common counter: at 663,552
+// sites the same number of tiles each took 2.50 to 3.45 ms (both SMs of a TPC
+// the same time, not the same TPCs from run to run), so that a fixed share each
+// made the slowest hold the kernel. The row producer draws them, a few ahead,
+// and hands them to the other warps through a small queue.
+constexpr int kQueue = 4;
+constexpr int kQueueReaders = 2 + kDWarps + kEWarps;  // B producer, MMA, D and epilogue warps
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kRowBytes = kRowF32 * 4;  // 3072
 
@@ -133,9 +143,10 @@ struct __align__(1024) SmemT {
   uint64_t s_full[kSGroups], s_empty[kSGroups], y_full[kYSlots], y_empty[kYSlots];
   uint64_t a_full[kSt], b_full[kSt], a_empty[kSt], b_empty[kSt];
   uint64_t acc_full, folded, dotted, mma_done;
+  uint64_t q_full[kQueue], q_empty[kQueue];
+  uint32_t unit[kQueue];  // the queue of this CTA's (pair, tile) units
   uint32_t taddr;
   int fail;
-  double red[kEWarps][2][2];
 };
 using Smem = SmemT<false>;
 static_assert(sizeof(SmemT<false>) <= 232448 && sizeof(SmemT<true>) <= 232448,
@@ -429,20 +440,17 @@ static_assert(d_ph(2, 0) == 0 && d_ph(2, 1) == 2 && d_ph(2, 2) == 0 && d_ph(2, 3
 template <bool kGeneric, bool kF16>
 __global__ void __launch_bounds__(kThreads, 1)
 p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
-            const float* __restrict__ bscale, double* __restrict__ partials, int* __restrict__ err) {
+            const float* __restrict__ bscale, int npairs, double* __restrict__ tsum,
+            unsigned* __restrict__ next_unit, int* __restrict__ err) {
   using Sm = SmemT<kF16>;
   constexpr int kSt = Sm::kSt, kSGroups = Sm::kSGroups, kYSlots = Sm::kYSlots;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   Sm& sm = *reinterpret_cast<Sm*>(smem_raw);
   volatile int* fail = &sm.fail;
   int const t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  int const pi = blockIdx.y;
-  long long const ntiles = (geo.V + kSites - 1) / kSites;
-  long long const my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  int const nph = (int)(2 * my_tiles);
-  const float* __restrict__ x32 = tb.x32[pi];
+  uint32_t const ntiles = (uint32_t)((geo.V + kSites - 1) / kSites), nunits = ntiles * (uint32_t)npairs;
   const float* __restrict__ y32 = tb.y32;
-  auto row_ptr = [&](const float* base, int f, int ia, long long tile) {
+  auto row_ptr = [&](const float* base, int f, int ia, uint32_t tile) {
     return base + ((size_t)(f * 12 + ia) * ntiles + tile) * kRowF32;
   };
 
@@ -455,6 +463,7 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
     mbar_init(&sm.folded, kEWarps);
     mbar_init(&sm.dotted, kEWarps);
     mbar_init(&sm.mma_done, 1);
+    for (int i = 0; i < kQueue; ++i) { mbar_init(&sm.q_full[i], 1); mbar_init(&sm.q_empty[i], kQueueReaders); }
     fence_mbar_init();
     sm.fail = 0;
   }
@@ -467,15 +476,22 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
   __syncthreads();
   tc_fence_after();
   uint32_t const tmem = sm.taddr;
-  // FP16: the A scale per flavour f from the tile copies' maxima, x[1 - f]
-  // (rows S) and y[f] (rows Y): |D| <= 12 |Y| |S| <= 24 max|Y| max|S|
-  float ascale0 = 1.f, ascale1 = 1.f;
-  if constexpr (kF16) {
+  // FP16: the A scale of pair pi and flavour f from the tile copies' maxima,
+  // x[1 - f] (rows S) and y[f] (rows Y): |D| <= 12 |Y| |S| <= 24 max|Y| max|S|
+  auto a_scale = [&](uint32_t pi, int f) -> float {
     const float* tx = tb.x32[pi] + f32_tile_floats(geo.V);
     const float* ty = tb.y32 + f32_tile_floats(geo.V);
-    ascale0 = f16_scale(24.f * tx[1] * ty[0]);
-    ascale1 = f16_scale(24.f * tx[0] * ty[1]);
-  }
+    return f16_scale(24.f * tx[1 - f] * ty[f]);
+  };
+  // the i-th unit of this CTA (>= nunits: no more), for a whole warp
+  auto next = [&](int i, uint32_t& unit) -> bool {
+    int const qs = i % kQueue;
+    if (!wait_or_fail(&sm.q_full[qs], (uint32_t)((i / kQueue) & 1), fail)) return false;
+    unit = *reinterpret_cast<volatile uint32_t*>(&sm.unit[qs]);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sm.q_empty[qs]);
+    return unit < nunits;
+  };
 
   // issue tracking for the teardown after a failure
   int rows_issued_s = -1, rows_issued_y = -1;  // last S block / Y p-block use issued
@@ -488,54 +504,72 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
     // then the S rows of its three blocks. A wait here is for the ring slot
     // of a use two (Y) or three (S) steps back, whose readers need only rows
     // issued before it.
-    if (lane == 0 && nph > 0) {
+    if (lane == 0) {
       bool ok = true;
+      uint32_t unit = blockIdx.x;
 #pragma unroll 1
-      for (int P = 0; ok && P < nph; ++P) {
-        int const f = P & 1;
-        long long const tile = blockIdx.x + (long long)(P >> 1) * gridDim.x;
+      for (int i = 0; ok; ++i) {
+        int const qs = i % kQueue;
+        if (!wait_or_fail(&sm.q_empty[qs], (uint32_t)(((i / kQueue) & 1) ^ 1), fail)) break;
+        *reinterpret_cast<volatile uint32_t*>(&sm.unit[qs]) = unit;
+        mbar_arrive(&sm.q_full[qs]);
+        if (unit >= nunits) break;
+        uint32_t const pi = unit / ntiles, tile = unit - pi * ntiles;
+        // the next unit: drawn while this one's rows are issued
+        unit = gridDim.x + atomicAdd(next_unit, 1u);
+        const float* __restrict__ x32 = tb.x32[pi];
 #pragma unroll 1
-        for (int bp = 0; ok && bp < 3; ++bp) {
+        for (int P = 2 * i; ok && P < 2 * i + 2; ++P) {
+          int const f = P & 1;
 #pragma unroll 1
-          for (int h = 0; ok && h < 2; ++h) {
-            int const uy = (P * 3 + bp) * 2 + h, ys = uy % kYSlots;
-            if (!wait_or_fail(&sm.y_empty[ys], (uint32_t)(((uy / kYSlots) & 1) ^ 1), fail)) { ok = false; break; }
-            fence_proxy_async_smem();
-            mbar_arrive_expect_tx(&sm.y_full[ys], kYRows * kRowBytes);
-            for (int r = 0; r < kYRows; ++r)
-              bulk_g2s(sm.Y[ys][r], row_ptr(y32, f, 4 * bp + 2 * h + r, tile), kRowBytes, &sm.y_full[ys]);
-            rows_issued_y = uy;
-          }
+          for (int bp = 0; ok && bp < 3; ++bp) {
 #pragma unroll 1
-          for (int bq = 0; ok && bq < kBlocksQ; ++bq) {
-            int const us = P * kBlocks + bp * kBlocksQ + bq, ss = us % kSGroups;
-            if (!wait_or_fail(&sm.s_empty[ss], (uint32_t)(((us / kSGroups) & 1) ^ 1), fail)) { ok = false; break; }
-            fence_proxy_async_smem();
-            mbar_arrive_expect_tx(&sm.s_full[ss], kRowsPerGroup * kRowBytes);
-            for (int r = 0; r < kRowsPerGroup; ++r)
-              bulk_g2s(sm.S[ss][r], row_ptr(x32, 1 - f, 4 * bq + r, tile), kRowBytes, &sm.s_full[ss]);
-            rows_issued_s = us;
+            for (int h = 0; ok && h < 2; ++h) {
+              int const uy = (P * 3 + bp) * 2 + h, ys = uy % kYSlots;
+              if (!wait_or_fail(&sm.y_empty[ys], (uint32_t)(((uy / kYSlots) & 1) ^ 1), fail)) { ok = false; break; }
+              fence_proxy_async_smem();
+              mbar_arrive_expect_tx(&sm.y_full[ys], kYRows * kRowBytes);
+              for (int r = 0; r < kYRows; ++r)
+                bulk_g2s(sm.Y[ys][r], row_ptr(y32, f, 4 * bp + 2 * h + r, tile), kRowBytes, &sm.y_full[ys]);
+              rows_issued_y = uy;
+            }
+#pragma unroll 1
+            for (int bq = 0; ok && bq < kBlocksQ; ++bq) {
+              int const us = P * kBlocks + bp * kBlocksQ + bq, ss = us % kSGroups;
+              if (!wait_or_fail(&sm.s_empty[ss], (uint32_t)(((us / kSGroups) & 1) ^ 1), fail)) { ok = false; break; }
+              fence_proxy_async_smem();
+              mbar_arrive_expect_tx(&sm.s_full[ss], kRowsPerGroup * kRowBytes);
+              for (int r = 0; r < kRowsPerGroup; ++r)
+                bulk_g2s(sm.S[ss][r], row_ptr(x32, 1 - f, 4 * bq + r, tile), kRowBytes, &sm.s_full[ss]);
+              rows_issued_s = us;
+            }
           }
         }
       }
     }
   } else if (warp == kWarpB) {
     // ---- B chunks -------------------------------------------------------------
-    if (lane == 0) {
-      int bc = 0;
-      bool ok = true;
+    constexpr int kBP = OpT<kF16>::kBParts;
+    int bc = 0;
+    bool ok = true;
+    uint32_t unit;
 #pragma unroll 1
-      for (int P = 0; ok && P < nph; ++P) {
-        constexpr int kBP = OpT<kF16>::kBParts;
+    for (int i = 0; ok && next(i, unit); ++i) {
+      uint32_t const pi = unit / ntiles;
+#pragma unroll 1
+      for (int f = 0; ok && f < 2; ++f) {
         const unsigned char* src =
-            static_cast<const unsigned char*>(btu) + ((size_t)pi * 2 + (P & 1)) * kChunks * kBP * Sm::kBPartB;
+            static_cast<const unsigned char*>(btu) + ((size_t)pi * 2 + f) * kChunks * kBP * Sm::kBPartB;
 #pragma unroll 1
         for (int c = 0; c < kChunks; ++c, ++bc) {
           int const st = bc % kSt;
           if (!wait_or_fail(&sm.a_empty[st], (uint32_t)(((bc / kSt) & 1) ^ 1), fail)) { ok = false; break; }
-          fence_proxy_async_smem();
-          mbar_arrive_expect_tx(&sm.b_full[st], kBP * Sm::kBPartB);
-          bulk_g2s(sm.B[st][0], src + (size_t)c * kBP * Sm::kBPartB, kBP * Sm::kBPartB, &sm.b_full[st]);
+          if (lane == 0) {
+            fence_proxy_async_smem();
+            mbar_arrive_expect_tx(&sm.b_full[st], kBP * Sm::kBPartB);
+            bulk_g2s(sm.B[st][0], src + (size_t)c * kBP * Sm::kBPartB, kBP * Sm::kBPartB, &sm.b_full[st]);
+          }
+          __syncwarp();
           b_issued = bc;
         }
       }
@@ -563,8 +597,10 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
       uint32_t aph = 0, bph = 0;
       uint32_t const dc = tmem + kCorrCol;
       bool ok = true;
+      uint32_t unit = 0;
 #pragma unroll 1
-      for (int P = 0; ok && P < nph; ++P) {
+      for (int P = 0; ok; ++P) {
+        if ((P & 1) == 0 && !next(P >> 1, unit)) break;
         // first half into main buffer P&1 (phase P-1's second half, free once
         // folded), second half into buffer (P+1)&1 (free once dotted)
         if (!wait_or_fail(&sm.folded, (uint32_t)((P & 1) ^ 1), fail)) break;
@@ -617,10 +653,21 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
     int const j = (warp - kWarpD0) % kDGroup;    // the chunk's j-th pair of (p, q)
     int const s = lane;
     bool ok = true;
+    uint32_t unit = 0, last_pi = 0xFFFFFFFFu;
+    int nvalid = 0;
+    float ascale0 = 1.f, ascale1 = 1.f;
 #pragma unroll 1
-    for (int P = 0; ok && P < nph; ++P) {
-      long long const tile = blockIdx.x + (long long)(P >> 1) * gridDim.x;
-      int const nvalid = (int)min((long long)kSites, geo.V - tile * kSites);
+    for (int P = 0; ok; ++P) {
+      if ((P & 1) == 0) {
+        if (!next(P >> 1, unit)) break;
+        uint32_t const pi = unit / ntiles, tile = unit - pi * ntiles;
+        nvalid = (int)min((long long)kSites, geo.V - (long long)tile * kSites);
+        if (kF16 && pi != last_pi) {
+          ascale0 = a_scale(pi, 0);
+          ascale1 = a_scale(pi, 1);
+          last_pi = pi;
+        }
+      }
 #pragma unroll 1
       for (int c = grp; c < kChunks; c += kDGroups) {
         // chunk c is half c & 1 of block b = (bp, bq): this warp's
@@ -745,26 +792,37 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
     int const quad = warp & 3;  // the TMEM lanes this warp may access; mu = quad
     int const s = lane;
     uint32_t const lane_addr = tmem + ((uint32_t)(quad * 32) << 16);
-    const int gsx[4] = {tb.gsx[pi][0], tb.gsx[pi][1], tb.gsx[pi][2], tb.gsx[pi][3]};
-    const int yv[4] = {tb.yv[pi][0], tb.yv[pi][1], tb.yv[pi][2], tb.yv[pi][3]};
-    const double* __restrict__ wq = kGeneric ? nullptr : args.w + (size_t)pi * geo.V * 3 * HLBL_QED_NW;
-    const float* __restrict__ cg =
-        kGeneric ? static_cast<const float*>(args.coef) + (size_t)pi * args.coef_stride : nullptr;
     double const xu = args.xunit;
     SiteQ q;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) q.ym[r] = (float)(coord_map(mod_pos(yv[r], geo.global[r]), geo.global[r]) * xu);
-    Neu run0, run1;
+    uint32_t unit = 0, pi = 0, tile = 0, last_pi = 0xFFFFFFFFu;
+    float inv0 = 1.f, inv1 = 1.f;  // FP16: the inverse scales per flavour (powers of two)
+    bool valid = false;
 #pragma unroll 1
-    for (int P = 0; P < nph; ++P) {
-      long long const tile = blockIdx.x + (long long)(P >> 1) * gridDim.x;
-      long long const v = tile * kSites + s;
-      bool const valid = v < geo.V;
+    for (int P = 0;; ++P) {
+      if ((P & 1) == 0) {
+        if (!next(P >> 1, unit)) break;
+        pi = unit / ntiles;
+        tile = unit - pi * ntiles;
+        valid = (long long)tile * kSites + s < geo.V;
+        if (pi != last_pi) {
+          if constexpr (kF16) {
+            inv0 = 1.f / (a_scale(pi, 0) * bscale[2 * pi]);
+            inv1 = 1.f / (a_scale(pi, 1) * bscale[2 * pi + 1]);
+          }
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            q.ym[r] = (float)(coord_map(mod_pos(tb.yv[pi][r], geo.global[r]), geo.global[r]) * xu);
+          last_pi = pi;
+        }
+      }
       if (!kGeneric && (P & 1) == 0) {
         // the row's site data, for both flavours of the tile
-        long long const vv = valid ? v : geo.V - 1;
+        const int gsx[4] = {tb.gsx[pi][0], tb.gsx[pi][1], tb.gsx[pi][2], tb.gsx[pi][3]};
+        const int yv[4] = {tb.yv[pi][0], tb.yv[pi][1], tb.yv[pi][2], tb.yv[pi][3]};
+        const double* __restrict__ wq = args.w + (size_t)pi * geo.V * 3 * HLBL_QED_NW;
+        long long const vv = valid ? (long long)tile * kSites + s : geo.V - 1;
         int rel[4];
-        rel_coords(geo, gsx, vv, rel);
+        rel_coords_fast(geo, gsx, vv, rel);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           q.xm[r] = (float)(coord_map(rel[r], geo.global[r]) * xu);
@@ -799,7 +857,8 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
       float a;
       if constexpr (kGeneric) {
         // the row (mu = quad, site s of the tile); pad sites' coefficients are zero
-        a = epilogue_row_generic(lane_addr, c0, cg + coef32_index(tile * kSites, quad, 0) + (size_t)s * 4);
+        const float* __restrict__ cg = static_cast<const float*>(args.coef) + (size_t)pi * args.coef_stride;
+        a = epilogue_row_generic(lane_addr, c0, cg + coef32_index((long long)tile * kSites, quad, 0) + (size_t)s * 4);
       } else {
         switch (quad) {
           case 0: a = epilogue_row<0>(lane_addr, c0, q); break;
@@ -811,27 +870,12 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.dotted);
-      if constexpr (kF16) a *= 1.f / (((P & 1) ? ascale1 : ascale0) * bscale[2 * pi + (P & 1)]);  // powers of two: exact
-      if (valid) {
-        if (P & 1) run1.add(-(double)a);
-        else run0.add(-(double)a);
-      }
-    }
-    if (!*fail) {
-      // fixed-order compensated reduction over the epilogue's 128 threads
-      Neu r0 = run0, r1 = run1;
+      if constexpr (kF16) a *= (P & 1) ? inv1 : inv0;  // a power of two: exact
+      // the quadrant's sum for this (tile, flavour), in a fixed order
+      double v = valid ? -(double)a : 0.0;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        double const s0v = __shfl_down_sync(0xffffffffu, r0.s, o), c0v = __shfl_down_sync(0xffffffffu, r0.c, o);
-        double const s1v = __shfl_down_sync(0xffffffffu, r1.s, o), c1v = __shfl_down_sync(0xffffffffu, r1.c, o);
-        r0.add(s0v); r0.c += c0v;
-        r1.add(s1v); r1.c += c1v;
-      }
-      if (lane == 0) {
-        int const ew = warp - kWarpE0;
-        sm.red[ew][0][0] = r0.s; sm.red[ew][0][1] = r0.c;
-        sm.red[ew][1][0] = r1.s; sm.red[ew][1][1] = r1.c;
-      }
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0) tsum[((size_t)unit * 2 + (P & 1)) * kEWarps + quad] = v;
     }
   }
 
@@ -854,12 +898,6 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
       mbar_wait(&sm.mma_done, 0);
     }
     if (t == 0 && err) atomicExch(err, kErrWaitTimeout);
-  } else if (t == kWarpE0 * 32) {
-    for (int f = 0; f < 2; ++f) {
-      Neu acc;
-      for (int w = 0; w < kEWarps; ++w) { acc.add(sm.red[w][f][0]); acc.c += sm.red[w][f][1]; }
-      partials[((size_t)pi * gridDim.x + blockIdx.x) * 2 + f] = acc.get();
-    }
   }
   __syncthreads();
   tc_fence_after();
@@ -941,6 +979,82 @@ __global__ void __launch_bounds__(256) btu_build_kernel(const double* __restrict
   }
 }
 
+// The pair's two sums from the tiles' (tsum[pair][tile][flavour][4]), in a fixed
+// order: a thread takes every (32 gridDim.x)-th tile's value of one (flavour,
+// quadrant), compensated, then the threads of a CTA, then the CTAs in order (by
+// the last one to finish). It also readies the counters of the next call.
+constexpr int kRedThreads = 256, kRedCtas = 64;
+__global__ void __launch_bounds__(kRedThreads)
+tile_reduce_kernel(const double* __restrict__ tsum, long long ntiles, double* __restrict__ part,
+                   unsigned* __restrict__ next_unit, unsigned* __restrict__ done, PairBatch batch, int add) {
+  __shared__ double rs[kRedThreads / 32][2], rc[kRedThreads / 32][2];
+  static_assert(kRedThreads == 256 && kRedCtas == 64, "one warp adds eight warps' and 64 CTAs' sums");
+  int const t = threadIdx.x, warp = t >> 5, lane = t & 31, pi = blockIdx.y;
+  tsum += (size_t)pi * ntiles * 8;
+  Neu a;
+  for (long long i = (long long)blockIdx.x * kRedThreads + t; i < ntiles * 8; i += (long long)gridDim.x * kRedThreads)
+    a.add(tsum[i]);
+  // lanes: bits 0, 1 the quadrant, bit 2 the flavour, bits 3, 4 the tile
+#pragma unroll
+  for (int o : {16, 8, 2, 1}) {
+    double const os = __shfl_xor_sync(0xffffffffu, a.s, o), oc = __shfl_xor_sync(0xffffffffu, a.c, o);
+    a.add(os);
+    a.c += oc;
+  }
+  if ((lane & ~4) == 0) {
+    rs[warp][lane >> 2] = a.s;
+    rc[warp][lane >> 2] = a.c;
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  // the warps' sums: lane 2 w + f
+  a = Neu();
+  if (lane < 2 * (kRedThreads / 32)) {
+    a.s = rs[lane >> 1][lane & 1];
+    a.c = rc[lane >> 1][lane & 1];
+  }
+#pragma unroll
+  for (int o : {8, 4, 2}) {
+    double const os = __shfl_xor_sync(0xffffffffu, a.s, o), oc = __shfl_xor_sync(0xffffffffu, a.c, o);
+    a.add(os);
+    a.c += oc;
+  }
+  if (gridDim.x > 1) {
+    double* const parts = part + (size_t)pi * kRedCtas * 4;
+    if (lane < 2) {
+      parts[blockIdx.x * 4 + lane * 2] = a.s;
+      parts[blockIdx.x * 4 + lane * 2 + 1] = a.c;
+      __threadfence();
+    }
+    __syncwarp();
+    int last = 0;
+    if (lane == 0) last = atomicAdd(done + pi, 1u) == gridDim.x - 1;
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __threadfence();
+    // the CTAs' sums: lane 2 i + f takes CTAs i, i + 16, i + 32, i + 48
+    a = Neu();
+    for (unsigned g = lane >> 1; g < gridDim.x; g += 16) {
+      a.add(__ldcg(parts + g * 4 + (lane & 1) * 2));
+      a.c += __ldcg(parts + g * 4 + (lane & 1) * 2 + 1);
+    }
+#pragma unroll
+    for (int o : {16, 8, 4, 2}) {
+      double const os = __shfl_xor_sync(0xffffffffu, a.s, o), oc = __shfl_xor_sync(0xffffffffu, a.c, o);
+      a.add(os);
+      a.c += oc;
+    }
+  }
+  if (lane < 2) {
+    double* out = batch.p[pi].out;
+    if (add) out[lane] += a.get();
+    else out[lane] = a.get();
+  }
+  if (lane == 0) {
+    done[pi] = 0u;
+    if (pi == 0) *next_unit = 0u;
+  }
+}
+
 }  // namespace tc
 
 size_t tc_smem_bytes() { return sizeof(tc::Smem); }
@@ -975,18 +1089,29 @@ void tc_launch_btu(const double* d_dz, int npairs, void* d_btu, bool f16, float*
   else tc::btu_build_kernel<false><<<gb, 256, 0, st>>>(d_dz, d_bscale, d_btu);
 }
 
-void tc_launch_p2(int grid, int npairs, cudaStream_t st, const TcBatch& tb, const Geometry& geo,
-                  const P2Args& a, const void* d_btu, bool f16, const float* d_bscale, double* partials, int* err) {
-  dim3 const gr(grid, npairs);
+void tc_launch_p2(int nsm, int npairs, cudaStream_t st, const TcBatch& tb, const Geometry& geo, const P2Args& a,
+                  const void* d_btu, bool f16, const float* d_bscale, double* tsum, unsigned* next_unit, int* err) {
+  long long const units = tc_tiles(geo.V) * npairs;
+  int const gr = (int)(units < nsm ? units : nsm);
   if (f16) {
     size_t const smem = sizeof(tc::SmemT<true>);
-    if (a.coef) tc::p2tc_kernel<true, true><<<gr, tc::kThreads, smem, st>>>(tb, geo, a, d_btu, d_bscale, partials, err);
-    else tc::p2tc_kernel<false, true><<<gr, tc::kThreads, smem, st>>>(tb, geo, a, d_btu, d_bscale, partials, err);
+    if (a.coef) tc::p2tc_kernel<true, true><<<gr, tc::kThreads, smem, st>>>(tb, geo, a, d_btu, d_bscale, npairs, tsum, next_unit, err);
+    else tc::p2tc_kernel<false, true><<<gr, tc::kThreads, smem, st>>>(tb, geo, a, d_btu, d_bscale, npairs, tsum, next_unit, err);
   } else {
     size_t const smem = sizeof(tc::SmemT<false>);
-    if (a.coef) tc::p2tc_kernel<true, false><<<gr, tc::kThreads, smem, st>>>(tb, geo, a, d_btu, d_bscale, partials, err);
-    else tc::p2tc_kernel<false, false><<<gr, tc::kThreads, smem, st>>>(tb, geo, a, d_btu, d_bscale, partials, err);
+    if (a.coef) tc::p2tc_kernel<true, false><<<gr, tc::kThreads, smem, st>>>(tb, geo, a, d_btu, d_bscale, npairs, tsum, next_unit, err);
+    else tc::p2tc_kernel<false, false><<<gr, tc::kThreads, smem, st>>>(tb, geo, a, d_btu, d_bscale, npairs, tsum, next_unit, err);
   }
+}
+
+size_t tc_tsum_len(long long V, int npairs) { return (size_t)tc_tiles(V) * npairs * 2 * tc::kEWarps; }
+
+void tc_launch_reduce(int npairs, cudaStream_t st, const Geometry& geo, const double* tsum, double* part,
+                      unsigned* next_unit, unsigned* done, const PairBatch& b, int add) {
+  long long const tiles = tc_tiles(geo.V);
+  // 64 tiles' sums per CTA (two per thread), up to 64 CTAs
+  int const g = (int)std::min<long long>(tc::kRedCtas, (tiles + 63) / 64);
+  tc::tile_reduce_kernel<<<dim3(g, npairs), tc::kRedThreads, 0, st>>>(tsum, tiles, part, next_unit, done, b, add);
 }
 
 long long tc_tiles(long long V) { return (V + tc::kSites - 1) / tc::kSites; }

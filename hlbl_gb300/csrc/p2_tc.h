@@ -40,8 +40,16 @@ int tc_init(int nsm, int& grid);
 // f16: FP16 operands (B built with a per-(pair, flavour) scale into
 // d_bscale[2 * pair + flavour]; the copies' trailers give A's scale)
 void tc_launch_btu(const double* d_dz, int npairs, void* d_btu, bool f16, float* d_bscale, cudaStream_t st);
-void tc_launch_p2(int grid, int npairs, cudaStream_t st, const TcBatch& tb, const Geometry& geo,
-                  const P2Args& a, const void* d_btu, bool f16, const float* d_bscale, double* partials, int* err);
+// per-tile sums into tsum (tc_tsum_len doubles); next_unit: the tile counter,
+// zero before the launch
+void tc_launch_p2(int nsm, int npairs, cudaStream_t st, const TcBatch& tb, const Geometry& geo, const P2Args& a,
+                  const void* d_btu, bool f16, const float* d_bscale, double* tsum, unsigned* next_unit, int* err);
+size_t tc_tsum_len(long long V, int npairs);
+// the pairs' sums from tsum; part: kTcRedPart doubles, done: kMaxBatch counters,
+// zero before the launch (left zero, as next_unit)
+constexpr int kTcRedPart = kMaxBatch * 64 * 4;
+void tc_launch_reduce(int npairs, cudaStream_t st, const Geometry& geo, const double* tsum, double* part,
+                      unsigned* next_unit, unsigned* done, const PairBatch& b, int add);
 long long tc_tiles(long long V);
 
 // Pass 1 on FP32 tile copies (p1_f32.cu); partials in p1_kernel's layout.
