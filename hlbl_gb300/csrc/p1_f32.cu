@@ -35,39 +35,55 @@ constexpr uint32_t kRowBytes = kRowFloats * 4;
 constexpr int kRowStride = kRowFloats + 4;
 template <int NFL> __host__ __device__ constexpr int rows() { return 24 * NFL; }   // (x, y) x flavours x 12
 template <int NFL> __host__ __device__ constexpr int threads() { return 144 * NFL; }
-template <int ST, int NFL> __host__ __device__ constexpr int min_ctas() { return NFL == 1 ? 3 : (ST == 1 ? 2 : 1); }
 
 // One tile's contribution of thread (fl, ia, ib): per site the eight
-// spin-block products and X_sigma; added into the Kahan accumulators.
-// The zerohalf weights zh_0..zh_2 are constant along a run of sites of
-// fixed (t, x, y) (z fastest), so per site only the run sums S_g = sum X_g and
-// T_g = sum zh_3 X_g are formed, and at the end of a run
+// spin-block products P[s1][s2] = sum_c conj(B[s1][c]) A[s2][c] enter the four
+// X_sigma only through
+//   al = P02 - P31, be = P13 - P20, ev = P03 + P21, od = P12 + P30:
+//   X_0 = -(al + be), X_1 = -i (ev + od), X_2 = od - ev, X_3 = i (be - al),
+// and the zerohalf weights zh_0..zh_2 are constant along a run of sites of
+// fixed (t, x, y) (z fastest), so per site only the run sums S of these four
+// and T of zh_3 times them are formed (32 additions and multiply-adds per site
+// besides the products, 64 with the X_sigma per site: 1.43 -> 1.21 ms per pair at
+// 663,552 sites), and at the end of a run
 //   dzu[(r,g)] += zh_r S_g - zh_g S_r  (g < 3),   zh_r S_3 - T_r  (g = 3),
-//   dzsu[g]    += S_g.
+//   dzsu[g]    += S_g
+// of the X_sigma go into the Kahan accumulators' tile sums.
 // z0: the tile's first site's local z, LZ: the local extent in z.
 __device__ __forceinline__ void tile_sums(const float* __restrict__ Arow, const float* __restrict__ Brow,
                                           const float (*zhs)[4], int nvalid, int z0, int LZ,
                                           KahanF (&acc_u)[6][2], KahanF (&acc_s)[4][2]) {
-  float tu[6][2], ts[4][2], S[4][2], T[4][2];
+  float tu[6][2], ts[4][2];
+  float2 S[4], T[4];  // al, be, ev, od as (re, im)
 #pragma unroll
   for (int k = 0; k < 6; ++k) tu[k][0] = tu[k][1] = 0.f;
 #pragma unroll
-  for (int g = 0; g < 4; ++g) ts[g][0] = ts[g][1] = S[g][0] = S[g][1] = T[g][0] = T[g][1] = 0.f;
+  for (int g = 0; g < 4; ++g) {
+    ts[g][0] = ts[g][1] = 0.f;
+    S[g] = T[g] = make_float2(0.f, 0.f);
+  }
+  auto to_x = [](const float2 q[4], float x[4][2]) {
+    x[0][0] = -(q[0].x + q[1].x); x[0][1] = -(q[0].y + q[1].y);
+    x[1][0] = q[2].y + q[3].y;    x[1][1] = -(q[2].x + q[3].x);
+    x[2][0] = q[3].x - q[2].x;    x[2][1] = q[3].y - q[2].y;
+    x[3][0] = q[0].y - q[1].y;    x[3][1] = q[1].x - q[0].x;
+  };
   auto flush = [&](const float* zh) {
+    float X[4][2], W[4][2];
+    to_x(S, X);
+    to_x(T, W);
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
       int const r = comb_rho(k), g = comb_sigma(k);
 #pragma unroll
       for (int c = 0; c < 2; ++c)
-        tu[k][c] += g == 3 ? zh[r] * S[3][c] - T[r][c] : zh[r] * S[g][c] - zh[g] * S[r][c];
+        tu[k][c] += g == 3 ? zh[r] * X[3][c] - W[r][c] : zh[r] * X[g][c] - zh[g] * X[r][c];
     }
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        ts[g][c] += S[g][c];
-        S[g][c] = T[g][c] = 0.f;
-      }
+      ts[g][0] += X[g][0];
+      ts[g][1] += X[g][1];
+      S[g] = T[g] = make_float2(0.f, 0.f);
     }
   };
   int z = z0;
@@ -86,39 +102,48 @@ __device__ __forceinline__ void tile_sums(const float* __restrict__ Arow, const 
       A[4 * c4] = a.x; A[4 * c4 + 1] = a.y; A[4 * c4 + 2] = a.z; A[4 * c4 + 3] = a.w;
       B[4 * c4] = b.x; B[4 * c4 + 1] = b.y; B[4 * c4 + 2] = b.z; B[4 * c4 + 3] = b.w;
     }
-    // P[s1][s2] = sum_c conj(B[s1][c]) A[s2][c] for s2 = s1^2 and 3-s1, as
-    // packed FP32 pairs: with y = (Re B, Im B), U = sum_c y Re A and
+    // products as packed FP32 pairs: with y = (Re B, Im B), U = sum_c y Re A and
     // V = sum_c y Im A (the A part broadcast to both halves), Re P = U.x + V.y
     // and Im P = V.x - U.y -- two packed FMAs per (c, s2) instead of four
-    float pa[4][2], pb[4][2];
-#pragma unroll
-    for (int s1 = 0; s1 < 4; ++s1) {
-      float2 ua = make_float2(0.f, 0.f), va = ua, ub = ua, vb = ua;
+    auto prod = [&](int s1, int s2, float2& u, float2& v) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         float2 const y = make_float2(B[2 * (3 * s1 + c)], B[2 * (3 * s1 + c) + 1]);
-        int const sa = 2 * (3 * (s1 ^ 2) + c), sb = 2 * (3 * (3 - s1) + c);
-        ua = __ffma2_rn(y, make_float2(A[sa], A[sa]), ua);
-        va = __ffma2_rn(y, make_float2(A[sa + 1], A[sa + 1]), va);
-        ub = __ffma2_rn(y, make_float2(A[sb], A[sb]), ub);
-        vb = __ffma2_rn(y, make_float2(A[sb + 1], A[sb + 1]), vb);
+        int const i = 2 * (3 * s2 + c);
+        u = __ffma2_rn(y, make_float2(A[i], A[i]), u);
+        v = __ffma2_rn(y, make_float2(A[i + 1], A[i + 1]), v);
       }
-      pa[s1][0] = ua.x + va.y; pa[s1][1] = va.x - ua.y;
-      pb[s1][0] = ub.x + vb.y; pb[s1][1] = vb.x - ub.y;
+    };
+    float2 const z2 = make_float2(zhs[s][3], zhs[s][3]);
+    auto add = [&](int g, float re, float im) {
+      S[g].x += re;
+      S[g].y += im;
+      T[g] = __ffma2_rn(z2, make_float2(re, im), T[g]);
+    };
+    float2 const zero = make_float2(0.f, 0.f);
+    {
+      float2 u = zero, v = zero, u2 = zero, v2 = zero;
+      prod(0, 2, u, v);
+      prod(3, 1, u2, v2);
+      add(0, (u.x + v.y) - (u2.x + v2.y), (v.x - u.y) - (v2.x - u2.y));
     }
-    float const z3 = zhs[s][3];
-#pragma unroll
-    for (int sg = 0; sg < 4; ++sg) {
-      float xr = 0, xi = 0;
-#pragma unroll
-      for (int s1 = 0; s1 < 4; ++s1) {
-        float const* pp = (sg == 0 || sg == 3) ? pa[s1] : pb[s1];
-        float vr, vi;
-        mul_iph(g5g_ph(sg, s1), pp[0], pp[1], vr, vi);
-        xr += vr; xi += vi;
-      }
-      S[sg][0] += xr; S[sg][1] += xi;
-      T[sg][0] = fmaf(z3, xr, T[sg][0]); T[sg][1] = fmaf(z3, xi, T[sg][1]);
+    {
+      float2 u = zero, v = zero, u2 = zero, v2 = zero;
+      prod(1, 3, u, v);
+      prod(2, 0, u2, v2);
+      add(1, (u.x + v.y) - (u2.x + v2.y), (v.x - u.y) - (v2.x - u2.y));
+    }
+    {
+      float2 u = zero, v = zero;
+      prod(0, 3, u, v);
+      prod(2, 1, u, v);
+      add(2, u.x + v.y, v.x - u.y);
+    }
+    {
+      float2 u = zero, v = zero;
+      prod(1, 2, u, v);
+      prod(3, 0, u, v);
+      add(3, u.x + v.y, v.x - u.y);
     }
   }
   if (nvalid > 0) flush(zhs[nvalid - 1]);
@@ -134,8 +159,11 @@ struct Smem {
   float zh[2][kTS][4];  // this tile's zero-half weights and the next one's
 };
 
+// 128 registers where more than one CTA is to be resident: 18 or 15 warps (a
+// bound in CTAs makes the compiler assume a worse spread of five warps over the
+// four schedulers: 96 registers and spills, 1.24 against 1.21 ms)
 template <int ST, int NFL>
-__global__ void __launch_bounds__(threads<NFL>(), min_ctas<ST, NFL>())
+__global__ void __maxnreg__((NFL == 1 || ST == 1) ? 128 : 168)
 p1f32_kernel(TcBatch tb, Geometry geo, double* __restrict__ partials, int* __restrict__ err) {
   constexpr int kRows = rows<NFL>();
   extern __shared__ __align__(128) unsigned char smem_raw[];
