@@ -113,8 +113,15 @@ __global__ void wait_timeout_selftest_kernel(int* err) {
 // FP64 block -> FP32 tile copy. A warp takes one (row, 32-site tile, 16-byte
 // group c4): lane = site of the tile, so each lane reads one 32-byte sector
 // of the block and the warp writes two contiguous 256-byte runs of the copy;
-// 32-bit index arithmetic (V * 6 < 2^31), blockIdx.y = row (f, ia).
-__global__ void f32_tile_copy_kernel(const double* __restrict__ blk, Geometry geo, float* __restrict__ out) {
+// 32-bit index arithmetic (V * 6 < 2^31), blockIdx.y = row (f, ia), blockIdx.z =
+// the block of the batch.
+struct CopyBatch {
+  const double* src[kMaxBatch + 1];
+  float* dst[kMaxBatch + 1];
+};
+__global__ void f32_tile_copy_kernel(CopyBatch cb, Geometry geo) {
+  const double* __restrict__ blk = cb.src[blockIdx.z];
+  float* __restrict__ out = cb.dst[blockIdx.z];
   unsigned const nt32 = (unsigned)((geo.V + 31) / 32), V = (unsigned)geo.V;
   unsigned const n = nt32 * 6 * 32;  // (tile, c4, lane)
   int const row = blockIdx.y;
@@ -139,6 +146,16 @@ __global__ void f32_tile_copy_kernel(const double* __restrict__ blk, Geometry ge
     atomicMax(reinterpret_cast<int*>(out + f32_tile_floats(geo.V)) + row / 12, __float_as_int(m));
 }
 
+// The copies' trailers, zeroed before their maxima are taken.
+__global__ void f32_trailer_zero_kernel(CopyBatch cb, Geometry geo) {
+  cb.dst[blockIdx.x][f32_tile_floats(geo.V) + threadIdx.x] = 0.f;
+}
+
+void launch_tile_copies(const CopyBatch& cb, int n, const Geometry& geo, int nsm, cudaStream_t st) {
+  f32_trailer_zero_kernel<<<n, kF32Trailer, 0, st>>>(cb, geo);
+  f32_tile_copy_kernel<<<dim3(std::max(1, nsm * 8 / 24), 24, n), 256, 0, st>>>(cb, geo);
+}
+
 // ---- launch plumbing -------------------------------------------------------
 template <int NF, int TS>
 struct P1Launch {
@@ -160,8 +177,8 @@ struct P1Launch {
     return HLBL_OK;
   }
   static void launch(int grid, cudaStream_t st, const double* y, const PairBatch& b,
-                     const Geometry& geo, int f0, double* partials, int* err, float* y32 = nullptr) {
-    p1_kernel<NF, TS><<<dim3(grid, b.n), threads, smem, st>>>(y, b, geo, f0, partials, err, y32);
+                     const Geometry& geo, int f0, double* partials, int* err) {
+    p1_kernel<NF, TS><<<dim3(grid, b.n), threads, smem, st>>>(y, b, geo, f0, partials, err);
   }
   static long long tiles(long long V) { return (V + TS - 1) / TS; }
 };
@@ -238,9 +255,9 @@ struct hlbl_ctx {
   int tc = 1;
   int grid_tc = 0;
   int grid_p1f[kP1f32Variants] = {};  // pass 1 on FP32 tile copies, per variant (p2_tc.h)
-  int p1f_var = 1;
+  int p1f_var = 2;            // one flavour per CTA: the fastest from 8,192 to 663,552 sites (p1_f32.cu)
   int group_f32 = 0;          // pairs per launch on the FP32-copy path (0: kMaxBatch)
-  float* d_x32 = nullptr;     // FP32 tile copies: [1 + pair][f32 block] (y first)
+  float* d_x32 = nullptr;     // FP32 tile copies of FP64 blocks: [1 + pair][f32 block] (y first)
   size_t x32_floats = 0;
   float* d_btu = nullptr;     // tensor-core B operand [kMaxBatch][tc_btu_floats_per_pair]
   float* d_bscale = nullptr;  // FP16 operands: B scale [kMaxBatch][2]
@@ -353,33 +370,30 @@ int ensure_x32(hlbl_ctx* c, const Geometry& geo, int npairs) {
 }
 float* x32_block(hlbl_ctx* c, const Geometry& geo, int slot) { return c->d_x32 + (size_t)slot * f32_block_floats(geo.V); }
 
+// Blocks staged on the side stream must have landed before what follows.
+int wait_staged(hlbl_ctx* c) {
+  if (!c->stage_pending) return HLBL_OK;
+  cudaError_t e = cudaStreamWaitEvent(c->stream, c->stage_ev, 0);
+  if (e != cudaSuccess) return cuda_fail(e, "wait for staged block");
+  c->stage_pending = false;
+  return HLBL_OK;
+}
+
 // Pass 1 + reduction + gamma insertion + Bt for the batch's pairs, flavours
 // [f0, f0+nf). Pair i, flavour fl: dz at d_dz + (i*nf + fl)*kDzLen, g at
 // d_g + (i*nf + fl)*kGLen, Bt at d_bt + (i*nf + fl)*kBtK*kBtN. The FP64 pass 2
 // takes dz itself, as dzq (quat_basis.cuh), instead of g and Bt.
 int run_pass1(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch& b, int f0,
               int nf, int precision, double* add_dzu, double* add_dzsu, bool build_bt) {
-  if (c->stage_pending) {  // blocks staged on the side stream must have landed
-    cudaError_t e = cudaStreamWaitEvent(c->stream, c->stage_ev, 0);
-    if (e != cudaSuccess) return cuda_fail(e, "wait for staged block");
-    c->stage_pending = false;
-  }
+  if (int rc = wait_staged(c)) return rc;
   int grid;
-  bool const tcp = use_tc(c, precision, nf) && build_bt;
-  PairBatch bb = b;
-  float* y32 = nullptr;
-  if (tcp) {
-    if (int rc = ensure_x32(c, geo, b.n)) return rc;
-    y32 = x32_block(c, geo, 0);
-    for (int i = 0; i < b.n; ++i) bb.p[i].src32 = x32_block(c, geo, 1 + i);
-  }
   prof_begin(c, 0);
   if (precision == HLBL_FP64) {
     grid = per_pair_grid(c->grid_p1d[nf - 1], b.n, p1f64_tiles(geo.V));
     p1f64_launch(nf, grid, c->stream, y, b, geo, f0, c->d_part1, c->d_err);
   } else {
-    if (nf == 2 && c->p1_small) { grid = per_pair_grid(c->grid_p1f2s, b.n, P1F2s::tiles(geo.V)); P1F2s::launch(grid, c->stream, y, bb, geo, f0, c->d_part1, c->d_err, y32); }
-    else if (nf == 2) { grid = per_pair_grid(c->grid_p1f2, b.n, P1F2::tiles(geo.V)); P1F2::launch(grid, c->stream, y, bb, geo, f0, c->d_part1, c->d_err, y32); }
+    if (nf == 2 && c->p1_small) { grid = per_pair_grid(c->grid_p1f2s, b.n, P1F2s::tiles(geo.V)); P1F2s::launch(grid, c->stream, y, b, geo, f0, c->d_part1, c->d_err); }
+    else if (nf == 2) { grid = per_pair_grid(c->grid_p1f2, b.n, P1F2::tiles(geo.V)); P1F2::launch(grid, c->stream, y, b, geo, f0, c->d_part1, c->d_err); }
     else { grid = per_pair_grid(c->grid_p1f1, b.n, P1F1::tiles(geo.V)); P1F1::launch(grid, c->stream, y, b, geo, f0, c->d_part1, c->d_err); }
   }
   prof_end(c, 0);
@@ -388,10 +402,6 @@ int run_pass1(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch
   if (!build_bt) return HLBL_OK;
   if (precision == HLBL_FP64) {
     p2f64_launch_dzq(c->d_dz, nullptr, nullptr, nf, b.n, c->d_dzq, nullptr, c->stream);
-    return HLBL_OK;
-  }
-  if (tcp) {
-    tc_launch_btu(c->d_dz, b.n, c->d_btu, false, nullptr, c->stream);
     return HLBL_OK;
   }
   g_build_kernel<<<dim3((kGLen / 2 + 255) / 256, nf, b.n), 256, 0, c->stream>>>(c->d_dz, nf, c->d_g);
@@ -520,25 +530,12 @@ int run_pass2(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch
   a.xunit = xunit;
   a.f0 = f0;
   int grid;
-  if (use_tc(c, precision, nf))
-    if (int rc = ensure_tsum(c, geo, b.n)) return rc;
   prof_begin(c, 1);
   if (precision == HLBL_FP64) {
     grid = per_pair_grid(c->grid_p2d[nf - 1], b.n, p2f64_tiles(geo.V));
     p2f64_launch(nf, grid, c->stream, y, b, geo, a, c->d_dzq, c->d_part2, c->d_err, bad);
     if (bad != nullptr)  // the same partials, from the other kernel
       P2D1::launch(grid, c->stream, y, b, geo, a, static_cast<const double*>(c->d_bt), c->d_part2, c->d_err, bad);
-  } else if (use_tc(c, precision, nf)) {
-    TcBatch tb{};
-    tb.y32 = x32_block(c, geo, 0);
-    for (int i = 0; i < b.n; ++i) {
-      tb.x32[i] = x32_block(c, geo, 1 + i);
-      for (int r = 0; r < 4; ++r) { tb.gsx[i][r] = b.p[i].gsx[r]; tb.yv[i][r] = b.p[i].yv[r]; }
-    }
-    tc_launch_p2(c->grid_tc, b.n, c->stream, tb, geo, a, c->d_btu, false, nullptr, c->d_tsum, c->d_tcnt, c->d_err);
-    prof_end(c, 1);
-    tc_launch_reduce(b.n, c->stream, geo, c->d_tsum, c->d_tred, c->d_tcnt, c->d_tcnt + 1, b, add);
-    return HLBL_OK;
   } else {
     const float* bt = static_cast<const float*>(c->d_bt);
     if (nf == 2 && c->p2_small) { grid = per_pair_grid(c->grid_p2f2s, b.n, P2F2s::tiles(geo.V)); P2F2s::launch(grid, c->stream, y, b, geo, a, bt, c->d_part2, c->d_err); }
@@ -553,13 +550,8 @@ int run_pass2(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch
 // The FP32-copy path for one pair group: pass 1 on the copies, reduction,
 // gamma insertion, the tensor-core B operand, the weights and the
 // tensor-core pass 2 (b gives outputs and coordinates; tb the copies).
-int run_group_f32(hlbl_ctx* c, const PairBatch& b, const TcBatch& tb, double xunit) {
-  if (c->stage_pending) {
-    cudaError_t e = cudaStreamWaitEvent(c->stream, c->stage_ev, 0);
-    if (e != cudaSuccess) return cuda_fail(e, "wait for staged block");
-    c->stage_pending = false;
-  }
-  Geometry const& geo = c->geo;
+int run_group_f32(hlbl_ctx* c, const Geometry& geo, const PairBatch& b, const TcBatch& tb, double xunit) {
+  if (int rc = wait_staged(c)) return rc;
   int const v = c->p1f_var;
   int const g1 = per_pair_grid(c->grid_p1f[v], b.n, p1f32_tiles(geo.V));
   prof_begin(c, 0);
@@ -578,6 +570,31 @@ int run_group_f32(hlbl_ctx* c, const PairBatch& b, const TcBatch& tb, double xun
   prof_end(c, 1);
   tc_launch_reduce(b.n, c->stream, geo, c->d_tsum, c->d_tred, c->d_tcnt, c->d_tcnt + 1, b, 0);
   return HLBL_OK;
+}
+
+// The tensor-core path for one pair group on FP64 blocks: their FP32 tile
+// copies (of y only with the first group of a call), then as above. The copies
+// run at the HBM rate (0.72 ms for 3.06 GB), pass 1 converting the blocks as it
+// read them did not (131,072 sites, four pairs: 2.74 ms with the conversion,
+// 0.69 + 0.95 ms apart), and the copies carry the maxima that FP16 operands need.
+int run_blocks_f32(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch& b, bool copy_y, double xunit) {
+  if (int rc = wait_staged(c)) return rc;
+  CopyBatch cb{};
+  TcBatch tb{};
+  int n = 0;
+  tb.y32 = x32_block(c, geo, 0);
+  if (copy_y) {
+    cb.src[n] = y;
+    cb.dst[n++] = x32_block(c, geo, 0);
+  }
+  for (int i = 0; i < b.n; ++i) {
+    tb.x32[i] = x32_block(c, geo, 1 + i);
+    cb.src[n] = b.p[i].src;
+    cb.dst[n++] = x32_block(c, geo, 1 + i);
+    for (int r = 0; r < 4; ++r) { tb.gsx[i][r] = b.p[i].gsx[r]; tb.yv[i][r] = b.p[i].yv[r]; }
+  }
+  launch_tile_copies(cb, n, geo, c->nsm, c->stream);
+  return run_group_f32(c, geo, b, tb, xunit);
 }
 
 PairBatch one_pair(const double* src, double* out, const int gsx[4], const int yv[4]) {
@@ -752,8 +769,13 @@ int hlbl_kernel_sum_async(hlbl_ctx* c, const double* src, const double* y, const
   for (int r = 0; r < 4; ++r)
     if (gsx[r] < 0 || gsx[r] >= c->geo.global[r]) return fail(HLBL_EINVAL, "hlbl_kernel_sum: gsx[%d] = %d outside [0, %d)", r, gsx[r], c->geo.global[r]);
   PairBatch const b = one_pair(src, d_out, gsx, yv);
-  if (int rc = run_pass1(c, c->geo, y, b, 0, 2, precision, nullptr, nullptr, true)) return rc;
-  if (int rc = run_pass2(c, c->geo, y, b, xunit, 0, 2, precision, 0)) return rc;
+  if (use_tc(c, precision, 2)) {
+    if (int rc = ensure_x32(c, c->geo, 1)) return rc;
+    if (int rc = run_blocks_f32(c, c->geo, y, b, true, xunit)) return rc;
+  } else {
+    if (int rc = run_pass1(c, c->geo, y, b, 0, 2, precision, nullptr, nullptr, true)) return rc;
+    if (int rc = run_pass2(c, c->geo, y, b, xunit, 0, 2, precision, 0)) return rc;
+  }
   return check_launch("hlbl_kernel_sum launch");
 }
 
@@ -791,7 +813,7 @@ int hlbl_kernel_sums_batched_f32(hlbl_ctx* c, const float* y32, int n, const flo
         b.p[i].yv[r] = tb.yv[i][r] = yv[4 * (i0 + i) + r];
       }
     }
-    if (int rc = run_group_f32(c, b, tb, xunit)) return rc;
+    if (int rc = run_group_f32(c, c->geo, b, tb, xunit)) return rc;
   }
   return check_launch("hlbl_kernel_sums_batched_f32 launch");
 }
@@ -851,6 +873,9 @@ int hlbl_kernel_sums_batched(hlbl_ctx* c, const double* y, int n, const double* 
         return fail(HLBL_EINVAL, "hlbl_kernel_sums_batched: gsx of pair %d outside the lattice", i);
   }
   int const group = c->batch_group > 0 ? std::min(c->batch_group, kMaxBatch) : kMaxBatch;
+  bool const tc = use_tc(c, precision, 2);
+  if (tc && n > 0)
+    if (int rc = ensure_x32(c, c->geo, std::min(n, group))) return rc;
   for (int i0 = 0; i0 < n; i0 += group) {
     PairBatch b{};
     b.n = std::min(group, n - i0);
@@ -862,6 +887,10 @@ int hlbl_kernel_sums_batched(hlbl_ctx* c, const double* y, int n, const double* 
         b.p[i].yv[r] = yv[4 * (i0 + i) + r];
       }
     }
+    if (tc) {
+      if (int rc = run_blocks_f32(c, c->geo, y, b, i0 == 0, xunit)) return rc;
+      continue;
+    }
     if (int rc = run_pass1(c, c->geo, y, b, 0, 2, precision, nullptr, nullptr, true)) return rc;
     if (int rc = run_pass2(c, c->geo, y, b, xunit, 0, 2, precision, 0)) return rc;
   }
@@ -871,14 +900,11 @@ int hlbl_kernel_sums_batched(hlbl_ctx* c, const double* y, int n, const double* 
 int hlbl_f32_tile_copy(hlbl_ctx* c, const double* d_block, float* d_out) {
   if (!c || !d_block || !d_out) return fail(HLBL_EINVAL, "hlbl_f32_tile_copy: null argument");
   if (!aligned16(d_block) || !aligned16(d_out)) return fail(HLBL_EINVAL, "hlbl_f32_tile_copy: pointers must be 16-byte aligned");
-  if (c->stage_pending) {  // a block staged on the side stream must have landed
-    cudaError_t e = cudaStreamWaitEvent(c->stream, c->stage_ev, 0);
-    if (e != cudaSuccess) return cuda_fail(e, "wait for staged block");
-    c->stage_pending = false;
-  }
-  cudaError_t e = cudaMemsetAsync(d_out + f32_tile_floats(c->geo.V), 0, kF32Trailer * sizeof(float), c->stream);
-  if (e != cudaSuccess) return cuda_fail(e, "hlbl_f32_tile_copy trailer");
-  f32_tile_copy_kernel<<<dim3(std::max(1, c->nsm * 8 / 24), 24), 256, 0, c->stream>>>(d_block, c->geo, d_out);
+  if (int rc = wait_staged(c)) return rc;
+  CopyBatch cb{};
+  cb.src[0] = d_block;
+  cb.dst[0] = d_out;
+  launch_tile_copies(cb, 1, c->geo, c->nsm, c->stream);
   return check_launch("hlbl_f32_tile_copy launch");
 }
 
@@ -1104,6 +1130,10 @@ int hlbl_reserve_kernel_memory(hlbl_ctx* c, size_t* bytes) {
     for (int prec : {HLBL_FP64, HLBL_FP32}) {
       for (int nf : {1, 2}) {
         PairBatch const b = one_pair(blk, c->d_out, zero, one);
+        if (use_tc(c, prec, nf)) {
+          if (ensure_x32(c, geo, 1) == HLBL_OK) run_blocks_f32(c, geo, blk, b, true, 1.0);
+          continue;
+        }
         run_pass1(c, geo, blk, b, 0, nf, prec, nullptr, nullptr, true);
         run_pass2(c, geo, blk, b, 1.0, 0, nf, prec, 0);
       }

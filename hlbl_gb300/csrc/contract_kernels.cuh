@@ -32,7 +32,6 @@ constexpr int kMaxBatch = 16;
 struct PairDesc {
   const double* src;  // the partner's block (the pair's x = gsx)
   double* out;        // its two kernel sums (pass 2 reduction target)
-  float* src32;       // FP32 path: pass 1 writes the block's FP32 tile copy here (or null)
   int gsx[4];
   int yv[4];
 };
@@ -121,36 +120,6 @@ __device__ __forceinline__ void load_row(const float* __restrict__ p, float r[24
 }
 
 
-// Pass 1's FP32 path: convert a landed FP64 stage into the FP32 compute copy
-// and, in the same pass, into the FP32 tile copies (y32 by pair 0's CTAs).
-// One unit = (row, 16-byte group c4, site); consecutive threads take
-// consecutive sites, so the global stores of 8 threads cover 128 contiguous
-// bytes.
-template <int NF, int TS>
-__device__ __forceinline__ void convert_and_copy(const double* __restrict__ st, float* __restrict__ cp,
-                                                 float* __restrict__ a32, float* __restrict__ b32, int f0,
-                                                 long long V, long long s0, int nvalid) {
-  static_assert(32 % TS == 0, "a tile lies inside one 32-site tile of the copy");
-  constexpr int kRows = 2 * NF * 12, RS = row_stride<float, TS>();
-  long long const nt32 = (V + 31) / 32;
-  for (int u = threadIdx.x; u < kRows * 6 * TS; u += blockDim.x) {
-    int const si = u % TS, c4 = (u / TS) % 6, row = u / (6 * TS);
-    if (si >= nvalid) continue;
-    const double2* src = reinterpret_cast<const double2*>(st + ((size_t)row * TS + si) * 24 + 4 * c4);
-    double2 const v0 = src[0], v1 = src[1];
-    float4 const f = make_float4(f64_to_f32(v0.x), f64_to_f32(v0.y), f64_to_f32(v1.x), f64_to_f32(v1.y));
-    *reinterpret_cast<float4*>(cp + (size_t)row * RS + si * 24 + 4 * c4) = f;
-    int const which = row / (NF * 12), fl = (row / 12) % NF, ia = row % 12;
-    float* dst = which == 0 ? a32 : b32;
-    if (dst != nullptr) {
-      int const ff = which == 0 ? f0 + fl : 1 - f0 - fl;
-      long long const v = s0 + si;
-      *reinterpret_cast<float4*>(dst + ((size_t)(ff * 12 + ia) * nt32 + (size_t)(v >> 5)) * (32 * 24) +
-                                 f32_tile_off((int)(v & 31), c4)) = f;
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Pass 1 (ker_dzu_dzsu, cuda_lattice.cu:160-262), per CTA partial sums.
 // Thread (fl, ia, ib) owns dzu[k][ia][ib] and dzsu[s][ia][ib] of flavour
@@ -160,14 +129,12 @@ __device__ __forceinline__ void convert_and_copy(const double* __restrict__ st, 
 // X_s is assembled from the eight spin-block products
 //   P[s1][s2] = sum_c conj(B[s1][c]) A[s2][c],  s2 = src(s, s1),
 // which is all of g5 g_s's support. On FP64 blocks with FP32 products (the FP64
-// products are p1_f64.cu's), accumulated per tile in FP32, then into
-// compensated FP32 sums. As it converts a tile, pass 1 also writes it into the
-// FP32 tile copies the tensor-core pass 2 reads (y32 by pair 0's CTAs, each
-// partner's by its own; null pointers: no copy).
+// products are p1_f64.cu's; on FP32 tile copies p1_f32.cu's), accumulated per
+// tile in FP32, then into compensated FP32 sums: pass 1 of the CUDA-core path.
 template <int NF, int TS>
 __global__ void __launch_bounds__(NF * 144, 2)
 p1_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0,
-          double* __restrict__ partials, int* __restrict__ err, float* __restrict__ y32) {
+          double* __restrict__ partials, int* __restrict__ err) {
   constexpr int kRows = 2 * NF * 12;
   using T = float;
   constexpr size_t kStage = (size_t)kRows * TS * 24;  // doubles of the stage
@@ -235,7 +202,7 @@ p1_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0,
     __syncthreads();
     if (s_fail) break;
     // convert once, then the stage takes the next tile while we compute
-    convert_and_copy<NF, TS>(s_stage, s_copy, batch.p[pi].src32, pi == 0 ? y32 : nullptr, f0, geo.V, s0, nvalid);
+    convert_stage<NF, TS>(s_stage, s_copy);
     __syncthreads();
     if (t == 0 && tile + gridDim.x < ntiles) {
       fence_proxy_async_smem();

@@ -41,8 +41,7 @@
 //   commit per chunk frees both stages,
 //   MMA -> epilogue (acc_full), epilogue -> MMA (folded, dotted).
 //
-// Inputs are the FP32 tile copies pass 1 writes while it converts each
-// block (x32/y32: [f][ia][tile][2][6][16][4] floats, f32_tile_off: a site's
+// Inputs are the FP32 tile copies of the blocks (x32/y32: [f][ia][tile][2][6][16][4] floats, f32_tile_off: a site's
 // 24 components as six 16-byte groups, 32 sites per tile in two halves), so
 // pass 2 reads half the bytes of the FP64 blocks and converts nothing.
 #include <cuda_fp16.h>

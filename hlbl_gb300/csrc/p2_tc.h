@@ -9,9 +9,8 @@
 
 namespace hg {
 
-// FP32 tile copies of a propagator block, written by pass 1 (FP32 path) or
-// hlbl_f32_tile_copy and read by the tensor-core pass 2 and the FP32-input
-// pass 1: [f][ia][tile][2][6][16][4] floats (f32_tile_off), tiles of 32
+// FP32 tile copies of a propagator block (f32_tile_copy_kernel), read by the
+// tensor-core pass 2 and the FP32-input pass 1: [f][ia][tile][2][6][16][4] floats (f32_tile_off), tiles of 32
 // sites in two halves (the last tile padded), a site's 24 sink components as
 // six 16-byte groups.
 // A copy ends with a trailer of kF32Trailer floats: [0] and [1] hold the

@@ -113,7 +113,7 @@ int hlbl_stage_async(hlbl_ctx* ctx, void* d_dst, const void* h_src, size_t bytes
                      int after_compute);
 
 /* Autotuner: times one batch (FP32 products) under each FP32 variant of
- * pass 1 (best_p1: 0 = tiles of 8 sites, 1 = 4) and pass 2 (best_p2:
+ * pass 1 on the CUDA-core path (best_p1: 0 = tiles of 8 sites, 1 = 4) and pass 2 (best_p2:
  * 0 = CUDA cores, tiles of 4 sites; 1 = CUDA cores, 2 sites; 2 = tensor
  * cores) and each batch group (1, 2, 4, 8, 16 pairs per launch) and keeps
  * the fastest in the context. Writes the sums of the last trial to d_out.
@@ -122,8 +122,8 @@ int hlbl_autotune(hlbl_ctx* ctx, const double* d_fwd_y, int n, const double* con
                   const int* gsx, const int* yv, double xunit, double* d_out, int* best_p1,
                   int* best_p2, int* best_group, double* best_ms);
 
-/* The FP32 tile copy of a block that pass 1 of the FP32 path writes and the
- * tensor-core pass 2 and hlbl_kernel_sums_batched_f32 read:
+/* The FP32 tile copy of a block that the tensor-core path and
+ * hlbl_kernel_sums_batched_f32 read:
  * d_out[f][ia][tile][half][6][16][4] floats, tiles of 32 sites ((V + 31) / 32
  * of them, the last padded and its pad left untouched) in two halves of 16, a
  * site's 24 sink components as six groups of 4; each value rounded to
@@ -167,13 +167,14 @@ int hlbl_ctx_set_p1f32_variant(hlbl_ctx* ctx, int variant, int group);
 int hlbl_ctx_set_qed_fp32(hlbl_ctx* ctx, int on, double r64);
 
 /* FP32 two-flavour pass 2 on the tensor cores (on = 1, the default:
- * tcgen05 MMAs with split hi + lo products, FP32 tile copies of the blocks
- * written by pass 1 or by hlbl_f32_tile_copy; the operand type as
- * hlbl_ctx_set_tc_fp16 sets it, TF32 for FP64 blocks) or on the CUDA cores
- * (on = 0). No counterpart in the reference. */
+ * tcgen05 MMAs with split hi + lo products on FP32 tile copies of the blocks,
+ * which a call on FP64 blocks makes in the context's own buffers; the operand
+ * type as hlbl_ctx_set_tc_fp16 sets it) or on the CUDA cores (on = 0). No
+ * counterpart in the reference. */
 int hlbl_ctx_set_tensor_cores(hlbl_ctx* ctx, int on);
 
-/* Operands of the FP32-copy path's tensor-core pass 2 (hlbl_kernel_sums_batched_f32):
+/* Operands of the tensor-core pass 2 (hlbl_kernel_sums_batched_f32, and the FP32
+ * kernel sums of FP64 blocks):
  * on = 1 (the default), FP16: the same hi + lo split as 3xTF32 (22
  * significant bits) in half the bytes and half the MMAs, with power-of-two
  * scales from the largest magnitudes the tile copies carry, so the copies
