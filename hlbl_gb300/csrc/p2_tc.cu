@@ -14,8 +14,8 @@
 //   0      TMA producer of the FP32 input rows (S = x[1-f] rows q, Y = y[f]
 //          rows p: 3 KB per (flavour, ia, tile)) -- one thread
 //   1      TMA producer of the B chunks (16 k x 160 n, hi and lo, 20 KB) -- one thread
-//   2      TMEM allocation; tcgen05.mma issue and commits -- one thread
-//   3-14   D formation, three groups of four warps on every third chunk of
+//   3      TMEM allocation; tcgen05.mma issue and commits
+//   2, 4-14  D formation, three groups of four warps on every third chunk of
 //          16 k (8 (p, q): half of a block of 4 p x 4 q): warp j of a group
 //          forms the chunk's j-th pair of (p, q) (one Y row, two S rows) for
 //          its lane's site: O = Y conj(S) spin blocks -> D_mu -> hi/lo ->
@@ -37,8 +37,8 @@
 // Pipelines (mbarriers; every wait bounded, kWaitLimit polls):
 //   rows -> D warps (S rows of a block in a ring of 2 blocks, Y rows of a
 //   p-block by halves in a ring of 3),
-//   D warps -> MMA (A ring of 5), B producer -> MMA (B ring of 5), one
-//   commit per chunk frees both stages,
+//   D warps and B producer -> MMA (operand stages, a ring of 5 or 6: one
+//   barrier per stage, one commit per chunk frees it),
 //   MMA -> epilogue (acc_full), epilogue -> MMA (folded, dotted).
 //
 // Inputs are the FP32 tile copies of the blocks (x32/y32: [f][ia][tile][2][6][16][4] floats, f32_tile_off: a site's
@@ -82,10 +82,12 @@ constexpr int kHalf = kChunks / 2;               // chunks per main-accumulator 
 constexpr uint32_t kCorrCol = 2 * kBtN;          // the correction accumulator's first column
 constexpr int kAPart = kM * kKc;           // floats per A part (hi or lo)
 constexpr int kBPart = kBtN * kKc;         // floats per B part
-constexpr int kWarpRows = 0, kWarpB = 1, kWarpMma = 2, kWarpD0 = 3, kDWarps = 12;
+// The MMA warp shares its scheduler (warp % 4) with the fewest others: of 19
+// warps the fourth scheduler has four. D warps: 2 and 4-14.
+constexpr int kWarpRows = 0, kWarpB = 1, kWarpMma = 3, kDWarps = 12;
 constexpr int kDGroup = 4;  // D warps per chunk (a group); kDGroups chunks in flight
 constexpr int kDGroups = kDWarps / kDGroup;
-constexpr int kWarpE0 = kWarpD0 + kDWarps, kEWarps = 4;
+constexpr int kWarpE0 = 3 + kDWarps, kEWarps = 4;
 constexpr int kThreads = 32 * (kWarpE0 + kEWarps);
 // The CTAs take their units (pair, tile) from a common counter: at 663,552
 // sites the same number of tiles each took 2.50 to 3.45 ms (both SMs of a TPC
@@ -140,12 +142,12 @@ struct __align__(1024) SmemT {
   __align__(16) unsigned char A[kSt][2][kAPartB];
   __align__(16) unsigned char B[kSt][OpT<F16>::kBParts][kBPartB];
   uint64_t s_full[kSGroups], s_empty[kSGroups], y_full[kYSlots], y_empty[kYSlots];
-  uint64_t a_full[kSt], b_full[kSt], a_empty[kSt], b_empty[kSt];
+  uint64_t full[kSt], empty[kSt];  // operand stages: A by a D group, B by its copy
   uint64_t acc_full, folded, dotted, mma_done;
   uint64_t q_full[kQueue], q_empty[kQueue];
   uint32_t unit[kQueue];  // the queue of this CTA's (pair, tile) units
   uint32_t taddr;
-  int fail;
+  int fail, b_last;
 };
 using Smem = SmemT<false>;
 static_assert(sizeof(SmemT<false>) <= 232448 && sizeof(SmemT<true>) <= 232448,
@@ -200,11 +202,23 @@ __device__ __forceinline__ void mma_tf32(uint32_t d, uint64_t a, uint64_t b, uin
       " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}" ::"r"(d),
       "l"(a), "l"(b), "r"(kIdesc), "r"(acc));
 }
-__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+// The four products of a chunk (hi.hi into d; hi.lo, lo.hi and hi.lo2 into dc)
+// and the commit that frees its stage, issued by one elected lane of the
+// converged warp: predicated instructions, no branch.
+__device__ __forceinline__ void mma_chunk_f16(uint32_t d, uint32_t dc, uint64_t ahi, uint64_t alo, uint64_t bhi,
+                                              uint64_t b_part, uint32_t acc_d, uint32_t acc_c, uint64_t* bar) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc<true>()), "r"(acc));
+      "{\n .reg .pred p, q, r, t;\n"
+      " elect.sync _|p, 0xffffffff;\n"
+      " setp.ne.b32 q, %7, 0;\n setp.ne.b32 r, %8, 0;\n setp.eq.b32 t, 0, 0;\n"
+      " @p tcgen05.mma.cta_group::1.kind::f16 [%0], %2, %4, %9, q;\n"
+      " @p tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %5, %9, r;\n"
+      " @p tcgen05.mma.cta_group::1.kind::f16 [%1], %3, %4, %9, t;\n"
+      " @p tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %6, %9, t;\n"
+      " @p tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%10];\n}" ::"r"(d),
+      "r"(dc), "l"(ahi), "l"(alo), "l"(bhi), "l"(bhi + b_part), "l"(bhi + 2 * b_part), "r"(acc_d), "r"(acc_c),
+      "r"(idesc<true>()), "r"(smem_u32(bar))
+      : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -456,8 +470,7 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
   if (t == 0) {
     for (int i = 0; i < kSGroups; ++i) { mbar_init(&sm.s_full[i], 1); mbar_init(&sm.s_empty[i], 2 * kDGroup); }
     for (int i = 0; i < kYSlots; ++i) { mbar_init(&sm.y_full[i], 1); mbar_init(&sm.y_empty[i], kDGroups * kDGroup); }
-    for (int i = 0; i < kSt; ++i) { mbar_init(&sm.a_full[i], kDGroup); mbar_init(&sm.a_empty[i], 1); }
-    for (int i = 0; i < kSt; ++i) { mbar_init(&sm.b_full[i], 1); mbar_init(&sm.b_empty[i], 1); }
+    for (int i = 0; i < kSt; ++i) { mbar_init(&sm.full[i], kDGroup + 1); mbar_init(&sm.empty[i], 1); }
     mbar_init(&sm.acc_full, 1);
     mbar_init(&sm.folded, kEWarps);
     mbar_init(&sm.dotted, kEWarps);
@@ -495,6 +508,7 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
   // issue tracking for the teardown after a failure
   int rows_issued_s = -1, rows_issued_y = -1;  // last S block / Y p-block use issued
   int b_issued = -1;
+  int d_next = -1;  // D warps: the next chunk of this warp's group
   bool mma_any = false;
 
   if (warp == kWarpRows) {
@@ -562,11 +576,11 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
 #pragma unroll 1
         for (int c = 0; c < kChunks; ++c, ++bc) {
           int const st = bc % kSt;
-          if (!wait_or_fail(&sm.a_empty[st], (uint32_t)(((bc / kSt) & 1) ^ 1), fail)) { ok = false; break; }
+          if (!wait_or_fail(&sm.empty[st], (uint32_t)(((bc / kSt) & 1) ^ 1), fail)) { ok = false; break; }
           if (lane == 0) {
             fence_proxy_async_smem();
-            mbar_arrive_expect_tx(&sm.b_full[st], kBP * Sm::kBPartB);
-            bulk_g2s(sm.B[st][0], src + (size_t)c * kBP * Sm::kBPartB, kBP * Sm::kBPartB, &sm.b_full[st]);
+            mbar_arrive_expect_tx(&sm.full[st], kBP * Sm::kBPartB);
+            bulk_g2s(sm.B[st][0], src + (size_t)c * kBP * Sm::kBPartB, kBP * Sm::kBPartB, &sm.full[st]);
           }
           __syncwarp();
           b_issued = bc;
@@ -592,8 +606,8 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
       constexpr uint64_t kAStage16 = 2 * Sm::kAPartB / 16, kALo16 = Sm::kAPartB / 16, kAK16 = 2 * (kM / 8) * 128 / 16;
       constexpr uint64_t kBStage16 = OpT<kF16>::kBParts * Sm::kBPartB / 16, kBLo16 = Sm::kBPartB / 16,
                          kBK16 = 2 * (kBtN / 8) * 128 / 16;
-      int as = 0, bs = 0;
-      uint32_t aph = 0, bph = 0;
+      int as = 0;
+      uint32_t aph = 0;
       uint32_t const dc = tmem + kCorrCol;
       bool ok = true;
       uint32_t unit = 0;
@@ -611,35 +625,32 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
             if (!wait_or_fail(&sm.dotted, (uint32_t)((P & 1) ^ 1), fail)) { ok = false; break; }
             tc_fence_after();
           }
-          if (!wait_or_fail(&sm.a_full[as], aph, fail) || !wait_or_fail(&sm.b_full[bs], bph, fail)) {
+          if (!wait_or_fail(&sm.full[as], aph, fail)) {
             ok = false;
             break;
           }
           tc_fence_after();
           uint32_t const d = c < kHalf ? d0 : d1;
-          uint64_t const ahi = a_desc0 + (uint64_t)as * kAStage16, bhi = b_desc0 + (uint64_t)bs * kBStage16;
+          uint64_t const ahi = a_desc0 + (uint64_t)as * kAStage16, bhi = b_desc0 + (uint64_t)as * kBStage16;
           // hi.hi into the main buffer, hi.lo and lo.hi into the correction
           // accumulator
-          if (elect_one()) {
           if constexpr (kF16) {
-            mma_f16(d, ahi, bhi, (c != 0 && c != kHalf) ? 1u : 0u);
-            mma_f16(dc, ahi, bhi + kBLo16, c ? 1u : 0u);
-            mma_f16(dc, ahi + kALo16, bhi, 1u);
-            mma_f16(dc, ahi, bhi + 2 * kBLo16, 1u);  // hi.lo2
+            mma_chunk_f16(d, dc, ahi, ahi + kALo16, bhi, kBLo16, (c != 0 && c != kHalf) ? 1u : 0u, c ? 1u : 0u,
+                          &sm.empty[as]);
           } else {
-            mma_tf32(d, ahi, bhi, (c != 0 && c != kHalf) ? 1u : 0u);
-            mma_tf32(dc, ahi, bhi + kBLo16, c ? 1u : 0u);
-            mma_tf32(dc, ahi + kALo16, bhi, 1u);
-            mma_tf32(d, ahi + kAK16, bhi + kBK16, 1u);
-            mma_tf32(dc, ahi + kAK16, bhi + kBK16 + kBLo16, 1u);
-            mma_tf32(dc, ahi + kAK16 + kALo16, bhi + kBK16, 1u);
+            if (elect_one()) {
+              mma_tf32(d, ahi, bhi, (c != 0 && c != kHalf) ? 1u : 0u);
+              mma_tf32(dc, ahi, bhi + kBLo16, c ? 1u : 0u);
+              mma_tf32(dc, ahi + kALo16, bhi, 1u);
+              mma_tf32(d, ahi + kAK16, bhi + kBK16, 1u);
+              mma_tf32(dc, ahi + kAK16, bhi + kBK16 + kBLo16, 1u);
+              mma_tf32(dc, ahi + kAK16 + kALo16, bhi + kBK16, 1u);
+              mma_commit(&sm.empty[as]);  // frees the A and the B stage
+            }
+            __syncwarp();
           }
-          mma_commit(&sm.a_empty[as]);  // also frees B stage bs (= as)
-          }
-          __syncwarp();
           mma_any = true;
           if (++as == kSt) { as = 0; aph ^= 1u; }
-          if (++bs == kSt) { bs = 0; bph ^= 1u; }
         }
         if (!ok) break;
         if (elect_one()) mma_commit(&sm.acc_full);
@@ -648,8 +659,10 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
     }
   } else if (warp < kWarpE0) {
     // ---- D formation ----------------------------------------------------------------
-    int const grp = (warp - kWarpD0) / kDGroup;  // chunks c = grp, grp + 2, ...
-    int const j = (warp - kWarpD0) % kDGroup;    // the chunk's j-th pair of (p, q)
+    int const dw = warp == 2 ? 0 : warp - 3;    // 0 .. 11
+    int const grp = dw / kDGroup;  // chunks c = grp, grp + 3, ...
+    int const j = dw % kDGroup;    // the chunk's j-th pair of (p, q)
+    d_next = grp;
     int const s = lane;
     bool ok = true;
     uint32_t unit = 0, last_pi = 0xFFFFFFFFu;
@@ -678,7 +691,7 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
         ok = ok && wait_or_fail(&sm.y_full[ys], (uint32_t)((uy / kYSlots) & 1), fail);
         ok = ok && wait_or_fail(&sm.s_full[ss], (uint32_t)((us / kSGroups) & 1), fail);
         int const ac = P * kChunks + c, as = ac % kSt;
-        if (!ok || !wait_or_fail(&sm.a_empty[as], (uint32_t)(((ac / kSt) & 1) ^ 1), fail)) { ok = false; break; }
+        if (!ok || !wait_or_fail(&sm.empty[as], (uint32_t)(((ac / kSt) & 1) ^ 1), fail)) { ok = false; break; }
         int const p_in = j >> 1, q_in = 2 * (j & 1);  // rows of the Y half and of the S group
         // k = 4j .. 4j+3 of the chunk, row (mu*32 + s). TF32: core column j,
         // the whole 16-byte row; FP16: core column j/2, its half j&1 (8 bytes)
@@ -778,7 +791,8 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          mbar_arrive(&sm.a_full[as]);
+          mbar_arrive(&sm.full[as]);
+          d_next = ac + kDGroups;
           // two groups read each S block, in one chunk each; every group
           // reads each Y half, in one of its three chunks (bq = 0..2)
           mbar_arrive(&sm.s_empty[ss]);
@@ -889,9 +903,17 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
       for (int u = rows_issued_y - kYSlots + 1; u <= rows_issued_y; ++u)
         if (u >= 0) mbar_wait(&sm.y_full[u % kYSlots], (uint32_t)((u / kYSlots) & 1));
     }
+    // the B copies complete the operand stages' barriers together with the D
+    // warps, which may have stopped short: they make up their arrivals first
+    // (a stage's barrier is in the phase of the last chunk issued into it)
+    if (warp == kWarpB && lane == 0) sm.b_last = b_issued;
+    __syncthreads();
+    if (d_next >= 0 && lane == 0)
+      for (int u = max(0, sm.b_last - kSt + 1); u <= sm.b_last; ++u)
+        if (u >= d_next && (u - d_next) % kDGroups == 0) mbar_arrive(&sm.full[u % kSt]);
     if (warp == kWarpB && lane == 0)
-      for (int u = b_issued - kSt + 1; u <= b_issued; ++u)
-        if (u >= 0) mbar_wait(&sm.b_full[u % kSt], (uint32_t)((u / kSt) & 1));
+      for (int u = max(0, b_issued - kSt + 1); u <= b_issued; ++u)
+        mbar_wait(&sm.full[u % kSt], (uint32_t)((u / kSt) & 1));
     if (warp == kWarpMma && lane == 0 && mma_any) {
       mma_commit(&sm.mma_done);
       mbar_wait(&sm.mma_done, 0);
