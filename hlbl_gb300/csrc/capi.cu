@@ -15,6 +15,7 @@
 #include "hlbl_gb300_rng.h"
 #include "hlbl_internal.h"
 #include "p1_f64.h"
+#include "p2_dig.h"
 #include "p2_f64.h"
 #include "p2_tc.h"
 #include "pieces_2p2.h"
@@ -279,6 +280,8 @@ struct hlbl_ctx {
   double* d_g = nullptr;      // [2][11520]
   void* d_bt = nullptr;       // [2][288*160] of double (float uses half of it)
   double* d_dzq = nullptr;    // FP64 pass 2: dz in block-diagonal form, [kMaxBatch][2][p2f64_dzq_len]
+  void* d_dig = nullptr;      // FP64 pass 2: work buffer of p2_dig.cu
+  size_t dig_cap = 0;         // its bytes
   int* d_bad = nullptr;       // hlbl_cu_4pt_contraction: sums that are not the gamma images of one dz
   double* d_w = nullptr;      // QED weights [V][3][6]
   long long w_cap = 0;        // sites d_w holds
@@ -379,6 +382,30 @@ int wait_staged(hlbl_ctx* c) {
   return HLBL_OK;
 }
 
+// Whether the FP64 pass 2 goes through digit products (p2_dig.cu), where its
+// work buffer exists or can be had (not during a capture; p2_f64.cu needs
+// none). p2_f64.cu takes all pairs of a batch in one launch, p2_dig.cu a handful
+// of launches for each pair: whole kernel sums with p2_f64.cu and p2_dig.cu, in us,
+//   128 sites: 399, 343 (one pair), 413, 748 (four); 256: 403, 347; 587, 750;
+//   512: 407, 351; 994, 830; 3320, 2893 (16 pairs); 2048: 997, 551; 3068, 1678.
+constexpr long long kDigMinSites = 128, kDigMinSitesBatch = 512;
+bool dig_ready(hlbl_ctx* c, const Geometry& geo, int npairs) {
+  if (geo.V < (npairs == 1 ? kDigMinSites : kDigMinSitesBatch)) return false;
+  size_t const need = p2dig_ws_bytes(geo.V, c->nsm);
+  if (need <= c->dig_cap) return true;
+  if (c->capturing) return false;
+  cudaStreamSynchronize(c->stream);
+  cudaFree(c->d_dig);
+  c->d_dig = nullptr;
+  c->dig_cap = 0;
+  if (cudaMalloc(&c->d_dig, need) != cudaSuccess) {
+    cudaGetLastError();  // not an error of the call
+    return false;
+  }
+  c->dig_cap = need;
+  return true;
+}
+
 // Pass 1 + reduction + gamma insertion + Bt for the batch's pairs, flavours
 // [f0, f0+nf). Pair i, flavour fl: dz at d_dz + (i*nf + fl)*kDzLen, g at
 // d_g + (i*nf + fl)*kGLen, Bt at d_bt + (i*nf + fl)*kBtK*kBtN. The FP64 pass 2
@@ -401,7 +428,7 @@ int run_pass1(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch
       c->d_part1, grid, nf, c->d_dz, add_dzu, add_dzsu);
   if (!build_bt) return HLBL_OK;
   if (precision == HLBL_FP64) {
-    p2f64_launch_dzq(c->d_dz, nullptr, nullptr, nf, b.n, c->d_dzq, nullptr, c->stream);
+    if (!dig_ready(c, geo, b.n)) p2f64_launch_dzq(c->d_dz, nullptr, nullptr, nf, b.n, c->d_dzq, nullptr, c->stream);
     return HLBL_OK;
   }
   g_build_kernel<<<dim3((kGLen / 2 + 255) / 256, nf, b.n), 256, 0, c->stream>>>(c->d_dz, nf, c->d_g);
@@ -522,15 +549,32 @@ int run_qed(hlbl_ctx* c, const Geometry& geo, const PairBatch& b, double xunit, 
 
 // Pass 2 for the batch's pairs with Bt (or dzq) already built; pair i's sums go to
 // b.p[i].out[0..nf) (added if add). bad: an FP64 flag on the device; where it is
-// set, the sums come from the general kernel with Bt instead of dzq.
+// set, the sums come from the general kernel with Bt instead of dzq. g_dzu, g_dzsu
+// (FP64, one pair): sums with the gammas inserted, in place of pass 1's.
 int run_pass2(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch& b, double xunit,
-              int f0, int nf, int precision, int add, const int* bad = nullptr) {
+              int f0, int nf, int precision, int add, const int* bad = nullptr,
+              const double* g_dzu = nullptr, const double* g_dzsu = nullptr) {
   P2Args a{};
   if (int rc = run_qed(c, geo, b, xunit, precision, a)) return rc;
   a.xunit = xunit;
   a.f0 = f0;
   int grid;
   prof_begin(c, 1);
+  if (precision == HLBL_FP64 && dig_ready(c, geo, b.n)) {
+    for (int i = 0; i < b.n; ++i) {
+      PairBatch one{};
+      one.n = 1;
+      one.p[0] = b.p[i];
+      P2Args ai = a;
+      if (ai.w) ai.w += (size_t)i * geo.V * 3 * HLBL_QED_NW;
+      if (ai.coef) ai.coef = static_cast<const double*>(ai.coef) + (size_t)i * a.coef_stride;
+      p2dig_launch(nf, c->nsm, c->stream, y, one, geo, ai, g_dzu ? nullptr : c->d_dz + (size_t)i * nf * kDzLen, g_dzu, g_dzsu,
+                   c->d_dig, c->d_part2, c->d_err);
+      p2_reduce_kernel<<<1, 64, 0, c->stream>>>(c->d_part2, c->nsm, nf, one, add);
+    }
+    prof_end(c, 1);
+    return HLBL_OK;
+  }
   if (precision == HLBL_FP64) {
     grid = per_pair_grid(c->grid_p2d[nf - 1], b.n, p2f64_tiles(geo.V));
     p2f64_launch(nf, grid, c->stream, y, b, geo, a, c->d_dzq, c->d_part2, c->d_err, bad);
@@ -646,7 +690,7 @@ int hlbl_ctx_create(hlbl_ctx** out, const int global[4], const int local[4],
   int rc;
   if ((rc = p1f64_init(2, c->nsm, c->grid_p1d[1])) || (rc = p1f64_init(1, c->nsm, c->grid_p1d[0])) ||
       (rc = P1F2::init(c->nsm, c->grid_p1f2)) || (rc = P1F1::init(c->nsm, c->grid_p1f1)) ||
-      (rc = p2f64_init(c->nsm, c->grid_p2d)) || (rc = P2D1::init(c->nsm, c->grid_p2d1)) ||
+      (rc = p2f64_init(c->nsm, c->grid_p2d)) || (rc = p2dig_init()) || (rc = P2D1::init(c->nsm, c->grid_p2d1)) ||
       (rc = P2F2::init(c->nsm, c->grid_p2f2)) || (rc = P2F1::init(c->nsm, c->grid_p2f1)) ||
       (rc = P1F2s::init(c->nsm, c->grid_p1f2s)) || (rc = P2F2s::init(c->nsm, c->grid_p2f2s)) ||
       (rc = tc_init(c->nsm, c->grid_tc)) || (rc = p1f32_init(c->nsm, c->grid_p1f)) ||
@@ -704,6 +748,7 @@ void hlbl_ctx_destroy(hlbl_ctx* c) {
   cudaFree(c->d_g);
   cudaFree(c->d_bt);
   cudaFree(c->d_dzq);
+  cudaFree(c->d_dig);
   cudaFree(c->d_bad);
   cudaFree(c->d_btu);
   cudaFree(c->d_bscale);
@@ -995,12 +1040,16 @@ int hlbl_cu_4pt_contraction(hlbl_ctx* c, double* d_ks, const double* d_g_dzu,
   // the sums are four gamma images of one dz (contract.cpp:58-77), from which
   // the block-diagonal form is built; a caller may pass other numbers, which
   // the build finds, and then the general form's kernel does the work
+  PairBatch const b = one_pair(src, d_ks, gsx, yv);
+  if (dig_ready(c, geo, 1)) {
+    if (int rc = run_pass2(c, geo, y, b, xunit, iflavor, 1, HLBL_FP64, 1, nullptr, d_g_dzu, d_g_dzsu)) return rc;
+    return check_launch("hlbl_cu_4pt_contraction launch");
+  }
   cudaError_t e = cudaMemsetAsync(c->d_bad, 0, sizeof(int), c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "hlbl_cu_4pt_contraction");
   p2f64_launch_dzq(nullptr, d_g_dzu, d_g_dzsu, 1, 1, c->d_dzq, c->d_bad, c->stream);
   bt_build_kernel<double><<<dim3((kBtK * kBtN + 255) / 256, 1, 1), 256, 0, c->stream>>>(
       d_g_dzu, d_g_dzsu, 0, 0, 1, static_cast<double*>(c->d_bt));
-  PairBatch const b = one_pair(src, d_ks, gsx, yv);
   if (int rc = run_pass2(c, geo, y, b, xunit, iflavor, 1, HLBL_FP64, 1, c->d_bad)) return rc;
   return check_launch("hlbl_cu_4pt_contraction launch");
 }

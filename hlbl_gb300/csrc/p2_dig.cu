@@ -1,0 +1,784 @@
+// p2_dig.cu -- the FP64 pass 2 (ker_4pt_contraction, cuda_lattice.cu:277-484)
+// without FP64 products: the spin-block products in 64-bit integers and the
+// contraction as exact products of digits on the tensor cores.
+//
+// What bounds the direct form is the FP64 pipe (two lanes per SM and cycle
+// here): 14.9 k multiply-adds per site and flavour for D_mu and 46.1 k for the
+// contraction even in the block-diagonal form of p2_f64.cu. Here
+//   D_mu   the blocks' values as 58-bit integers of a common exponent per site,
+//          two limbs of 29 bits, three 32 x 32 -> 64-bit integer multiply-adds
+//          per product (the product of the low limbs, below 2^-56 of the
+//          largest product, is dropped): sums of 24 such products stay below
+//          2^61, so nothing is rounded before the one rounding to 57 bits (with
+//          the sign) below the site's largest |D|;
+//   F = D Bt  D and Bt (per column) as eight balanced digits, seven of base 128
+//          and a top one of up to 128, in FP16; digit products with i + j <= 7
+//          (i = 0 the top) are accumulated by weight in eight FP32 accumulators
+//          in TMEM: each is an integer below 2^24 (288 k; at most two products of
+//          128 x 64 and six of 64 x 64), hence exact; the weights are put
+//          together in 64-bit integers.
+// The only roundings are those of the inputs to fixed point (2^-58 of the
+// site's largest component), of D and Bt (2^-57 of the site's and the column's
+// largest), the dropped products (i + j > 7: below 2^-53 of a typical F) and F's
+// conversion; the FP64 form rounds at 2^-53 of every partial sum. Roundings with a
+// mean add up over the sites where random ones do not, so D's is to nearest even,
+// and the mean of the products of weight 8 (D's lower digits, -64 to 63, have the
+// mean -1/2) is added per column.
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+
+#include "contract_kernels.cuh"
+#include "hlbl_gb300.h"
+#include "hlbl_internal.h"
+#include "p2_dig.h"
+#include "qed_entry.cuh"
+#include "tc_ops.cuh"
+
+namespace hg {
+namespace dig {
+
+using ll = long long;
+using ull = unsigned long long;
+
+constexpr int kSites = 32;            // sites per tile
+constexpr int kRows = 4 * kSites;     // rows (mu, site) of a tile: M of the MMA
+constexpr int kChunks = kBtK / 16;    // MMA steps of K = 16
+constexpr int kDig = 8;               // digits of a value
+constexpr int kAcc = kDig;            // accumulators: weights i + j
+constexpr int kParts = 3;             // the 160 columns in parts of 64, 64, 32 (eight accumulators in 512 TMEM columns)
+constexpr int kMaxTiles = 304;        // tiles of a batch
+constexpr int kMaxSites = kMaxTiles * kSites;
+// words of a tile and flavour: [chunk][k / 8][row][k % 8]
+constexpr int kTileWords = kChunks * 2 * kRows * 8;
+// digits are stored with 64 (the top: 128) added to each, as one 58-bit number:
+// the fields 0-3 in the low word, 4-7 in the high word, seven bits each (the top
+// digit's nine: 0 to 256)
+constexpr ull kBias = 64ull * ((1ull << 49) - 1) / 127 + (128ull << 49);
+// exponents of a site or column: with an infinite or NaN value; of zeros only
+constexpr int kNoScale = 1 << 20, kZeroExp = -(1 << 20);
+constexpr int kZeroRow = -20000;      // row exponent of a row of Bt of zeros only
+constexpr int kRowExp = 24;           // per flavour: of Y's rows p, of S's rows q
+
+__host__ __device__ constexpr int part_n0(int p) { return 64 * p; }
+__host__ __device__ constexpr int part_n(int p) { return p < 2 ? 64 : 32; }
+// bytes before part p's digits of Bt, and of one of its chunks
+__host__ __device__ constexpr int part_base(int p) { return part_n0(p) * kChunks * kDig * 32; }
+__host__ __device__ constexpr int part_chunk(int p) { return part_n(p) * kDig * 32; }
+constexpr size_t kBtBytes = (size_t)kBtN * kChunks * kDig * 32;  // per flavour
+
+// v 2^r as an integer x with |x| <= 2^(52 + kUp + 1), v 2^r = x 2^(em - 1075 - kUp), em
+// the largest exponent (exp_of) of the group, rounded to nearest
+template <int kUp>
+__device__ __forceinline__ ll to_fixed(double v, int r, int em) {
+  ull const b = (ull)__double_as_longlong(v);
+  int const f = (int)((b >> 52) & 0x7FFu);
+  ull const m = (b & 0xFFFFFFFFFFFFFull) | (f ? 1ull << 52 : 0ull);
+  int const sh = em - (f ? f : 1) - r;
+  ull x = m << kUp;
+  if (sh > 0) x = sh > 60 ? 0ull : (x + (1ull << (sh - 1))) >> sh;
+  return (b >> 63) ? -(ll)x : (ll)x;
+}
+// the biased exponent of v 2^r
+__device__ __forceinline__ int exp_of(double v, int r) {
+  int const f = (__double2hiint(v) >> 20) & 0x7FF;
+  return f == 0x7FF ? kNoScale : (v == 0.0 ? kZeroExp : (f ? f : 1) + r);
+}
+
+// ---- Bt's digits ---------------------------------------------------------------
+// Entry (p, q) of column n = (j, nu, lam) of Bt (bt_build_kernel's values), complex,
+// from pass 1's sums dz or from sums with the gammas inserted.
+__device__ __forceinline__ void bt_entry(const double* __restrict__ dz, const double* __restrict__ g_dzu,
+                                         const double* __restrict__ g_dzsu, int n, int p, int q, double& re, double& im) {
+  int const lam = n & 3, nu = (n >> 2) & 3, j = n >> 4;
+  int const s2 = gg5_src(lam, q / 3), sp = p / 3;  // an involution
+  int const ia = 3 * s2 + q % 3;
+  if (dz != nullptr) {
+    const double* v = dz + ((j * 12 + ia) * 12 + 3 * gg5_src(nu, sp) + p % 3) * 2;
+    mul_iph((gg5_ph(lam, s2) + gg5_ph(nu, sp)) & 3, v[0], v[1], re, im);
+  } else {
+    const double* g = (j < 6 ? g_dzu + (size_t)j * 1152 : g_dzsu + (size_t)(j - 6) * 1152) + ((nu * 12 + ia) * 12 + p) * 2;
+    mul_iph(gg5_ph(lam, s2), g[0], g[1], re, im);
+  }
+}
+
+// Powers of two that take the scale of the rows out of Bt and into D, so that a
+// D's fixed-point error is measured by what the value contributes (rows, e.g. of
+// one colour, may differ in scale): Bt(p, q) 2^(-b_p - c_q), Y_p 2^b_p, S_q 2^c_q.
+constexpr int kRowThreads = 576;
+__global__ void __launch_bounds__(kRowThreads)
+brow_kernel(const double* __restrict__ dz, const double* __restrict__ g_dzu, const double* __restrict__ g_dzsu,
+            int* __restrict__ rowexp) {
+  __shared__ int s_e[144], s_b[12];
+  int const fl = blockIdx.x, t = threadIdx.x, pq = t >> 2;
+  if (dz != nullptr) dz += (size_t)fl * kDzLen;
+  int m = kZeroExp;
+#pragma unroll 8
+  for (int n = t & 3; n < kBtN; n += 4) {
+    double re, im;
+    bt_entry(dz, g_dzu, g_dzsu, n, pq / 12, pq % 12, re, im);
+    m = max(m, max(exp_of(re, 0), exp_of(im, 0)));
+  }
+  m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+  m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+  if ((t & 3) == 0) s_e[pq] = min(m, 2047);
+  __syncthreads();
+  if (t < 12) {
+    int b = kZeroExp;
+    for (int q = 0; q < 12; ++q) b = max(b, s_e[t * 12 + q]);
+    s_b[t] = b == kZeroExp ? kZeroRow : b;
+    rowexp[fl * kRowExp + t] = s_b[t];
+  }
+  __syncthreads();
+  if (t < 12) {
+    int c = kZeroExp;
+    for (int p = 0; p < 12; ++p)
+      if (s_e[p * 12 + t] != kZeroExp) c = max(c, s_e[p * 12 + t] - s_b[p]);
+    rowexp[fl * kRowExp + 12 + t] = c == kZeroExp ? kZeroRow : c;
+  }
+}
+
+// Column n's digits, k = 2 (12 p + q) + e; em[fl][n]: the exponent of its largest value;
+// corr[fl][n]: the mean of the dropped products of weight 8, in units of weight 7.
+__global__ void __launch_bounds__(kBtK)
+bdig_build_kernel(const double* __restrict__ dz, const double* __restrict__ g_dzu, const double* __restrict__ g_dzsu,
+                  const int* __restrict__ rowexp, unsigned char* __restrict__ bt, int* __restrict__ em,
+                  int* __restrict__ corr) {
+  __shared__ int s_em, s_sum;
+  int const n = blockIdx.x, fl = blockIdx.y, k = threadIdx.x;
+  int const e = k & 1, q = (k >> 1) % 12, p = k / 24;
+  if (dz != nullptr) dz += (size_t)fl * kDzLen;
+  double re, im;
+  bt_entry(dz, g_dzu, g_dzsu, n, p, q, re, im);
+  double const x = e == 0 ? re : -im;
+  int const r = -rowexp[fl * kRowExp + p] - rowexp[fl * kRowExp + 12 + q];
+  if (k == 0) {
+    s_em = kZeroExp;
+    s_sum = 0;
+  }
+  __syncthreads();
+  atomicMax(&s_em, exp_of(x, r));
+  __syncthreads();
+  int const m = s_em;
+  if (k == 0) em[fl * kBtN + n] = m;
+  ull const w = (ull)to_fixed<3>(x, r, m) + kBias;
+  int const part = n < 128 ? n >> 6 : 2, np = part_n(part);
+  unsigned char* out = bt + (size_t)fl * kBtBytes + part_base(part) + (size_t)(k >> 4) * part_chunk(part) +
+                       (((k >> 3) & 1) * np + n - part_n0(part)) * 16 + (k & 7) * 2;
+  int sum = 0;
+#pragma unroll
+  for (int i = 0; i < kDig; ++i) {
+    int const u = (int)(w >> (7 * (kDig - 1 - i))) & (i == 0 ? 0x1FF : 0x7F), b = u - (i == 0 ? 128 : 64);
+    *reinterpret_cast<__half*>(out + (size_t)i * 2 * np * 16) = __int2half_rn(b);
+    if (i > 0) sum += b;
+  }
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if ((k & 31) == 0) atomicAdd(&s_sum, sum);
+  __syncthreads();
+  if (k == 0) corr[fl * kBtN + n] = (int)rintf(-0.5f / 128.f * (float)s_sum);
+}
+
+// ---- D's words -----------------------------------------------------------------
+constexpr int kTS = 4;                  // sites per CTA
+constexpr int kDThreads = 320;          // two groups of five warps, 144 threads (p, q) at work in each
+constexpr int kRowD = kTS * 24 + 2;     // staged row: 16 bytes of padding against bank conflicts
+
+// CTA: the sites s_begin + 4 blockIdx.x ... of the batch. words[tile][fl][kTileWords],
+// esc[fl][site]: D (its rows scaled by rowexp) = integer 2^esc.
+template <int NF>
+__global__ void __launch_bounds__(kDThreads, 2)
+dform_kernel(const double* __restrict__ y, const double* __restrict__ src, Geometry geo, int f0, ll s_begin,
+             const int* __restrict__ rowexp, uint2* __restrict__ words, int* __restrict__ esc, int* __restrict__ err) {
+  __shared__ __align__(128) double stage[2 * NF * 12][kRowD];
+  __shared__ __align__(8) uint64_t s_bar;
+  __shared__ int s_em[2][NF][kTS];
+  __shared__ uint32_t s_or[2][2][5][2];
+  int const t = threadIdx.x, l0 = kTS * blockIdx.x;
+  ll const s0 = s_begin + l0;
+  int const nvalid = (int)min((ll)kTS, geo.V - s0);
+  if (t == 0) {
+    mbar_init(&s_bar, 1);
+    fence_mbar_init();
+  }
+  if (t < 2 * NF * kTS) (&s_em[0][0][0])[t] = kZeroExp;
+  __syncthreads();
+  if (t == 0) {
+    // S = src at flavour 1-f, Y = y at flavour f, f = f0 + fl; rows [S | Y][fl][12]
+    uint32_t const bytes = (uint32_t)nvalid * 192u;
+    mbar_arrive_expect_tx(&s_bar, bytes * 2 * NF * 12);
+    for (int row = 0; row < 2 * NF * 12; ++row) {
+      int const which = row / (NF * 12), fl = (row / 12) % NF, ia = row % 12;
+      int const f = which == 0 ? 1 - f0 - fl : f0 + fl;
+      bulk_g2s(stage[row], (which == 0 ? src : y) + ((size_t)(f * 12 + ia) * geo.V + s0) * 24, bytes, &s_bar);
+    }
+  }
+  bool const ok = mbar_wait(&s_bar, 0);
+  if (__syncthreads_or(!ok)) {
+    // the copies land before the CTA exits (bounded, as everything else)
+    if (t == 0) {
+      if (err) atomicExch(err, kErrWaitTimeout);
+      mbar_wait(&s_bar, 0);
+    }
+    return;
+  }
+  {
+    // to fixed point in place: (site, fl, S or Y) by 20 (one flavour: 40) threads each
+    constexpr int kGroups = 2 * NF * kTS, kPer = kDThreads / kGroups, kVals = (288 + kPer - 1) / kPer;
+    int const g = t / kPer, i0 = t % kPer, s = g % kTS, fl = (g / kTS) % NF, which = g / (kTS * NF);
+    double (*const rows)[kRowD] = &stage[(which * NF + fl) * 12];
+    const int* const rx = rowexp + fl * kRowExp + (which == 0 ? 12 : 0);  // S: of rows q, Y: of rows p
+    double v[kVals];
+    int m = kZeroExp;
+    if (s < nvalid) {
+#pragma unroll
+      for (int i = 0; i < kVals; ++i) {
+        int const idx = i0 + i * kPer;
+        v[i] = idx < 288 ? rows[idx / 24][s * 24 + idx % 24] : 0.0;
+        m = max(m, exp_of(v[i], idx < 288 ? __ldg(rx + idx / 24) : 0));
+      }
+      atomicMax(&s_em[which][fl][s], m);
+    }
+    __syncthreads();
+    if (s < nvalid) {
+      m = s_em[which][fl][s];
+#pragma unroll
+      for (int i = 0; i < kVals; ++i) {
+        int const idx = i0 + i * kPer;
+        if (idx < 288) {
+          ll const x = to_fixed<4>(v[i], __ldg(rx + idx / 24), m);  // |x| <= 2^57
+          int const hi = (int)((x + (1ll << 28)) >> 29), lo = (int)(x - ((ll)hi << 29));
+          *reinterpret_cast<int2*>(&rows[idx / 24][s * 24 + idx % 24]) = make_int2(hi, lo);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  int const grp = t / 160, r = t % 160, p = r / 12, q = r % 12;
+  bool const active = r < 144;
+#pragma unroll 1
+  for (int it = 0; it < (NF == 2 ? kTS : kTS / 2); ++it) {
+    int const fl = NF == 2 ? grp : 0, s = NF == 2 ? it : 2 * it + grp;
+    ll X[4][2];
+    ull o = 0;
+    if (active) {
+      const int4* S = reinterpret_cast<const int4*>(&stage[fl * 12 + q][s * 24]);
+      const int4* Y = reinterpret_cast<const int4*>(&stage[(NF + fl) * 12 + p][s * 24]);
+      // O[s1][s2] = sum_c Y[s1][c] conj(S[s2][c]): al = O02 - O31, be = O13 - O20,
+      // ev = O03 + O21, od = O12 + O30; D_0 = al + be, D_3 = i (be - al),
+      // D_1 = -i (ev + od), D_2 = ev - od. Each sum as hi.hi and hi.lo + lo.hi.
+      ll h[8], m[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) h[i] = m[i] = 0;
+      // (ah, al), (bh, bl): limbs
+      auto mac = [&](int i, int ah, int al, int bh, int bl) {
+        h[i] += (ll)ah * bh;
+        m[i] += (ll)ah * bl;
+        m[i] += (ll)al * bh;
+      };
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        int4 const y0 = Y[c], y1 = Y[3 + c], y2 = Y[6 + c], y3 = Y[9 + c];
+        {
+          int4 const x2 = S[6 + c];
+          mac(0, y0.x, y0.y, x2.x, x2.y); mac(0, y0.z, y0.w, x2.z, x2.w);
+          mac(1, y0.z, y0.w, x2.x, x2.y); mac(1, -y0.x, -y0.y, x2.z, x2.w);
+          mac(6, y1.x, y1.y, x2.x, x2.y); mac(6, y1.z, y1.w, x2.z, x2.w);
+          mac(7, y1.z, y1.w, x2.x, x2.y); mac(7, -y1.x, -y1.y, x2.z, x2.w);
+        }
+        {
+          int4 const x3 = S[9 + c];
+          mac(2, y1.x, y1.y, x3.x, x3.y); mac(2, y1.z, y1.w, x3.z, x3.w);
+          mac(3, y1.z, y1.w, x3.x, x3.y); mac(3, -y1.x, -y1.y, x3.z, x3.w);
+          mac(4, y0.x, y0.y, x3.x, x3.y); mac(4, y0.z, y0.w, x3.z, x3.w);
+          mac(5, y0.z, y0.w, x3.x, x3.y); mac(5, -y0.x, -y0.y, x3.z, x3.w);
+        }
+        {
+          int4 const x1 = S[3 + c];
+          mac(0, -y3.x, -y3.y, x1.x, x1.y); mac(0, -y3.z, -y3.w, x1.z, x1.w);
+          mac(1, -y3.z, -y3.w, x1.x, x1.y); mac(1, y3.x, y3.y, x1.z, x1.w);
+          mac(4, y2.x, y2.y, x1.x, x1.y); mac(4, y2.z, y2.w, x1.z, x1.w);
+          mac(5, y2.z, y2.w, x1.x, x1.y); mac(5, -y2.x, -y2.y, x1.z, x1.w);
+        }
+        {
+          int4 const x0 = S[c];
+          mac(2, -y2.x, -y2.y, x0.x, x0.y); mac(2, -y2.z, -y2.w, x0.z, x0.w);
+          mac(3, -y2.z, -y2.w, x0.x, x0.y); mac(3, y2.x, y2.y, x0.z, x0.w);
+          mac(6, y3.x, y3.y, x0.x, x0.y); mac(6, y3.z, y3.w, x0.z, x0.w);
+          mac(7, y3.z, y3.w, x0.x, x0.y); mac(7, -y3.x, -y3.y, x0.z, x0.w);
+        }
+      }
+      // in units of 2^58 input units
+#pragma unroll
+      for (int i = 0; i < 8; ++i) h[i] += (m[i] + (1ll << 28)) >> 29;
+      X[0][0] = h[0] + h[2];  X[0][1] = h[1] + h[3];
+      X[3][0] = h[1] - h[3];  X[3][1] = h[2] - h[0];
+      X[1][0] = h[5] + h[7];  X[1][1] = -(h[4] + h[6]);
+      X[2][0] = h[4] - h[6];  X[2][1] = h[5] - h[7];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) o |= (ull)(X[i >> 1][i & 1] ^ (X[i >> 1][i & 1] >> 63));
+    }
+    // the position of the site's largest |D|'s top bit
+    uint32_t const oh = __reduce_or_sync(0xffffffffu, (uint32_t)(o >> 32));
+    uint32_t const ol = __reduce_or_sync(0xffffffffu, (uint32_t)o);
+    if ((t & 31) == 0) {
+      s_or[it & 1][grp][r >> 5][0] = oh;
+      s_or[it & 1][grp][r >> 5][1] = ol;
+    }
+    asm volatile("bar.sync %0, 160;" ::"r"(1 + grp) : "memory");
+    uint32_t ah = 0, al = 0;
+#pragma unroll
+    for (int w = 0; w < 5; ++w) {
+      ah |= s_or[it & 1][grp][w][0];
+      al |= s_or[it & 1][grp][w][1];
+    }
+    int const sh = 64 - __clzll((ll)(((ull)ah << 32) | al)) - 56;  // to |D| <= 2^56
+    if (active && s < nvalid) {
+      int const l = l0 + s;
+      uint2* out = words + ((size_t)(l / kSites) * NF + fl) * kTileWords +
+                   ((size_t)(r >> 2) * kRows + l % kSites) * 8 + 2 * (r & 3);
+#pragma unroll
+      for (int mu = 0; mu < 4; ++mu) {
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          ll const v = X[mu][e];
+          // to nearest even
+          ull const d = (ull)(sh > 0 ? (v + (1ll << (sh - 1)) - 1 + ((v >> sh) & 1)) >> sh : v << -sh) + kBias;
+          w[2 * e] = (uint32_t)d & 0xFFFFFFFu;
+          w[2 * e + 1] = (uint32_t)(d >> 28);
+        }
+        *reinterpret_cast<uint4*>(out + mu * kSites * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      if (r == 0) {
+        int const a = s_em[0][fl][s], b = s_em[1][fl][s];
+        esc[fl * kMaxSites + l] = a == kNoScale || b == kNoScale ? kNoScale : a + b - 2100 + sh;
+      }
+    }
+  }
+}
+
+// ---- the coefficients of the closed-form weight ------------------------------------
+// coef[site][mu][n] of the batch's sites (the layout of the generic coefficient
+// stage), four sites per CTA.
+struct CoefSmem {
+  double vec[kTS][12];                    // xm, x - y, zerohalf x
+  double tab[kTS * 3][kQedTab + 1];
+  double e3[kTS][6][64];                  // E3(k, lam, nu, mu) as [k][lam][nu][mu]
+};
+__global__ void __launch_bounds__(320)
+coef_closed_kernel(PairBatch batch, Geometry geo, double xu, const double* __restrict__ w, ll s_begin,
+                   double* __restrict__ coef) {
+  __shared__ CoefSmem sm;
+  int const t = threadIdx.x, nthr = blockDim.x;
+  int const gsx[4] = {batch.p[0].gsx[0], batch.p[0].gsx[1], batch.p[0].gsx[2], batch.p[0].gsx[3]};
+  int const yv[4] = {batch.p[0].yv[0], batch.p[0].yv[1], batch.p[0].yv[2], batch.p[0].yv[3]};
+  ll const s0 = s_begin + (ll)kTS * blockIdx.x;
+  int const nvalid = (int)min((ll)kTS, geo.V - s0);
+  if (t < kTS * 4) {
+    int const s = t >> 2, r = t & 3;
+    int rel[4];
+    rel_coords_fast(geo, gsx, min(s0 + s, geo.V - 1), rel);
+    sm.vec[s][r] = coord_map(rel[r], geo.global[r]) * xu;
+    sm.vec[s][4 + r] = coord_map_diff(rel[r], yv[r], geo.global[r]) * xu;
+    sm.vec[s][8 + r] = (double)coord_map_zerohalf(rel[r], geo.global[r]);
+  }
+  __syncthreads();
+  // the tensor's factors per (site, evaluation): e = 0: K(x, y), 1: K(y, x), 2: K(x, x - y)
+  for (int it = t; it < kTS * 3 * kQedTab; it += nthr) {
+    int const se = it / kQedTab, i = it % kQedTab, s = se / 3, e = se % 3;
+    const double* xm = sm.vec[s];
+    double ym[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) ym[r] = coord_map(mod_pos(yv[r], geo.global[r]), geo.global[r]) * xu;
+    sm.tab[se][i] = qed_tab_value(i, e == 1 ? ym : xm, e == 0 ? ym : (e == 1 ? xm : xm + 4),
+                                  w + (size_t)(min(s0 + s, geo.V - 1) * 3 + e) * HLBL_QED_NW);
+  }
+  __syncthreads();
+  for (int it = t; it < kTS * 384; it += nthr) {
+    int const s = it / 384, i = it % 384, k = i >> 6;
+    sm.e3[s][k][i & 63] =
+        qed_entry_tab(sm.tab[s * 3 + 2], k, comb_rho(k), comb_sigma(k), (i >> 4) & 3, (i >> 2) & 3, i & 3);
+  }
+  __syncthreads();
+  for (int it = t; it < nvalid * kCoefPerSite; it += nthr) {
+    int const s = it / kCoefPerSite, mu = (it / kBtN) & 3, n = it % kBtN;
+    int const lam = n & 3, nu = (n >> 2) & 3, j = n >> 4, e3 = lam * 16 + nu * 4 + mu;
+    double cf;
+    if (j < 6) {
+      int const r = comb_rho(j), g = comb_sigma(j);
+      cf = qed_entry_tab(sm.tab[s * 3], j, r, g, mu, nu, lam) + qed_entry_tab(sm.tab[s * 3 + 1], j, r, g, nu, mu, lam) -
+           sm.e3[s][j][e3];
+    } else {
+      // sum_k E3[k][lam][nu][mu] (zh_rho_k [sigma_k = tau] - zh_sigma_k [rho_k = tau])
+      int const tau = j - 6;
+      cf = 0.0;
+      for (int o = 0; o < 4; ++o) {
+        if (o == tau) continue;
+        int const r = min(o, tau), g = max(o, tau), k = r == 0 ? g - 1 : (r == 1 ? g + 1 : 5);
+        cf = fma(flip_sign(sm.vec[s][8 + o], tau < o ? 1u : 0u), sm.e3[s][k][e3], cf);
+      }
+    }
+    coef[(size_t)(kTS * blockIdx.x + s) * kCoefPerSite + mu * kBtN + n] = cf;
+  }
+}
+
+// ---- the products ------------------------------------------------------------------
+constexpr int kStages = 3;
+constexpr int kAPlane = kRows * 16 * 2;           // bytes of one digit of a chunk's A
+constexpr int kBMax = part_chunk(0);              // bytes of a chunk's Bt digits
+constexpr int kUnpackWarps = 8, kEWarps = 8, kWarpE0 = kUnpackWarps, kWarpMma = kWarpE0 + kEWarps, kWarpB = kWarpMma + 1;
+constexpr int kThreads = 32 * (kWarpB + 1);
+constexpr int kTmemCols = 512;
+static_assert(kAcc * part_n(0) == kTmemCols, "eight accumulators of 64 columns");
+
+struct __align__(1024) Smem {
+  unsigned char A[kStages][kDig * kAPlane];
+  unsigned char B[kStages][kBMax];
+  ll F[64][kRows];                                // the tile's F as integers (each thread its own)
+  uint64_t a_full[kStages], b_full[kStages], empty[kStages], acc_full, acc_free, mma_done;
+  double red[kEWarps][2][2];
+  int corr[2][kBtN];
+  int col_sh[2][kBtN];                            // a column's exponent relative to the largest, as a high word
+  int em_max[2];
+  uint32_t taddr;
+  int fail;
+};
+static_assert(sizeof(Smem) <= 232448, "shared memory above the 227 KB a CTA may have");
+
+// instruction descriptor: D F32, A and B FP16, both K-major, M = 128
+__device__ __forceinline__ uint32_t idesc(int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+}
+__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t desc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d),
+      "l"(a), "l"(b), "r"(desc), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, uint32_t r[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+// kOff + digit, of two values -> the digits in FP16 (1024 + u is exact there)
+template <uint32_t kOff>
+__device__ __forceinline__ uint32_t dig2(uint32_t u) {
+  uint32_t const x = u | 0x64006400u, k = 0x64006400u + kOff * 0x10001u;  // 1024 + u, 1024 + kOff
+  __half2 const h = __hsub2(*reinterpret_cast<const __half2*>(&x), *reinterpret_cast<const __half2*>(&k));
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// a converged warp's wait: the same answer in every lane
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* fail) {
+  return __all_sync(0xffffffffu, tc::wait_or_fail(bar, parity, fail));
+}
+
+// Units (tile, flavour, part) over the CTAs. state[cta][fl]: the compensated sum
+// over the batches; the last batch's launch writes partials.
+template <int NF>
+__global__ void __launch_bounds__(kThreads, 1)
+digit_mma_kernel(const uint2* __restrict__ words, const int* __restrict__ esc, const unsigned char* __restrict__ bt,
+                 const int* __restrict__ bem, const int* __restrict__ corr, const double* __restrict__ coef, int nsites, int first, int last,
+                 double* __restrict__ state, double* __restrict__ partials, int* __restrict__ err) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
+  int const t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  volatile int* const fail = &sm.fail;
+  if (t == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(&sm.a_full[i], kUnpackWarps);
+      mbar_init(&sm.b_full[i], 1);
+      mbar_init(&sm.empty[i], 1);
+    }
+    mbar_init(&sm.acc_full, 1);
+    mbar_init(&sm.acc_free, kEWarps);
+    mbar_init(&sm.mma_done, 1);
+    fence_mbar_init();
+    sm.fail = 0;
+  }
+  if (t < NF) {
+    int m = kZeroExp;
+    for (int n = 0; n < kBtN; ++n) m = max(m, bem[t * kBtN + n]);
+    sm.em_max[t] = m;
+  }
+  if (warp == kWarpMma) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.taddr)),
+                 "r"(kTmemCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  if (t < NF * kBtN) {
+    int const m = sm.em_max[t / kBtN];
+    sm.col_sh[t / kBtN][t % kBtN] = max(bem[t] - m, -900) * (1 << 20);
+    sm.corr[t / kBtN][t % kBtN] = corr[t];
+  }
+  __syncthreads();
+  uint32_t const tmem = sm.taddr;
+  int const nunits = (nsites + kSites - 1) / kSites * NF * kParts;
+
+  if (warp < kUnpackWarps) {
+    // ---- A's digits: thread = (row, k / 8) -----------------------------------------
+    int const row = t & (kRows - 1), kc = t >> 7;
+    int st = 0;
+    uint32_t ph = 1;
+    bool ok = true;
+#pragma unroll 1
+    for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
+      const uint4* w4 = reinterpret_cast<const uint4*>(words + (size_t)(u / kParts) * kTileWords + ((size_t)kc * kRows + row) * 8);
+      uint4 nx[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) nx[i] = __ldg(w4 + i);
+#pragma unroll 1
+      for (int c = 0; c < kChunks; ++c) {
+        uint4 cur[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) cur[i] = nx[i];
+        if (c + 1 < kChunks) {
+          const uint4* p = w4 + (size_t)(c + 1) * kRows * 8;  // a chunk: 2 x 128 x 8 words
+#pragma unroll
+          for (int i = 0; i < 4; ++i) nx[i] = __ldg(p + i);
+        }
+        if (!warp_wait(&sm.empty[st], ph, fail)) { ok = false; break; }
+        uint32_t d[kDig][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {  // the low word's fields: digits 7..4, the high word's: 3..0
+            uint32_t const a = h == 0 ? cur[i].x : cur[i].y, b = h == 0 ? cur[i].z : cur[i].w;
+            uint32_t const lo = __byte_perm(a, b, 0x5410), hi = __byte_perm(a >> 14, b >> 14, 0x5410);
+            d[(1 - h) * 4 + 3][i] = dig2<64>(lo & 0x007F007Fu);
+            d[(1 - h) * 4 + 2][i] = dig2<64>((lo >> 7) & 0x007F007Fu);
+            d[(1 - h) * 4 + 1][i] = dig2<64>(hi & 0x007F007Fu);
+            d[(1 - h) * 4 + 0][i] = h == 0 ? dig2<64>((hi >> 7) & 0x007F007Fu) : dig2<128>((hi >> 7) & 0x01FF01FFu);
+          }
+        }
+        unsigned char* A = sm.A[st] + ((size_t)kc * kRows + row) * 16;
+#pragma unroll
+        for (int i = 0; i < kDig; ++i)
+          *reinterpret_cast<uint4*>(A + i * kAPlane) = make_uint4(d[i][0], d[i][1], d[i][2], d[i][3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&sm.a_full[st]);
+        if (++st == kStages) { st = 0; ph ^= 1u; }
+      }
+    }
+  } else if (warp == kWarpB) {
+    // ---- Bt's digits -----------------------------------------------------------------
+    if (lane == 0) {
+      int st = 0, issued = 0;
+      uint32_t ph = 1;
+      bool ok = true;
+#pragma unroll 1
+      for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
+        int const part = u % kParts, fl = (u / kParts) % NF, bytes = part_chunk(part);
+        const unsigned char* b = bt + (size_t)fl * kBtBytes + part_base(part);
+#pragma unroll 1
+        for (int c = 0; c < kChunks; ++c) {
+          if (!tc::wait_or_fail(&sm.empty[st], ph, fail)) { ok = false; break; }
+          mbar_arrive_expect_tx(&sm.b_full[st], (uint32_t)bytes);
+          bulk_g2s(sm.B[st], b + (size_t)c * bytes, (uint32_t)bytes, &sm.b_full[st]);
+          ++issued;
+          if (++st == kStages) { st = 0; ph ^= 1u; }
+        }
+      }
+      // every copy lands before the CTA exits
+      for (int i = max(0, issued - kStages); i < issued; ++i) mbar_wait(&sm.b_full[i % kStages], (uint32_t)(i / kStages) & 1u);
+    }
+  } else if (warp == kWarpMma) {
+    // ---- MMA issue ---------------------------------------------------------------------
+    int st = 0, nu = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+#pragma unroll 1
+    for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x, ++nu) {
+      int const np = part_n(u % kParts);
+      uint32_t const desc = idesc(np);
+      if (!warp_wait(&sm.acc_free, (uint32_t)(nu & 1) ^ 1u, fail)) break;
+#pragma unroll 1
+      for (int c = 0; c < kChunks; ++c) {
+        if (!warp_wait(&sm.a_full[st], ph, fail) || !warp_wait(&sm.b_full[st], ph, fail)) { ok = false; break; }
+        tc::tc_fence_after();
+        uint64_t const a = tc::sdesc(smem_u32(sm.A[st]), kRows * 16, 128);
+        uint64_t const b = tc::sdesc(smem_u32(sm.B[st]), np * 16, 128);
+        if (tc::elect_one()) {
+#pragma unroll
+          for (int d = 0; d < kAcc; ++d)
+#pragma unroll
+            for (int i = 0; i <= d; ++i)
+              mma_f16(tmem + d * 64, a + (uint64_t)(i * (kAPlane >> 4)), b + (uint64_t)((d - i) * 2 * np), desc,
+                      i > 0 || c > 0 ? 1u : 0u);
+          tc::mma_commit(&sm.empty[st]);
+          if (c == kChunks - 1) tc::mma_commit(&sm.acc_full);
+        }
+        __syncwarp();
+        if (++st == kStages) { st = 0; ph ^= 1u; }
+      }
+    }
+    // no product in flight when the CTA exits
+    if (tc::elect_one()) {
+      tc::mma_commit(&sm.mma_done);
+      mbar_wait(&sm.mma_done, 0);
+    }
+    __syncwarp();
+  } else {
+    // ---- F from the accumulators, the dot ------------------------------------------------
+    int const ew = warp - kWarpE0, mu = ew & 3, half = ew >> 2, row = mu * 32 + lane;
+    uint32_t const lane_addr = tmem + ((uint32_t)(mu * 32) << 16);
+    Neu run[NF];
+    int nu = 0;
+#pragma unroll 1
+    for (int u = blockIdx.x; u < nunits; u += gridDim.x, ++nu) {
+      int const part = u % kParts, fl = (u / kParts) % NF, site = u / (kParts * NF) * kSites + lane;
+      int const nh = part_n(part) / 2, n0 = half * nh;
+      if (!warp_wait(&sm.acc_full, (uint32_t)nu & 1u, fail)) break;
+      tc::tc_fence_after();
+#pragma unroll 1
+      for (int n = n0; n < n0 + nh; n += 4) {
+        uint32_t r[kAcc][4];
+#pragma unroll
+        for (int d = 0; d < kAcc; ++d) tmem_ld4(lane_addr + d * 64 + n, r[d]);
+        tc::tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          int x[kAcc];
+#pragma unroll
+          for (int d = 0; d < kAcc; ++d) x[d] = __float2int_rn(__uint_as_float(r[d][i]));
+          ll const hi = ((((((ll)x[0] << 7) + x[1]) << 7) + x[2]) << 7) + x[3];
+          ll const lo = ((((((ll)x[4] << 7) + x[5]) << 7) + x[6]) << 7) + x[7] + sm.corr[fl][part_n0(part) + n + i];
+          sm.F[n + i][row] = (hi << 19) + ((lo + 256) >> 9);  // F 2^-58, below 2^63
+        }
+      }
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&sm.acc_free);
+      double part_sum = 0.0;
+      if (site < nsites) {
+        const double* cf = coef + (size_t)site * kCoefPerSite + mu * kBtN + part_n0(part);
+        const int* shp = &sm.col_sh[fl][part_n0(part)];
+#pragma unroll 4
+        for (int n = n0; n < n0 + nh; n += 2) {
+          double2 const c2 = __ldg(reinterpret_cast<const double2*>(cf + n));
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            ll const v = sm.F[n + i][row];
+            double const f = (double)v;
+            // times the column's power of two
+            double const g = __hiloint2double(__double2hiint(f) + (v != 0 ? shp[n + i] : 0), __double2loint(f));
+            part_sum = fma(i == 0 ? c2.x : c2.y, g, part_sum);
+          }
+        }
+        int const e = esc[fl * kMaxSites + site], m = sm.em_max[fl];
+        part_sum = e == kNoScale || m == kNoScale ? __longlong_as_double(0x7FF8000000000000ll)
+                                               : ldexp(part_sum, e + m - 1078 + 58);
+      }
+      if (NF == 1 || fl == 0) run[0].add(-part_sum);
+      else run[NF - 1].add(-part_sum);
+    }
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      Neu v = run[f];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        double const os = __shfl_down_sync(0xffffffffu, v.s, o);
+        double const oc = __shfl_down_sync(0xffffffffu, v.c, o);
+        v.add(os);
+        v.c += oc;
+      }
+      if (lane == 0) { sm.red[ew][f][0] = v.s; sm.red[ew][f][1] = v.c; }
+    }
+  }
+  __syncthreads();
+  if (t < NF && !*fail) {
+    Neu s;
+    double* const mine = state + ((size_t)blockIdx.x * 2 + t) * 2;
+    if (!first) { s.s = mine[0]; s.c = mine[1]; }
+    for (int w = 0; w < kEWarps; ++w) { s.add(sm.red[w][t][0]); s.c += sm.red[w][t][1]; }
+    mine[0] = s.s;
+    mine[1] = s.c;
+    if (last) partials[(size_t)blockIdx.x * NF + t] = s.get();
+  }
+  if (t == 0 && *fail && err) atomicExch(err, kErrWaitTimeout);
+  if (warp == kWarpMma)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+}
+
+// ---- the work buffer ------------------------------------------------------------------
+struct Ws {
+  size_t words, bt, coef, state, esc, bem, rowexp, corr, total;  // byte offsets
+};
+static int ws_tiles(ll V) { return (int)std::min<ll>(kMaxTiles, (V + kSites - 1) / kSites); }
+static Ws ws_layout(ll V, int nsm) {
+  Ws w{};
+  size_t o = 0;
+  auto take = [&](size_t bytes) {
+    size_t const at = o;
+    o += (bytes + 255) / 256 * 256;
+    return at;
+  };
+  size_t const tiles = (size_t)ws_tiles(V);
+  w.words = take(tiles * 2 * kTileWords * sizeof(uint2));
+  w.bt = take(2 * kBtBytes);
+  w.coef = take(tiles * kSites * kCoefPerSite * sizeof(double));
+  w.state = take((size_t)nsm * 4 * sizeof(double));
+  w.esc = take(2 * kMaxSites * sizeof(int));
+  w.bem = take(2 * kBtN * sizeof(int));
+  w.rowexp = take(2 * kRowExp * sizeof(int));
+  w.corr = take(2 * kBtN * sizeof(int));
+  w.total = o;
+  return w;
+}
+
+template <int NF>
+static void launch_t(int nsm, cudaStream_t st, const double* y, const PairBatch& b, const Geometry& geo,
+                     const P2Args& a, const double* dz, const double* g_dzu, const double* g_dzsu, void* ws,
+                     double* partials, int* err) {
+  Ws const l = ws_layout(geo.V, nsm);
+  unsigned char* const p = static_cast<unsigned char*>(ws);
+  uint2* const words = reinterpret_cast<uint2*>(p + l.words);
+  double* const coef = reinterpret_cast<double*>(p + l.coef);
+  int* const esc = reinterpret_cast<int*>(p + l.esc);
+  int* const bem = reinterpret_cast<int*>(p + l.bem);
+  int* const corr = reinterpret_cast<int*>(p + l.corr);
+  int* const rowexp = reinterpret_cast<int*>(p + l.rowexp);
+  brow_kernel<<<NF, kRowThreads, 0, st>>>(dz, g_dzu, g_dzsu, rowexp);
+  bdig_build_kernel<<<dim3(kBtN, NF), kBtK, 0, st>>>(dz, g_dzu, g_dzsu, rowexp, p + l.bt, bem, corr);
+  for (ll s0 = 0; s0 < geo.V; s0 += kMaxSites) {
+    int const n = (int)std::min<ll>(kMaxSites, geo.V - s0), cta = (n + kTS - 1) / kTS;
+    const double* cf = static_cast<const double*>(a.coef);
+    if (cf != nullptr) {
+      cf += (size_t)s0 * kCoefPerSite;
+    } else {
+      coef_closed_kernel<<<cta, 320, 0, st>>>(b, geo, a.xunit, a.w, s0, coef);
+      cf = coef;
+    }
+    dform_kernel<NF><<<cta, kDThreads, 0, st>>>(y, b.p[0].src, geo, a.f0, s0, rowexp, words, esc, err);
+    digit_mma_kernel<NF><<<nsm, kThreads, sizeof(Smem), st>>>(words, esc, p + l.bt, bem, corr, cf, n, s0 == 0,
+                                                              s0 + n >= geo.V, reinterpret_cast<double*>(p + l.state),
+                                                              partials, err);
+  }
+}
+
+}  // namespace dig
+
+int p2dig_init() {
+  cudaError_t e = cudaFuncSetAttribute(dig::digit_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dig::Smem));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(dig::digit_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dig::Smem));
+  return e == cudaSuccess ? HLBL_OK : cuda_fail(e, "digit product smem attribute");
+}
+
+size_t p2dig_ws_bytes(long long V, int nsm) { return dig::ws_layout(V, nsm).total; }
+
+void p2dig_launch(int nf, int nsm, cudaStream_t st, const double* y, const PairBatch& b, const Geometry& geo,
+                  const P2Args& a, const double* dz, const double* g_dzu, const double* g_dzsu, void* ws,
+                  double* partials, int* err) {
+  if (nf == 2) dig::launch_t<2>(nsm, st, y, b, geo, a, dz, g_dzu, g_dzsu, ws, partials, err);
+  else dig::launch_t<1>(nsm, st, y, b, geo, a, dz, g_dzu, g_dzsu, ws, partials, err);
+}
+
+}  // namespace hg

@@ -17,6 +17,7 @@
 #include "hlbl_gb300.h"
 #include "hlbl_internal.h"
 #include "p2_f64.h"
+#include "qed_entry.cuh"
 #include "quat_basis.cuh"
 
 namespace hg {
@@ -25,7 +26,6 @@ namespace p2d {
 constexpr int kTS = 4;                   // sites per tile
 constexpr int kThreads = 320;            // two flavours x 160 columns, or one flavour x two halves of the tile
 constexpr int kRowD = kTS * 24 + 2;      // staged row: 16 bytes of padding against bank conflicts
-constexpr int kTab = 63;                 // factors of the tensor's terms per (site, evaluation)
 template <int NF>
 struct __align__(128) Smem {
   double stage[2 * NF * 12][kRowD];
@@ -33,29 +33,9 @@ struct __align__(128) Smem {
   double coef[kTS][4][kBtN];
   double cq[quat::kBlk][kTS][4][kBtN];              // coefficients of [b*40 + j*4 + a] per block
   double vec[kTS][12];                              // xm, x - y, zerohalf x
-  double tab[kTS * 3][kTab + 1];
+  double tab[kTS * 3][kQedTab + 1];
 };
 static_assert(sizeof(Smem<2>) + 1024 <= 232448, "FP64 pass-2 shared memory above the 227 KB a CTA may have");
-
-// One entry kerv[k][mu][nu][lam] of the stand-in (qed_entry_t's six terms)
-// from the tabulated factors: two adds and three multiply-adds whatever the
-// indices (terms that vanish are selected to zero on the integer pipe; with
-// branches the lanes of a warp, which hold different entries, issue all
-// eleven).
-// tab: w0 a[4] | w1 b[4] | w2 (a-b)[4] | w3 (a_r b_s - a_s b_r)[6] | (a+b)[4] |
-//      w4 a[4] | b_i b_j [16] | w5 b[4] | a_i a_j [16] | 0
-__device__ __forceinline__ double entry(const double* __restrict__ tab, int k, int r, int s, int mu, int nu, int lam) {
-  double const t0 = mu == r && nu == s ? tab[lam] : (mu == s && nu == r ? quat::flip(tab[lam], 1u) : 0.0);
-  double const t1 = mu == r && lam == s ? tab[4 + nu] : (mu == s && lam == r ? quat::flip(tab[4 + nu], 1u) : 0.0);
-  double const t2 = nu == r && lam == s ? tab[8 + mu] : (nu == s && lam == r ? quat::flip(tab[8 + mu], 1u) : 0.0);
-  double const f3 = mu == nu ? tab[12 + k] : 0.0;
-  double const f4 = mu == s ? tab[22 + r] : (mu == r ? quat::flip(tab[22 + s], 1u) : 0.0);
-  double const f5 = lam == s ? tab[42 + r] : (lam == r ? quat::flip(tab[42 + s], 1u) : 0.0);
-  double v = t0 + t1 + t2;
-  v = fma(f3, tab[18 + lam], v);
-  v = fma(f4, tab[26 + 4 * nu + lam], v);
-  return fma(f5, tab[46 + 4 * mu + nu], v);
-}
 
 // dz in the form of quat_basis.cuh, halved: dzq[pair][fl][blk][k][j*4 + a],
 // k = (c_p*3 + c_q)*2 + e, the real part (e = 0) or minus the imaginary part
@@ -175,28 +155,14 @@ p2f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, P2Args
       }
     } else {
       // the tensor's factors per (site, evaluation): e = 0: K(x, y), 1: K(y, x), 2: K(x, x - y)
-      for (int it = t; it < kTS * 3 * kTab; it += nthr) {
-        int const se = it / kTab, i = it % kTab, s = se / 3, e = se % 3;
+      for (int it = t; it < kTS * 3 * kQedTab; it += nthr) {
+        int const se = it / kQedTab, i = it % kQedTab, s = se / 3, e = se % 3;
         const double* xm = sm.vec[s];
-        auto A = [&](int r) -> double {
-          return e == 1 ? coord_map(mod_pos(yv[r], geo.global[r]), geo.global[r]) * xu : xm[r];
-        };
-        auto Bv = [&](int r) -> double {
-          return e == 0 ? coord_map(mod_pos(yv[r], geo.global[r]), geo.global[r]) * xu : (e == 1 ? xm[r] : xm[4 + r]);
-        };
-        const double* w = wq + (size_t)(min(s0 + s, geo.V - 1) * 3 + e) * HLBL_QED_NW;
-        double v = 0.0;
-        if (i < 4) v = w[0] * A(i);
-        else if (i < 8) v = w[1] * Bv(i - 4);
-        else if (i < 12) v = w[2] * (A(i - 8) - Bv(i - 8));
-        else if (i < 18) {
-          int const r = comb_rho(i - 12), g = comb_sigma(i - 12);
-          v = w[3] * (A(r) * Bv(g) - A(g) * Bv(r));
-        } else if (i < 22) v = A(i - 18) + Bv(i - 18);
-        else if (i < 26) v = w[4] * A(i - 22);
-        else if (i < 42) v = Bv((i - 26) >> 2) * Bv((i - 26) & 3);
-        else if (i < 46) v = w[5] * Bv(i - 42);
-        else if (i < 62) v = A((i - 46) >> 2) * A((i - 46) & 3);
+        double ym[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) ym[r] = coord_map(mod_pos(yv[r], geo.global[r]), geo.global[r]) * xu;
+        double const v = qed_tab_value(i, e == 1 ? ym : xm, e == 0 ? ym : (e == 1 ? xm : xm + 4),
+                                       wq + (size_t)(min(s0 + s, geo.V - 1) * 3 + e) * HLBL_QED_NW);
         sm.tab[se][i] = v;
       }
       __syncthreads();
@@ -210,7 +176,7 @@ p2f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, P2Args
         double cf;
         if (j < 6) {
           int const r = comb_rho(j), g = comb_sigma(j);
-          cf = entry(q1, j, r, g, mu, nu, lam) + entry(q2, j, r, g, nu, mu, lam) - entry(q3, j, r, g, lam, nu, mu);
+          cf = qed_entry_tab(q1, j, r, g, mu, nu, lam) + qed_entry_tab(q2, j, r, g, nu, mu, lam) - qed_entry_tab(q3, j, r, g, lam, nu, mu);
         } else {
           // sum_k E3[k][lam][nu][mu] (zh_rho_k [sigma_k = tau] - zh_sigma_k [rho_k = tau])
           int const tau = j - 6;
@@ -218,7 +184,7 @@ p2f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, P2Args
           for (int o = 0; o < 4; ++o) {
             if (o == tau) continue;
             int const r = min(o, tau), g = max(o, tau), k = r == 0 ? g - 1 : (r == 1 ? g + 1 : 5);
-            cf = fma(quat::flip(sm.vec[s][8 + o], tau < o ? 1u : 0u), entry(q3, k, r, g, lam, nu, mu), cf);
+            cf = fma(flip_sign(sm.vec[s][8 + o], tau < o ? 1u : 0u), qed_entry_tab(q3, k, r, g, lam, nu, mu), cf);
           }
         }
         sm.coef[s][mu][n] = s < nvalid ? cf : 0.0;
