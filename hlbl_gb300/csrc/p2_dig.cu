@@ -33,6 +33,7 @@
 #include "contract_kernels.cuh"
 #include "hlbl_gb300.h"
 #include "hlbl_internal.h"
+#include "fixed_point.cuh"
 #include "p2_dig.h"
 #include "qed_entry.cuh"
 #include "tc_ops.cuh"
@@ -51,14 +52,13 @@ constexpr int kAcc = kDig;            // accumulators: weights i + j
 constexpr int kParts = 3;             // the 160 columns in parts of 64, 64, 32 (eight accumulators in 512 TMEM columns)
 constexpr int kMaxTiles = 304;        // tiles of a batch
 constexpr int kMaxSites = kMaxTiles * kSites;
-// words of a tile and flavour: [chunk][k / 8][row][k % 8]
-constexpr int kTileWords = kChunks * 2 * kRows * 8;
-// digits are stored with 64 (the top: 128) added to each, as one 58-bit number:
-// the fields 0-3 in the low word, 4-7 in the high word, seven bits each (the top
-// digit's nine: 0 to 256)
+// words of a tile and flavour: [chunk][k / 8][row][k % 8 / 2]
+constexpr int kTileWords = kChunks * 2 * kRows * 4;
+// digits are stored with 64 (the top: 128) added to each: D's as two values'
+// (re, im) 16-bit halves per word, digit 2 w + 1 in bits 0-6 and digit 2 w from
+// bit 7 (word w = 0..3; the top digit's nine bits: 0 to 256), as the MMA's A wants
+// neighbouring k side by side
 constexpr ull kBias = 64ull * ((1ull << 49) - 1) / 127 + (128ull << 49);
-// exponents of a site or column: with an infinite or NaN value; of zeros only
-constexpr int kNoScale = 1 << 20, kZeroExp = -(1 << 20);
 constexpr int kZeroRow = -20000;      // row exponent of a row of Bt of zeros only
 constexpr int kRowExp = 24;           // per flavour: of Y's rows p, of S's rows q
 
@@ -68,24 +68,6 @@ __host__ __device__ constexpr int part_n(int p) { return p < 2 ? 64 : 32; }
 __host__ __device__ constexpr int part_base(int p) { return part_n0(p) * kChunks * kDig * 32; }
 __host__ __device__ constexpr int part_chunk(int p) { return part_n(p) * kDig * 32; }
 constexpr size_t kBtBytes = (size_t)kBtN * kChunks * kDig * 32;  // per flavour
-
-// v 2^r as an integer x with |x| <= 2^(52 + kUp + 1), v 2^r = x 2^(em - 1075 - kUp), em
-// the largest exponent (exp_of) of the group, rounded to nearest
-template <int kUp>
-__device__ __forceinline__ ll to_fixed(double v, int r, int em) {
-  ull const b = (ull)__double_as_longlong(v);
-  int const f = (int)((b >> 52) & 0x7FFu);
-  ull const m = (b & 0xFFFFFFFFFFFFFull) | (f ? 1ull << 52 : 0ull);
-  int const sh = em - (f ? f : 1) - r;
-  ull x = m << kUp;
-  if (sh > 0) x = sh > 60 ? 0ull : (x + (1ull << (sh - 1))) >> sh;
-  return (b >> 63) ? -(ll)x : (ll)x;
-}
-// the biased exponent of v 2^r
-__device__ __forceinline__ int exp_of(double v, int r) {
-  int const f = (__double2hiint(v) >> 20) & 0x7FF;
-  return f == 0x7FF ? kNoScale : (v == 0.0 ? kZeroExp : (f ? f : 1) + r);
-}
 
 // ---- Bt's digits ---------------------------------------------------------------
 // Entry (p, q) of column n = (j, nu, lam) of Bt (bt_build_kernel's values), complex,
@@ -115,11 +97,17 @@ brow_kernel(const double* __restrict__ dz, const double* __restrict__ g_dzu, con
   int const fl = blockIdx.x, t = threadIdx.x, pq = t >> 2;
   if (dz != nullptr) dz += (size_t)fl * kDzLen;
   int m = kZeroExp;
-#pragma unroll 8
+  // over all columns (j, nu, lam) the entries are those of the images' spins: (p, q)'s
+  // colours with every pair of spins (a, b), or of each nu with every spin b of q
+  int const p = pq / 12, q = pq % 12;
+#pragma unroll 10
   for (int n = t & 3; n < kBtN; n += 4) {
-    double re, im;
-    bt_entry(dz, g_dzu, g_dzsu, n, pq / 12, pq % 12, re, im);
-    m = max(m, max(exp_of(re, 0), exp_of(im, 0)));
+    int const j = n >> 4, a = (n >> 2) & 3, b = n & 3;
+    const double* v = dz != nullptr ? dz + ((j * 12 + 3 * a + q % 3) * 12 + 3 * b + p % 3) * 2
+                                    : (j < 6 ? g_dzu + (size_t)j * 1152 : g_dzsu + (size_t)(j - 6) * 1152) +
+                                          ((a * 12 + 3 * b + q % 3) * 12 + p) * 2;
+    double2 const z = *reinterpret_cast<const double2*>(v);
+    m = max(m, max(exp_of(z.x, 0), exp_of(z.y, 0)));
   }
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
@@ -166,12 +154,12 @@ bdig_build_kernel(const double* __restrict__ dz, const double* __restrict__ g_dz
   ull const w = (ull)to_fixed<3>(x, r, m) + kBias;
   int const part = n < 128 ? n >> 6 : 2, np = part_n(part);
   unsigned char* out = bt + (size_t)fl * kBtBytes + part_base(part) + (size_t)(k >> 4) * part_chunk(part) +
-                       (((k >> 3) & 1) * np + n - part_n0(part)) * 16 + (k & 7) * 2;
+                       (((k >> 3) & 1) * kDig * np + n - part_n0(part)) * 16 + (k & 7) * 2;
   int sum = 0;
 #pragma unroll
   for (int i = 0; i < kDig; ++i) {
     int const u = (int)(w >> (7 * (kDig - 1 - i))) & (i == 0 ? 0x1FF : 0x7F), b = u - (i == 0 ? 128 : 64);
-    *reinterpret_cast<__half*>(out + (size_t)i * 2 * np * 16) = __int2half_rn(b);
+    *reinterpret_cast<__half*>(out + (size_t)i * np * 16) = __int2half_rn(b);
     if (i > 0) sum += b;
   }
   sum = __reduce_add_sync(0xffffffffu, sum);
@@ -190,7 +178,7 @@ constexpr int kRowD = kTS * 24 + 2;     // staged row: 16 bytes of padding again
 template <int NF>
 __global__ void __launch_bounds__(kDThreads, 2)
 dform_kernel(const double* __restrict__ y, const double* __restrict__ src, Geometry geo, int f0, ll s_begin,
-             const int* __restrict__ rowexp, uint2* __restrict__ words, int* __restrict__ esc, int* __restrict__ err) {
+             const int* __restrict__ rowexp, uint4* __restrict__ words, int* __restrict__ esc, int* __restrict__ err) {
   __shared__ __align__(128) double stage[2 * NF * 12][kRowD];
   __shared__ __align__(8) uint64_t s_bar;
   __shared__ int s_em[2][NF][kTS];
@@ -336,20 +324,21 @@ dform_kernel(const double* __restrict__ y, const double* __restrict__ src, Geome
     int const sh = 64 - __clzll((ll)(((ull)ah << 32) | al)) - 56;  // to |D| <= 2^56
     if (active && s < nvalid) {
       int const l = l0 + s;
-      uint2* out = words + ((size_t)(l / kSites) * NF + fl) * kTileWords +
-                   ((size_t)(r >> 2) * kRows + l % kSites) * 8 + 2 * (r & 3);
+      uint4* out = words + ((size_t)(l / kSites) * NF + fl) * kTileWords + ((size_t)(r >> 2) * kRows + l % kSites) * 4 + (r & 3);
 #pragma unroll
       for (int mu = 0; mu < 4; ++mu) {
-        uint32_t w[4];
+        uint32_t lo[2], hi[2];  // fields 0-3, 4-7
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           ll const v = X[mu][e];
           // to nearest even
           ull const d = (ull)(sh > 0 ? (v + (1ll << (sh - 1)) - 1 + ((v >> sh) & 1)) >> sh : v << -sh) + kBias;
-          w[2 * e] = (uint32_t)d & 0xFFFFFFFu;
-          w[2 * e + 1] = (uint32_t)(d >> 28);
+          lo[e] = (uint32_t)d;  // bits 28-31: masked below
+          hi[e] = (uint32_t)(d >> 28);
         }
-        *reinterpret_cast<uint4*>(out + mu * kSites * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+        out[mu * kSites * 4] = make_uint4(__byte_perm(hi[0] >> 14, hi[1] >> 14, 0x5410), __byte_perm(hi[0], hi[1], 0x5410) & 0x3FFF3FFFu,
+                                          __byte_perm(lo[0] >> 14, lo[1] >> 14, 0x5410) & 0x3FFF3FFFu,
+                                          __byte_perm(lo[0], lo[1], 0x5410) & 0x3FFF3FFFu);
       }
       if (r == 0) {
         int const a = s_em[0][fl][s], b = s_em[1][fl][s];
@@ -428,7 +417,7 @@ coef_closed_kernel(PairBatch batch, Geometry geo, double xu, const double* __res
 constexpr int kStages = 3;
 constexpr int kAPlane = kRows * 16 * 2;           // bytes of one digit of a chunk's A
 constexpr int kBMax = part_chunk(0);              // bytes of a chunk's Bt digits
-constexpr int kUnpackWarps = 8, kEWarps = 8, kWarpE0 = kUnpackWarps, kWarpMma = kWarpE0 + kEWarps, kWarpB = kWarpMma + 1;
+constexpr int kUnpackWarps = 16, kEWarps = 8, kWarpE0 = kUnpackWarps, kWarpMma = kWarpE0 + kEWarps, kWarpB = kWarpMma + 1;
 constexpr int kThreads = 32 * (kWarpB + 1);
 constexpr int kTmemCols = 512;
 static_assert(kAcc * part_n(0) == kTmemCols, "eight accumulators of 64 columns");
@@ -480,7 +469,7 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
 // over the batches; the last batch's launch writes partials.
 template <int NF>
 __global__ void __launch_bounds__(kThreads, 1)
-digit_mma_kernel(const uint2* __restrict__ words, const int* __restrict__ esc, const unsigned char* __restrict__ bt,
+digit_mma_kernel(const uint4* __restrict__ words, const int* __restrict__ esc, const unsigned char* __restrict__ bt,
                  const int* __restrict__ bem, const int* __restrict__ corr, const double* __restrict__ coef, int nsites, int first, int last,
                  double* __restrict__ state, double* __restrict__ partials, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -489,7 +478,7 @@ digit_mma_kernel(const uint2* __restrict__ words, const int* __restrict__ esc, c
   volatile int* const fail = &sm.fail;
   if (t == 0) {
     for (int i = 0; i < kStages; ++i) {
-      mbar_init(&sm.a_full[i], kUnpackWarps);
+      mbar_init(&sm.a_full[i], 8);
       mbar_init(&sm.b_full[i], 1);
       mbar_init(&sm.empty[i], 1);
     }
@@ -522,49 +511,47 @@ digit_mma_kernel(const uint2* __restrict__ words, const int* __restrict__ esc, c
   int const nunits = (nsites + kSites - 1) / kSites * NF * kParts;
 
   if (warp < kUnpackWarps) {
-    // ---- A's digits: thread = (row, k / 8) -----------------------------------------
-    int const row = t & (kRows - 1), kc = t >> 7;
-    int st = 0;
+    // ---- A's digits: thread = (row, k / 8) of every other chunk ----------------------
+    int const row = t & (kRows - 1), kc = (t >> 7) & 1, grp = t >> 8;
+    int st = grp % kStages;
     uint32_t ph = 1;
     bool ok = true;
 #pragma unroll 1
     for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
-      const uint4* w4 = reinterpret_cast<const uint4*>(words + (size_t)(u / kParts) * kTileWords + ((size_t)kc * kRows + row) * 8);
+      const uint4* w4 = words + (size_t)(u / kParts) * kTileWords + ((size_t)(2 * grp + kc) * kRows + row) * 4;
       uint4 nx[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) nx[i] = __ldg(w4 + i);
 #pragma unroll 1
-      for (int c = 0; c < kChunks; ++c) {
+      for (int c = grp; c < kChunks; c += 2) {
         uint4 cur[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) cur[i] = nx[i];
-        if (c + 1 < kChunks) {
-          const uint4* p = w4 + (size_t)(c + 1) * kRows * 8;  // a chunk: 2 x 128 x 8 words
+        if (c + 2 < kChunks) {
+          w4 += 4 * kRows * 4;  // a chunk: 2 x 128 x 4 words
 #pragma unroll
-          for (int i = 0; i < 4; ++i) nx[i] = __ldg(p + i);
+          for (int i = 0; i < 4; ++i) nx[i] = __ldg(w4 + i);
         }
         if (!warp_wait(&sm.empty[st], ph, fail)) { ok = false; break; }
-        uint32_t d[kDig][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {  // the low word's fields: digits 7..4, the high word's: 3..0
-            uint32_t const a = h == 0 ? cur[i].x : cur[i].y, b = h == 0 ? cur[i].z : cur[i].w;
-            uint32_t const lo = __byte_perm(a, b, 0x5410), hi = __byte_perm(a >> 14, b >> 14, 0x5410);
-            d[(1 - h) * 4 + 3][i] = dig2<64>(lo & 0x007F007Fu);
-            d[(1 - h) * 4 + 2][i] = dig2<64>((lo >> 7) & 0x007F007Fu);
-            d[(1 - h) * 4 + 1][i] = dig2<64>(hi & 0x007F007Fu);
-            d[(1 - h) * 4 + 0][i] = h == 0 ? dig2<64>((hi >> 7) & 0x007F007Fu) : dig2<128>((hi >> 7) & 0x01FF01FFu);
-          }
-        }
         unsigned char* A = sm.A[st] + ((size_t)kc * kRows + row) * 16;
 #pragma unroll
-        for (int i = 0; i < kDig; ++i)
-          *reinterpret_cast<uint4*>(A + i * kAPlane) = make_uint4(d[i][0], d[i][1], d[i][2], d[i][3]);
+        for (int w = 0; w < 4; ++w) {
+          uint32_t d[2][4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            uint32_t const x = w == 0 ? cur[i].x : (w == 1 ? cur[i].y : (w == 2 ? cur[i].z : cur[i].w));
+            d[1][i] = dig2<64>(x & 0x007F007Fu);
+            d[0][i] = w == 0 ? dig2<128>((x >> 7) & 0x01FF01FFu) : dig2<64>((x >> 7) & 0x007F007Fu);
+          }
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            *reinterpret_cast<uint4*>(A + (2 * w + e) * kAPlane) = make_uint4(d[e][0], d[e][1], d[e][2], d[e][3]);
+        }
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&sm.a_full[st]);
-        if (++st == kStages) { st = 0; ph ^= 1u; }
+        // two chunks on
+        if ((st += 2) >= kStages) { st -= kStages; ph ^= 1u; }
       }
     }
   } else if (warp == kWarpB) {
@@ -597,21 +584,27 @@ digit_mma_kernel(const uint2* __restrict__ words, const int* __restrict__ esc, c
 #pragma unroll 1
     for (int u = blockIdx.x; u < nunits && ok; u += gridDim.x, ++nu) {
       int const np = part_n(u % kParts);
-      uint32_t const desc = idesc(np);
       if (!warp_wait(&sm.acc_free, (uint32_t)(nu & 1) ^ 1u, fail)) break;
 #pragma unroll 1
       for (int c = 0; c < kChunks; ++c) {
         if (!warp_wait(&sm.a_full[st], ph, fail) || !warp_wait(&sm.b_full[st], ph, fail)) { ok = false; break; }
         tc::tc_fence_after();
         uint64_t const a = tc::sdesc(smem_u32(sm.A[st]), kRows * 16, 128);
-        uint64_t const b = tc::sdesc(smem_u32(sm.B[st]), np * 16, 128);
+        uint64_t const b = tc::sdesc(smem_u32(sm.B[st]), kDig * np * 16, 128);
         if (tc::elect_one()) {
+          // digit i of A with the digits j <= 7 - i of Bt, rows j np + n of one
+          // operand, into the accumulators' columns (i + j) np + n: 12 products of up
+          // to 256 columns (36 of 64 read A's digits from shared memory three times as
+          // often, which took twice the time of the products)
 #pragma unroll
-          for (int d = 0; d < kAcc; ++d)
+          for (int i = 0; i < kDig; ++i)
 #pragma unroll
-            for (int i = 0; i <= d; ++i)
-              mma_f16(tmem + d * 64, a + (uint64_t)(i * (kAPlane >> 4)), b + (uint64_t)((d - i) * 2 * np), desc,
-                      i > 0 || c > 0 ? 1u : 0u);
+            for (int r0 = 0; r0 < 64 * (kDig - i); r0 += 256) {
+              int const rows = min(np * (kDig - i) - r0, 256);
+              if (rows > 0)
+                mma_f16(tmem + i * np + r0, a + (uint64_t)(i * (kAPlane >> 4)), b + (uint64_t)r0, idesc(rows),
+                        i > 0 || c > 0 ? 1u : 0u);
+            }
           tc::mma_commit(&sm.empty[st]);
           if (c == kChunks - 1) tc::mma_commit(&sm.acc_full);
         }
@@ -641,7 +634,7 @@ digit_mma_kernel(const uint2* __restrict__ words, const int* __restrict__ esc, c
       for (int n = n0; n < n0 + nh; n += 4) {
         uint32_t r[kAcc][4];
 #pragma unroll
-        for (int d = 0; d < kAcc; ++d) tmem_ld4(lane_addr + d * 64 + n, r[d]);
+        for (int d = 0; d < kAcc; ++d) tmem_ld4(lane_addr + d * 2 * nh + n, r[d]);
         tc::tmem_wait_ld();
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -721,7 +714,7 @@ static Ws ws_layout(ll V, int nsm) {
     return at;
   };
   size_t const tiles = (size_t)ws_tiles(V);
-  w.words = take(tiles * 2 * kTileWords * sizeof(uint2));
+  w.words = take(tiles * 2 * kTileWords * sizeof(uint4));
   w.bt = take(2 * kBtBytes);
   w.coef = take(tiles * kSites * kCoefPerSite * sizeof(double));
   w.state = take((size_t)nsm * 4 * sizeof(double));
@@ -739,7 +732,7 @@ static void launch_t(int nsm, cudaStream_t st, const double* y, const PairBatch&
                      double* partials, int* err) {
   Ws const l = ws_layout(geo.V, nsm);
   unsigned char* const p = static_cast<unsigned char*>(ws);
-  uint2* const words = reinterpret_cast<uint2*>(p + l.words);
+  uint4* const words = reinterpret_cast<uint4*>(p + l.words);
   double* const coef = reinterpret_cast<double*>(p + l.coef);
   int* const esc = reinterpret_cast<int*>(p + l.esc);
   int* const bem = reinterpret_cast<int*>(p + l.bem);
