@@ -1,15 +1,20 @@
-// p1_f64.cu -- the FP64 pass 1 (ker_dzu_dzsu, cuda_lattice.cu:160-262).
+// p1_f64.cu -- the FP64 pass 1 (ker_dzu_dzsu, cuda_lattice.cu:160-262) with its
+// products in 64-bit integers.
 //
-// Thread (fl, ia, ib) owns dzu[k][ia][ib] and dzsu[s][ia][ib] of flavour
-// f = f0 + fl, as in p1_kernel. What bounds it is the FP64 pipe, so it is laid
-// out for few FP64 instructions per site and thread: the eight spin-block
-// products in four sums of two blocks each (96 multiply-adds, all that the four
-// X_sigma need), and, as the zerohalf weights zh_0..zh_2 are constant along a
-// run of sites in z, only the run's sums of the products and of zh_3 times them
-// (8 adds and 8 multiply-adds; 56 with all ten weighted sums per site). The
-// runs' sums go into the ten results at the end of each run, those into the
-// compensated sums every kFlushTiles tiles. Measured (both flavours, one pair):
-// 85.3 -> 42 ms at 663,552 sites, 1.11 -> 0.57 ms at 8,192.
+// Thread (ia, ib) of flavour f = f0 + blockIdx.z owns dzu[k][ia][ib] and
+// dzsu[s][ia][ib], as in p1_kernel. The FP64 pipe gives two multiply-adds per SM
+// and cycle here, the integer multiply-add (32 x 32 + 64 bits) 64: a tile's rows
+// are turned into integers of 55 bits and a sign below the row's largest value
+// (an exponent per row and tile of 8 sites), held as two limbs of 28 bits, and a
+// product takes three integer multiply-adds (the low limbs' product, below 2^-54
+// of the largest product, is dropped; no other rounding until a site's sum of 12
+// products is put together). As the zerohalf weights zh_0..zh_2 are constant along a
+// run of sites in z and zh_3 grows by one from site to site, a run needs the sum S
+// of its products and the sum W of S's partial sums, both exact in 64 bits; FP64
+// takes over at the end of the run: the ten results from S and T = sum zh_3 x
+// product = zh_3(first) S + (n S - W), those into the compensated sums every
+// kFlushTiles tiles. Measured (both flavours, one pair): with FP64 products 42 ms
+// at 663,552 sites and 0.54 ms at 8,192, so 16.7 and 0.25.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -17,6 +22,7 @@
 #include "contract_kernels.cuh"
 #include "hlbl_gb300.h"
 #include "hlbl_internal.h"
+#include "fixed_point.cuh"
 #include "p1_f64.h"
 
 namespace hg {
@@ -25,41 +31,40 @@ namespace p1d {
 constexpr int kTS = 8;                 // sites per tile
 constexpr int kRow = kTS * 24 + 2;     // staged row: 16 bytes of padding against bank conflicts
 constexpr int kFlushTiles = 4;         // tiles per addition into the compensated sums
-template <int NF>
+constexpr int kThreads = 144;
 struct __align__(128) Smem {
-  double stage[2][2 * NF * 12][kRow];
-  double zh[2][kTS][4];
+  double stage[2][24][kRow];           // rows [src | y][12]; a tile at work holds limbs (hi, lo) instead
+  int zh[2][kTS][4];
+  int em[24];                          // the rows' exponents (exp_of)
 };
 
-template <int NF>
-__global__ void __launch_bounds__(NF * 144, NF == 1 ? 2 : 1)
+__global__ void __launch_bounds__(kThreads, 3)
 p1f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0, double* __restrict__ partials,
              int* __restrict__ err) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  Smem<NF>& sm = *reinterpret_cast<Smem<NF>*>(smem_raw);
+  Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ int s_fail;
-  int const t = threadIdx.x, pi = blockIdx.y;
+  int const t = threadIdx.x, pi = blockIdx.y, fl = blockIdx.z, nf = gridDim.z;
   const double* __restrict__ src = batch.p[pi].src;
   int const gsx[4] = {batch.p[pi].gsx[0], batch.p[pi].gsx[1], batch.p[pi].gsx[2], batch.p[pi].gsx[3]};
-  int const fl = t / 144, ia = (t % 144) / 12, ib = t % 12;
-  // rows [src | y][fl][12]: src flavour f0 + fl, y flavour 1 - (f0 + fl)
+  int const ia = t / 12, ib = t % 12;
+  // src flavour f0 + fl, y flavour 1 - (f0 + fl)
   auto issue = [&](long long tile, int st) {
     long long const s0 = tile * kTS;
     uint32_t const bytes = (uint32_t)min((long long)kTS, geo.V - s0) * 192u;
-    mbar_arrive_expect_tx(&s_bar[st], bytes * 2 * NF * 12);
-    for (int row = 0; row < 2 * NF * 12; ++row) {
-      int const which = row / (NF * 12), f = (row / 12) % NF, i = row % 12;
-      int const ff = which == 0 ? f0 + f : 1 - f0 - f;
-      bulk_g2s(sm.stage[st][row], (which == 0 ? src : y) + ((size_t)(ff * 12 + i) * geo.V + s0) * 24, bytes, &s_bar[st]);
+    mbar_arrive_expect_tx(&s_bar[st], bytes * 24);
+    for (int row = 0; row < 24; ++row) {
+      int const i = row % 12, ff = row < 12 ? f0 + fl : 1 - f0 - fl;
+      bulk_g2s(sm.stage[st][row], (row < 12 ? src : y) + ((size_t)(ff * 12 + i) * geo.V + s0) * 24, bytes, &s_bar[st]);
     }
   };
   auto zh_fill = [&](long long tile, int buf) {
-    for (int s = t; s < kTS; s += blockDim.x) {
+    for (int s = t; s < kTS; s += kThreads) {
       int rel[4];
       rel_coords_fast(geo, gsx, min(tile * kTS + s, geo.V - 1), rel);
 #pragma unroll
-      for (int r = 0; r < 4; ++r) sm.zh[buf][s][r] = (double)coord_map_zerohalf(rel[r], geo.global[r]);
+      for (int r = 0; r < 4; ++r) sm.zh[buf][s][r] = coord_map_zerohalf(rel[r], geo.global[r]);
     }
   };
   if (t == 0) {
@@ -68,6 +73,7 @@ p1f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0
     fence_mbar_init();
     s_fail = 0;
   }
+  if (t < 24) sm.em[t] = kZeroExp;
   __syncthreads();
 
   Neu acc_u[6][2], acc_s[4][2];
@@ -113,49 +119,109 @@ p1f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0
       issue(tile + gridDim.x, st ^ 1);
     }
     if (!mbar_wait(&s_bar[st], (uint32_t)((it >> 1) & 1))) s_fail = 1;
-    else {
-      const double* A_base = sm.stage[st][fl * 12 + ia];
-      const double* B_base = sm.stage[st][NF * 12 + fl * 12 + ib];
-      const double (*zhs)[4] = sm.zh[st];
+    __syncthreads();
+    if (s_fail) break;
+    {
+      // the rows' exponents, then limbs in place: six threads per row
+      int const row = t / 6, nval = nvalid * 24;
+      double* const p = sm.stage[st][row];
+      int m = kZeroExp;
+#pragma unroll 8
+      for (int i = t % 6; i < nval; i += 6) m = max(m, exp_of(p[i], 0));
+      atomicMax(&sm.em[row], m);
+      __syncthreads();
+      m = sm.em[row];
+#pragma unroll 4
+      for (int i = t % 6; i < nval; i += 6) {
+        long long const x = to_fixed<2>(p[i], 0, m);  // |x| <= 2^55
+        int const hi = (int)((x + (1ll << 27)) >> 28), lo = (int)(x - ((long long)hi << 28));
+        *reinterpret_cast<int2*>(p + i) = make_int2(hi, lo);
+      }
+    }
+    __syncthreads();
+    {
+      const double* A_base = sm.stage[st][ia];
+      const double* B_base = sm.stage[st][12 + ib];
+      const int (*zhs)[4] = sm.zh[st];
+      // a product's unit 2^56 2^(em - 1077) 2^(em' - 1077)
+      int const ea = sm.em[ia], eb = sm.em[12 + ib];
+      double const scale = ea == kNoScale || eb == kNoScale ? __longlong_as_double(0x7FF8000000000000ll)
+                                                            : pow2(ea + eb - 2 * 1077 + 56);
       int z = (int)(s0 % geo.local[3]);
       int s = 0;
 #pragma unroll 1
       while (s < nvalid) {
-        // a run: sites of the tile with the same (t, x, y)
-        int const end = min(nvalid, s + geo.local[3] - z), last = end - 1;
-        // sums over the run, S of the products, T of zh_3 times them
-        double S[4][2], T[4][2];
+        // a run: sites of the tile with the same (t, x, y) and zh_3 growing by one
+        int const first = s;
+        long long S[8], W[8];
 #pragma unroll
-        for (int g = 0; g < 4; ++g) S[g][0] = S[g][1] = T[g][0] = T[g][1] = 0.0;
+        for (int i = 0; i < 8; ++i) S[i] = W[i] = 0;
 #pragma unroll 1
-        for (; s < end; ++s) {
-          const double2* A = reinterpret_cast<const double2*>(A_base + s * 24);
-          const double2* B = reinterpret_cast<const double2*>(B_base + s * 24);
+        do {
+          const int4* A = reinterpret_cast<const int4*>(A_base + s * 24);
+          const int4* B = reinterpret_cast<const int4*>(B_base + s * 24);
           // P[s1][s2] = sum_c conj(B[s1][c]) A[s2][c]: al = P02 - P31, be = P13 - P20,
-          // ev = P03 + P21, od = P12 + P30
-          double ar = 0, ai = 0, br = 0, bi = 0, er = 0, ei = 0, orr = 0, oi = 0;
+          // ev = P03 + P21, od = P12 + P30; each as hi.hi and hi.lo + lo.hi
+          long long h[8], m[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) h[i] = m[i] = 0;
+          auto mac = [&](int i, int ah, int al, int bh, int bl) {
+            h[i] += (long long)ah * bh;
+            m[i] += (long long)ah * bl;
+            m[i] += (long long)al * bh;
+          };
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            double2 const y0 = B[c], y1 = B[3 + c], y2 = B[6 + c], y3 = B[9 + c];
-            double2 const x0 = A[c], x1 = A[3 + c], x2 = A[6 + c], x3 = A[9 + c];
-            ar += y0.x * x2.x; ar += y0.y * x2.y; ar -= y3.x * x1.x; ar -= y3.y * x1.y;
-            ai += y0.x * x2.y; ai -= y0.y * x2.x; ai -= y3.x * x1.y; ai += y3.y * x1.x;
-            br += y1.x * x3.x; br += y1.y * x3.y; br -= y2.x * x0.x; br -= y2.y * x0.y;
-            bi += y1.x * x3.y; bi -= y1.y * x3.x; bi -= y2.x * x0.y; bi += y2.y * x0.x;
-            er += y0.x * x3.x; er += y0.y * x3.y; er += y2.x * x1.x; er += y2.y * x1.y;
-            ei += y0.x * x3.y; ei -= y0.y * x3.x; ei += y2.x * x1.y; ei -= y2.y * x1.x;
-            orr += y1.x * x2.x; orr += y1.y * x2.y; orr += y3.x * x0.x; orr += y3.y * x0.y;
-            oi += y1.x * x2.y; oi -= y1.y * x2.x; oi += y3.x * x0.y; oi -= y3.y * x0.x;
+            int4 const y0 = B[c], y1 = B[3 + c], y2 = B[6 + c], y3 = B[9 + c];
+            {
+              int4 const x2 = A[6 + c];
+              mac(0, y0.x, y0.y, x2.x, x2.y); mac(0, y0.z, y0.w, x2.z, x2.w);
+              mac(1, y0.x, y0.y, x2.z, x2.w); mac(1, -y0.z, -y0.w, x2.x, x2.y);
+              mac(6, y1.x, y1.y, x2.x, x2.y); mac(6, y1.z, y1.w, x2.z, x2.w);
+              mac(7, y1.x, y1.y, x2.z, x2.w); mac(7, -y1.z, -y1.w, x2.x, x2.y);
+            }
+            {
+              int4 const x3 = A[9 + c];
+              mac(2, y1.x, y1.y, x3.x, x3.y); mac(2, y1.z, y1.w, x3.z, x3.w);
+              mac(3, y1.x, y1.y, x3.z, x3.w); mac(3, -y1.z, -y1.w, x3.x, x3.y);
+              mac(4, y0.x, y0.y, x3.x, x3.y); mac(4, y0.z, y0.w, x3.z, x3.w);
+              mac(5, y0.x, y0.y, x3.z, x3.w); mac(5, -y0.z, -y0.w, x3.x, x3.y);
+            }
+            {
+              int4 const x1 = A[3 + c];
+              mac(0, -y3.x, -y3.y, x1.x, x1.y); mac(0, -y3.z, -y3.w, x1.z, x1.w);
+              mac(1, -y3.x, -y3.y, x1.z, x1.w); mac(1, y3.z, y3.w, x1.x, x1.y);
+              mac(4, y2.x, y2.y, x1.x, x1.y); mac(4, y2.z, y2.w, x1.z, x1.w);
+              mac(5, y2.x, y2.y, x1.z, x1.w); mac(5, -y2.z, -y2.w, x1.x, x1.y);
+            }
+            {
+              int4 const x0 = A[c];
+              mac(2, -y2.x, -y2.y, x0.x, x0.y); mac(2, -y2.z, -y2.w, x0.z, x0.w);
+              mac(3, -y2.x, -y2.y, x0.z, x0.w); mac(3, y2.z, y2.w, x0.x, x0.y);
+              mac(6, y3.x, y3.y, x0.x, x0.y); mac(6, y3.z, y3.w, x0.z, x0.w);
+              mac(7, y3.x, y3.y, x0.z, x0.w); mac(7, -y3.z, -y3.w, x0.x, x0.y);
+            }
           }
-          double const z3 = zhs[s][3];
-          S[0][0] += ar; S[0][1] += ai; S[1][0] += br; S[1][1] += bi;
-          S[2][0] += er; S[2][1] += ei; S[3][0] += orr; S[3][1] += oi;
-          T[0][0] = fma(z3, ar, T[0][0]); T[0][1] = fma(z3, ai, T[0][1]);
-          T[1][0] = fma(z3, br, T[1][0]); T[1][1] = fma(z3, bi, T[1][1]);
-          T[2][0] = fma(z3, er, T[2][0]); T[2][1] = fma(z3, ei, T[2][1]);
-          T[3][0] = fma(z3, orr, T[3][0]); T[3][1] = fma(z3, oi, T[3][1]);
+          // a site's sum stays below 2^57.6 units, eight sites' S and W below 2^63
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            S[i] += h[i] + ((m[i] + (1ll << 27)) >> 28);
+            W[i] += S[i];
+          }
+          ++s;
+          ++z;
+        } while (s < nvalid && z < geo.local[3] && zhs[s][3] == zhs[s - 1][3] + 1);
+        if (z == geo.local[3]) z = 0;
+        double Q[4][2], R[4][2];  // al, be, ev, od: S and T
+        {
+          int const n = s - first;
+          double const z0 = (double)zhs[first][3];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            Q[i >> 1][i & 1] = (double)S[i];
+            R[i >> 1][i & 1] = fma(z0, Q[i >> 1][i & 1], (double)(n * S[i] - W[i]));
+          }
         }
-        z = 0;
         // X_0 = -(al + be), X_1 = -i (ev + od), X_2 = od - ev, X_3 = i (be - al)
         auto to_x = [](const double q[4][2], double x[4][2]) {
           x[0][0] = -(q[0][0] + q[1][0]); x[0][1] = -(q[0][1] + q[1][1]);
@@ -163,25 +229,29 @@ p1f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0
           x[2][0] = q[3][0] - q[2][0];    x[2][1] = q[3][1] - q[2][1];
           x[3][0] = q[0][1] - q[1][1];    x[3][1] = q[1][0] - q[0][0];
         };
-        double X[4][2], W[4][2];
-        to_x(S, X);
-        to_x(T, W);
-        const double* zh = zhs[last];
+        double X[4][2];
+        double Y[4][2];
+        to_x(Q, X);
+        to_x(R, Y);
+        double const zh[3] = {(double)zhs[first][0], (double)zhs[first][1], (double)zhs[first][2]};
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
           int const r = comb_rho(k), g = comb_sigma(k);
 #pragma unroll
           for (int e = 0; e < 2; ++e)
-            tu[k][e] += g == 3 ? zh[r] * X[3][e] - W[r][e] : zh[r] * X[g][e] - zh[g] * X[r][e];
+            tu[k][e] = fma(scale, g == 3 ? zh[r] * X[3][e] - Y[r][e] : zh[r] * X[g][e] - zh[g] * X[r][e], tu[k][e]);
         }
 #pragma unroll
-        for (int g = 0; g < 4; ++g) { ts[g][0] += X[g][0]; ts[g][1] += X[g][1]; }
+        for (int g = 0; g < 4; ++g) {
+          ts[g][0] = fma(scale, X[g][0], ts[g][0]);
+          ts[g][1] = fma(scale, X[g][1], ts[g][1]);
+        }
       }
       if ((it & (kFlushTiles - 1)) == kFlushTiles - 1) flush();
     }
     if (more) zh_fill(tile + gridDim.x, st ^ 1);
-    __syncthreads();  // the stage and zh[st] are rewritten after this
-    if (s_fail) break;
+    __syncthreads();  // the stage, zh[st] and em are rewritten after this
+    if (t < 24) sm.em[t] = kZeroExp;
   }
   flush();
   if (s_fail) {
@@ -194,7 +264,7 @@ p1f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0
     }
     return;
   }
-  double* out = partials + (((size_t)pi * gridDim.x + blockIdx.x) * NF + fl) * kDzLen;
+  double* out = partials + (((size_t)pi * gridDim.x + blockIdx.x) * nf + fl) * kDzLen;
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
     out[((k * 12 + ia) * 12 + ib) * 2] = acc_u[k][0].get();
@@ -209,32 +279,25 @@ p1f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0
 
 }  // namespace p1d
 
-template <int NF>
-static int p1f64_init_t(int nsm, int& grid) {
-  size_t const smem = sizeof(p1d::Smem<NF>);
-  cudaError_t e = cudaFuncSetAttribute(p1d::p1f64_kernel<NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+int p1f64_init(int nf, int nsm, int& grid) {
+  size_t const smem = sizeof(p1d::Smem);
+  cudaError_t e = cudaFuncSetAttribute(p1d::p1f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(p1d::p1f64_kernel<NF>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
+    e = cudaFuncSetAttribute(p1d::p1f64_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return cuda_fail(e, "p1f64 smem attribute");
   int nb = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, p1d::p1f64_kernel<NF>, NF * 144, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, p1d::p1f64_kernel, p1d::kThreads, smem);
   if (e != cudaSuccess) return cuda_fail(e, "p1f64 occupancy");
   if (nb < 1) return fail(HLBL_ECUDA, "p1f64 kernel cannot be resident (smem %zu)", smem);
-  grid = nb * nsm;
+  grid = nb * nsm / nf;
   return HLBL_OK;
 }
-
-int p1f64_init(int nf, int nsm, int& grid) { return nf == 1 ? p1f64_init_t<1>(nsm, grid) : p1f64_init_t<2>(nsm, grid); }
 
 long long p1f64_tiles(long long V) { return (V + p1d::kTS - 1) / p1d::kTS; }
 
 void p1f64_launch(int nf, int grid, cudaStream_t st, const double* y, const PairBatch& b, const Geometry& geo,
                   int f0, double* partials, int* err) {
-  if (nf == 2)
-    p1d::p1f64_kernel<2><<<dim3(grid, b.n), 288, sizeof(p1d::Smem<2>), st>>>(y, b, geo, f0, partials, err);
-  else
-    p1d::p1f64_kernel<1><<<dim3(grid, b.n), 144, sizeof(p1d::Smem<1>), st>>>(y, b, geo, f0, partials, err);
+  p1d::p1f64_kernel<<<dim3(grid, b.n, nf), p1d::kThreads, sizeof(p1d::Smem), st>>>(y, b, geo, f0, partials, err);
 }
 
 }  // namespace hg
