@@ -798,6 +798,16 @@ p2tc_kernel(TcBatch tb, Geometry geo, P2Args args, const void* __restrict__ btu,
 #pragma unroll
           for (int k = 0; k < HLBL_QED_NW; ++k) q.w[e][k] = (float)wq[((size_t)vv * 3 + e) * HLBL_QED_NW + k];
       }
+      if (kGeneric && (P & 1) == 0) {
+        // the tile's coefficients of this row quadrant (20 KB) towards L2 while the
+        // accumulators fill: read from HBM they made the dot, which the next phase
+        // waits for, 4 % of the kernel longer
+        const float* c = static_cast<const float*>(args.coef) + (size_t)pi * args.coef_stride +
+                         coef32_index((long long)tile * kSites, quad, 0);
+#pragma unroll
+        for (int l = 0; l < kSites * kBtN / 32; l += 32)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(c + (l + lane) * 32));
+      }
       if (!wait_or_fail(&sm.acc_full, (uint32_t)(P & 1), fail)) break;
       tc_fence_after();
       uint32_t const c0 = (uint32_t)((P & 1) * kBtN), c1 = (uint32_t)(((P + 1) & 1) * kBtN);
