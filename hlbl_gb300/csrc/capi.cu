@@ -555,20 +555,27 @@ int run_pass2(hlbl_ctx* c, const Geometry& geo, const double* y, const PairBatch
               int f0, int nf, int precision, int add, const int* bad = nullptr,
               const double* g_dzu = nullptr, const double* g_dzsu = nullptr) {
   P2Args a{};
-  if (int rc = run_qed(c, geo, b, xunit, precision, a)) return rc;
+  bool const dig = precision == HLBL_FP64 && dig_ready(c, geo, b.n);
+  // (the digit products' kernels evaluate the exact weight themselves)
+  if (!(dig && c->qed_kind == kQedStandInClosed && c->qed_mode == HLBL_QED_EXACT))
+    if (int rc = run_qed(c, geo, b, xunit, precision, a)) return rc;
   a.xunit = xunit;
   a.f0 = f0;
   int grid;
   prof_begin(c, 1);
-  if (precision == HLBL_FP64 && dig_ready(c, geo, b.n)) {
+  if (dig) {
     for (int i = 0; i < b.n; ++i) {
       PairBatch one{};
       one.n = 1;
       one.p[0] = b.p[i];
+      WArgs wa{};
+      wa.batch = one;
+      wa.xunit = xunit;
+      wa.qp = c->qp;
       P2Args ai = a;
       if (ai.w) ai.w += (size_t)i * geo.V * 3 * HLBL_QED_NW;
       if (ai.coef) ai.coef = static_cast<const double*>(ai.coef) + (size_t)i * a.coef_stride;
-      p2dig_launch(nf, c->nsm, c->stream, y, one, geo, ai, g_dzu ? nullptr : c->d_dz + (size_t)i * nf * kDzLen, g_dzu, g_dzsu,
+      p2dig_launch(nf, c->nsm, c->stream, y, wa, c->qf, geo, ai, g_dzu ? nullptr : c->d_dz + (size_t)i * nf * kDzLen, g_dzu, g_dzsu,
                    c->d_dig, c->d_part2, c->d_err);
       p2_reduce_kernel<<<1, 64, 0, c->stream>>>(c->d_part2, c->nsm, nf, one, add);
     }

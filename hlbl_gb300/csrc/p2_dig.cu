@@ -170,21 +170,28 @@ bdig_build_kernel(const double* __restrict__ dz, const double* __restrict__ g_dz
 
 // ---- D's words -----------------------------------------------------------------
 constexpr int kTS = 4;                  // sites per CTA
-constexpr int kDThreads = 160;          // 144 threads (p, q) at work
+constexpr int kDThreads = 160;          // of a CTA of either role; here 144 threads (p, q) at work
 constexpr int kRowD = kTS * 24 + 2;     // staged row: 16 bytes of padding against bank conflicts
 
-// CTA: the sites s_begin + 4 blockIdx.x ... of the batch, flavour f0 + blockIdx.y
+// The sites s_begin + 4 block ... of the batch, flavour f0 + fl
 // (independent CTAs of 160 threads hide each other's copies and barriers: 188 -> 170 us
 // at 8,192 sites against 320 threads for both flavours). words[tile][fl][kTileWords],
 // esc[fl][site]: D (its rows scaled by rowexp) = integer 2^esc.
-__global__ void __launch_bounds__(kDThreads, 4)
-dform_kernel(const double* __restrict__ y, const double* __restrict__ src, Geometry geo, int f0, ll s_begin,
-             const int* __restrict__ rowexp, uint4* __restrict__ words, int* __restrict__ esc, int* __restrict__ err) {
-  __shared__ __align__(128) double stage[24][kRowD];
-  __shared__ __align__(8) uint64_t s_bar;
-  __shared__ int s_em[2][kTS];
-  __shared__ uint32_t s_or[2][5][2];
-  int const t = threadIdx.x, fl = blockIdx.y, nf = gridDim.y, l0 = kTS * blockIdx.x;
+struct __align__(128) DSmem {
+  double stage[24][kRowD];
+  uint64_t bar;
+  int em[2][kTS];
+  uint32_t top[2][5][2];
+};
+__device__ __forceinline__ void
+dform_cta(DSmem& sm, const double* __restrict__ y, const double* __restrict__ src, const Geometry& geo, int f0, int fl,
+          int nf, int block, ll s_begin, const int* __restrict__ rowexp, uint4* __restrict__ words, int* __restrict__ esc,
+          int* __restrict__ err) {
+  double (*const stage)[kRowD] = sm.stage;
+  uint64_t& s_bar = sm.bar;
+  int (*const s_em)[kTS] = sm.em;
+  uint32_t (*const s_or)[5][2] = sm.top;
+  int const t = threadIdx.x, l0 = kTS * block;
   ll const s0 = s_begin + l0;
   int const nvalid = (int)min((ll)kTS, geo.V - s0);
   if (t == 0) {
@@ -353,10 +360,10 @@ dform_kernel(const double* __restrict__ y, const double* __restrict__ src, Geome
 // same in all lanes and they are left out (1.6 FP64 instructions per entry instead
 // of five, on the pipe that bounds this), and E3(k, lam, nu, mu) of the six k serves
 // the ten columns j of (mu, nu, lam). 8,192 sites: 150 -> 118 us.
-constexpr int kCoefThreads = 256;
 struct CoefSmem {
   double tab[3][kQedTab][kSites];         // the tensor's factors per evaluation and site
   double zh[4][kSites];
+  double w[3][HLBL_QED_NW][kSites];       // the weight functions
 };
 // kerv[k][a][b][c] of the lane's site, (r, s) the k-th pair; qed_tab_value's factors
 __device__ __forceinline__ double entry_uniform(const double (*tab)[kSites], int k, int a, int b, int c, int lane) {
@@ -383,15 +390,31 @@ __device__ __forceinline__ double entry_uniform(const double (*tab)[kSites], int
   if (c == r) mad(tab[42 + s][lane], tab[46 + 4 * a + b][lane], true);
   return v;
 }
-__global__ void __launch_bounds__(kCoefThreads, 4)
-coef_closed_kernel(PairBatch batch, Geometry geo, double xu, const double* __restrict__ w, ll s_begin,
-                   double* __restrict__ coef) {
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  CoefSmem& sm = *reinterpret_cast<CoefSmem*>(smem_raw);
+__device__ __forceinline__ void coef_cta(CoefSmem& sm, const WArgs& wa, const QedF32& qf, const Geometry& geo,
+                                         const double* __restrict__ w, int block, ll s_begin, double* __restrict__ coef) {
+  constexpr int kWarps = kDThreads / 32;
   int const t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  double const xu = wa.xunit;
+  const PairBatch& batch = wa.batch;
   int const gsx[4] = {batch.p[0].gsx[0], batch.p[0].gsx[1], batch.p[0].gsx[2], batch.p[0].gsx[3]};
   int const yv[4] = {batch.p[0].yv[0], batch.p[0].yv[1], batch.p[0].yv[2], batch.p[0].yv[3]};
-  ll const site = min(s_begin + (ll)kSites * blockIdx.x + lane, geo.V - 1);
+  ll const site = min(s_begin + (ll)kSites * block + lane, geo.V - 1);
+  // e = 0: K(x, y), 1: K(y, x), 2: K(x, x - y)
+  if (warp < 3) {
+    double ww[HLBL_QED_NW];
+    if (w == nullptr) {
+      double a[4], b[4], X, c, Y;
+      qed_args(geo, gsx, yv, xu, site, warp, a, b);
+      hlbl_qed_invariants(a, b, &X, &c, &Y);
+      qed_weights_fp64(wa.qp, qf, X, c, Y, ww);
+    } else {
+#pragma unroll
+      for (int j = 0; j < HLBL_QED_NW; ++j) ww[j] = w[(size_t)(site * 3 + warp) * HLBL_QED_NW + j];
+    }
+#pragma unroll
+    for (int j = 0; j < HLBL_QED_NW; ++j) sm.w[warp][j][lane] = ww[j];
+  }
+  __syncthreads();
   {
     int rel[4];
     rel_coords_fast(geo, gsx, site, rel);
@@ -403,26 +426,25 @@ coef_closed_kernel(PairBatch batch, Geometry geo, double xu, const double* __res
       xy[r] = coord_map_diff(rel[r], yv[r], geo.global[r]) * xu;
       if (warp == 0) sm.zh[r][lane] = (double)coord_map_zerohalf(rel[r], geo.global[r]);
     }
-    // e = 0: K(x, y), 1: K(y, x), 2: K(x, x - y)
 #pragma unroll
     for (int e = 0; e < 3; ++e) {
       double wv[HLBL_QED_NW];
 #pragma unroll
-      for (int j = 0; j < HLBL_QED_NW; ++j) wv[j] = w[(size_t)(site * 3 + e) * HLBL_QED_NW + j];
+      for (int j = 0; j < HLBL_QED_NW; ++j) wv[j] = sm.w[e][j][lane];
       const double* A = e == 1 ? ym : xm;
       const double* B = e == 0 ? ym : (e == 1 ? xm : xy);
 #pragma unroll
       for (int i = 0; i < kQedTab; ++i)
-        if ((i & 7) == warp) sm.tab[e][i][lane] = qed_tab_value(i, A, B, wv);
+        if (i % kWarps == warp) sm.tab[e][i][lane] = qed_tab_value(i, A, B, wv);
     }
   }
   __syncthreads();
   double zh[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) zh[r] = sm.zh[r][lane];
-  double2* const out = reinterpret_cast<double2*>(coef) + (size_t)blockIdx.x * (kCoefPerSite / 2) * kSites + lane;
+  double2* const out = reinterpret_cast<double2*>(coef) + (size_t)block * (kCoefPerSite / 2) * kSites + lane;
 #pragma unroll 1
-  for (int task = warp; task < 32; task += kCoefThreads / 32) {
+  for (int task = warp; task < 32; task += kWarps) {
     int const mu = task >> 3, nu = (task >> 1) & 3, lam = 2 * (task & 1);
     double e3[2][6];
 #pragma unroll
@@ -450,6 +472,26 @@ coef_closed_kernel(PairBatch batch, Geometry geo, double xu, const double* __res
     }
   }
 }
+
+// One launch for both, so that the coefficients (FP64 pipe; first, as they take
+// longest) and D formation (integer pipe) share the SMs. ncoef: 0 where the caller
+// has coefficients; w: weights, or null to evaluate them here (exact mode). A
+// weights kernel and one kernel for each took 98 + 118 + 170 us per 8,192 sites,
+// this 282.
+__global__ void __launch_bounds__(kDThreads, 4)
+site_kernel(const double* __restrict__ y, WArgs wa, QedF32 qf, Geometry geo, int f0, int nf, ll s_begin, int ncoef,
+            const int* __restrict__ rowexp, const double* __restrict__ w, uint4* __restrict__ words, int* __restrict__ esc,
+            double* __restrict__ coef, int* __restrict__ err) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  if (blockIdx.x < ncoef) {
+    coef_cta(*reinterpret_cast<CoefSmem*>(smem_raw), wa, qf, geo, w, blockIdx.x, s_begin, coef);
+    return;
+  }
+  int const d = blockIdx.x - ncoef;
+  dform_cta(*reinterpret_cast<DSmem*>(smem_raw), y, wa.batch.p[0].src, geo, f0, d % nf, nf, d / nf, s_begin, rowexp, words,
+            esc, err);
+}
+constexpr size_t kSiteSmem = sizeof(CoefSmem) > sizeof(DSmem) ? sizeof(CoefSmem) : sizeof(DSmem);
 
 // ---- the products ------------------------------------------------------------------
 constexpr int kStages = 3;
@@ -769,7 +811,7 @@ static Ws ws_layout(ll V, int nsm) {
 }
 
 template <int NF>
-static void launch_t(int nsm, cudaStream_t st, const double* y, const PairBatch& b, const Geometry& geo,
+static void launch_t(int nsm, cudaStream_t st, const double* y, const WArgs& wa, const QedF32& qf, const Geometry& geo,
                      const P2Args& a, const double* dz, const double* g_dzu, const double* g_dzsu, void* ws,
                      double* partials, int* err) {
   Ws const l = ws_layout(geo.V, nsm);
@@ -785,13 +827,10 @@ static void launch_t(int nsm, cudaStream_t st, const double* y, const PairBatch&
   for (ll s0 = 0; s0 < geo.V; s0 += kMaxSites) {
     int const n = (int)std::min<ll>(kMaxSites, geo.V - s0), cta = (n + kTS - 1) / kTS;
     const double* cf = static_cast<const double*>(a.coef);
-    if (cf != nullptr) {
-      cf += (size_t)s0 * kCoefPerSite;
-    } else {
-      coef_closed_kernel<<<(n + kSites - 1) / kSites, kCoefThreads, sizeof(CoefSmem), st>>>(b, geo, a.xunit, a.w, s0, coef);
-      cf = coef;
-    }
-    dform_kernel<<<dim3(cta, NF), kDThreads, 0, st>>>(y, b.p[0].src, geo, a.f0, s0, rowexp, words, esc, err);
+    int const ncoef = cf != nullptr ? 0 : (n + kSites - 1) / kSites;
+    site_kernel<<<cta * NF + ncoef, kDThreads, ncoef > 0 ? kSiteSmem : sizeof(DSmem), st>>>(
+        y, wa, qf, geo, a.f0, NF, s0, ncoef, rowexp, a.w, words, esc, coef, err);
+    cf = cf != nullptr ? cf + (size_t)s0 * kCoefPerSite : coef;
     digit_mma_kernel<NF><<<nsm, kThreads, sizeof(Smem), st>>>(words, esc, p + l.bt, bem, corr, cf, a.coef == nullptr, n, s0 == 0,
                                                               s0 + n >= geo.V, reinterpret_cast<double*>(p + l.state),
                                                               partials, err);
@@ -801,7 +840,7 @@ static void launch_t(int nsm, cudaStream_t st, const double* y, const PairBatch&
 }  // namespace dig
 
 int p2dig_init() {
-  cudaError_t e = cudaFuncSetAttribute(dig::coef_closed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dig::CoefSmem));
+  cudaError_t e = cudaFuncSetAttribute(dig::site_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dig::kSiteSmem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(dig::digit_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dig::Smem));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(dig::digit_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(dig::Smem));
@@ -810,11 +849,11 @@ int p2dig_init() {
 
 size_t p2dig_ws_bytes(long long V, int nsm) { return dig::ws_layout(V, nsm).total; }
 
-void p2dig_launch(int nf, int nsm, cudaStream_t st, const double* y, const PairBatch& b, const Geometry& geo,
+void p2dig_launch(int nf, int nsm, cudaStream_t st, const double* y, const WArgs& wa, const QedF32& qf, const Geometry& geo,
                   const P2Args& a, const double* dz, const double* g_dzu, const double* g_dzsu, void* ws,
                   double* partials, int* err) {
-  if (nf == 2) dig::launch_t<2>(nsm, st, y, b, geo, a, dz, g_dzu, g_dzsu, ws, partials, err);
-  else dig::launch_t<1>(nsm, st, y, b, geo, a, dz, g_dzu, g_dzsu, ws, partials, err);
+  if (nf == 2) dig::launch_t<2>(nsm, st, y, wa, qf, geo, a, dz, g_dzu, g_dzsu, ws, partials, err);
+  else dig::launch_t<1>(nsm, st, y, wa, qf, geo, a, dz, g_dzu, g_dzsu, ws, partials, err);
 }
 
 }  // namespace hg
