@@ -356,39 +356,91 @@ dform_cta(DSmem& sm, const double* __restrict__ y, const double* __restrict__ sr
 
 // ---- the coefficients of the closed-form weight ------------------------------------
 // coef[tile][mu][n / 2][32 sites][2] of the batch's sites. A lane is a site and a warp
-// takes (mu, nu) and two lam at a time: which of an entry's terms vanish is then the
-// same in all lanes and they are left out (1.6 FP64 instructions per entry instead
-// of five, on the pipe that bounds this), and E3(k, lam, nu, mu) of the six k serves
-// the ten columns j of (mu, nu, lam). 8,192 sites: 150 -> 118 us.
+// takes (mu, nu) and two lam at a time: which of an entry's terms vanish is then known
+// at compile time, and E3(k, lam, nu, mu) of the six k serves the ten columns j of
+// (mu, nu, lam).
 struct CoefSmem {
   double tab[3][kQedTab][kSites];         // the tensor's factors per evaluation and site
   double zh[4][kSites];
   double w[3][HLBL_QED_NW][kSites];       // the weight functions
 };
-// kerv[k][a][b][c] of the lane's site, (r, s) the k-th pair; qed_tab_value's factors
-__device__ __forceinline__ double entry_uniform(const double (*tab)[kSites], int k, int a, int b, int c, int lane) {
-  int const r = comb_rho(k), s = comb_sigma(k);
+// kerv[K][A][B][C] of the lane's site, (R, S) the K-th pair; qed_tab_value's factors.
+// The indices are compile-time constants: an entry has 0 to 4 terms, and what it has
+// not costs no FP64 instruction (a vanishing term skipped at run time still did,
+// predicated: the coefficients took 6.4 k per site, with the weights' quadrature it is
+// 7.2 k now).
+constexpr bool pair_is(int x, int y, int K) {
+  int const r = comb_rho(K), s = comb_sigma(K);
+  return (x == r && y == s) || (x == s && y == r);
+}
+template <int K, int A, int B, int C>
+struct Entry {
+  static constexpr int R = comb_rho(K), S = comb_sigma(K);
+  static constexpr bool t0 = pair_is(A, B, K), t1 = pair_is(A, C, K), t2 = pair_is(B, C, K), f3 = A == B,
+                        f4 = A == R || A == S, f5 = C == R || C == S;
+  static constexpr bool none = !(t0 || t1 || t2 || f3 || f4 || f5);
+  static __device__ __forceinline__ double get(const double (*tab)[kSites], int lane) {
+    double v = 0.0;
+    if constexpr (t0) v = A == S ? -tab[C][lane] : tab[C][lane];
+    if constexpr (t1) {
+      double const x = A == S ? -tab[4 + B][lane] : tab[4 + B][lane];
+      v = t0 ? v + x : x;
+    }
+    if constexpr (t2) {
+      double const x = B == S ? -tab[8 + A][lane] : tab[8 + A][lane];
+      v = t0 || t1 ? v + x : x;
+    }
+    if constexpr (f3) {
+      double const x = tab[12 + K][lane], w = tab[18 + C][lane];
+      v = t0 || t1 || t2 ? fma(x, w, v) : x * w;
+    }
+    if constexpr (f4) {
+      double const x = A == S ? tab[22 + R][lane] : -tab[22 + S][lane], w = tab[26 + 4 * B + C][lane];
+      v = t0 || t1 || t2 || f3 ? fma(x, w, v) : x * w;
+    }
+    if constexpr (f5) {
+      double const x = C == S ? tab[42 + R][lane] : -tab[42 + S][lane], w = tab[46 + 4 * A + B][lane];
+      v = t0 || t1 || t2 || f3 || f4 ? fma(x, w, v) : x * w;
+    }
+    return v;
+  }
+};
+// The ten columns j of (MU, NU, LAM): c[0..5] = E1 + E2 - E3, c[6 + tau] = sum_k E3(k)
+// (zh_rho_k [sigma_k = tau] - zh_sigma_k [rho_k = tau])
+template <int K, int MU, int NU, int LAM>
+__device__ __forceinline__ void coef_k(const CoefSmem& sm, int lane, const double zh[4], double c[10]) {
+  using E1 = Entry<K, MU, NU, LAM>;
+  using E2 = Entry<K, NU, MU, LAM>;
+  using E3 = Entry<K, LAM, NU, MU>;
+  constexpr int R = comb_rho(K), S = comb_sigma(K);
   double v = 0.0;
-  bool any = false;
-  auto add = [&](double x, bool neg) {
-    x = flip_sign(x, neg ? 1u : 0u);
-    v = any ? v + x : x;
-    any = true;
-  };
-  auto mad = [&](double x, double w, bool neg) {
-    x = flip_sign(x, neg ? 1u : 0u);
-    v = any ? fma(x, w, v) : x * w;
-    any = true;
-  };
-  if ((a == r && b == s) || (a == s && b == r)) add(tab[c][lane], a == s);
-  if ((a == r && c == s) || (a == s && c == r)) add(tab[4 + b][lane], a == s);
-  if ((b == r && c == s) || (b == s && c == r)) add(tab[8 + a][lane], b == s);
-  if (a == b) mad(tab[12 + k][lane], tab[18 + c][lane], false);
-  if (a == s) mad(tab[22 + r][lane], tab[26 + 4 * b + c][lane], false);
-  if (a == r) mad(tab[22 + s][lane], tab[26 + 4 * b + c][lane], true);
-  if (c == s) mad(tab[42 + r][lane], tab[46 + 4 * a + b][lane], false);
-  if (c == r) mad(tab[42 + s][lane], tab[46 + 4 * a + b][lane], true);
-  return v;
+  if constexpr (!E1::none) v = E1::get(sm.tab[0], lane);
+  if constexpr (!E2::none) {
+    double const e = E2::get(sm.tab[1], lane);
+    v = E1::none ? e : v + e;
+  }
+  if constexpr (!E3::none) {
+    double const e = E3::get(sm.tab[2], lane);
+    v = E1::none && E2::none ? -e : v - e;
+    c[6 + S] = fma(zh[R], e, c[6 + S]);
+    c[6 + R] = fma(-zh[S], e, c[6 + R]);
+  }
+  c[K] = v;
+}
+template <int T>
+__device__ __forceinline__ void coef_task(const CoefSmem& sm, int lane, const double zh[4], double2* __restrict__ out) {
+  constexpr int MU = T >> 3, NU = (T >> 1) & 3, LAM = 2 * (T & 1);
+  double c[2][10];
+#pragma unroll
+  for (int l = 0; l < 2; ++l)
+#pragma unroll
+    for (int j = 6; j < 10; ++j) c[l][j] = 0.0;
+#define HG_COEF_K(K) coef_k<K, MU, NU, LAM>(sm, lane, zh, c[0]); coef_k<K, MU, NU, LAM + 1>(sm, lane, zh, c[1]);
+  HG_COEF_K(0) HG_COEF_K(1) HG_COEF_K(2) HG_COEF_K(3) HG_COEF_K(4) HG_COEF_K(5)
+#undef HG_COEF_K
+#pragma unroll
+  for (int j = 0; j < 10; ++j)
+    out[(size_t)(MU * (kBtN / 2) + 8 * j + 2 * NU + (LAM >> 1)) * kSites] = make_double2(c[0][j], c[1][j]);
 }
 __device__ __forceinline__ void coef_cta(CoefSmem& sm, const WArgs& wa, const QedF32& qf, const Geometry& geo,
                                          const double* __restrict__ w, int block, ll s_begin, double* __restrict__ coef) {
@@ -443,32 +495,16 @@ __device__ __forceinline__ void coef_cta(CoefSmem& sm, const WArgs& wa, const Qe
 #pragma unroll
   for (int r = 0; r < 4; ++r) zh[r] = sm.zh[r][lane];
   double2* const out = reinterpret_cast<double2*>(coef) + (size_t)block * (kCoefPerSite / 2) * kSites + lane;
+  if (warp == 4) return;  // four warps, one per scheduler
 #pragma unroll 1
-  for (int task = warp; task < 32; task += kWarps) {
-    int const mu = task >> 3, nu = (task >> 1) & 3, lam = 2 * (task & 1);
-    double e3[2][6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      double c[2];
-#pragma unroll
-      for (int l = 0; l < 2; ++l) {
-        e3[l][k] = entry_uniform(sm.tab[2], k, lam + l, nu, mu, lane);
-        c[l] = entry_uniform(sm.tab[0], k, mu, nu, lam + l, lane) + entry_uniform(sm.tab[1], k, nu, mu, lam + l, lane) - e3[l][k];
-      }
-      out[(size_t)(mu * (kBtN / 2) + 8 * k + 2 * nu + (lam >> 1)) * kSites] = make_double2(c[0], c[1]);
-    }
-    // sum_k E3[k][lam][nu][mu] (zh_rho_k [sigma_k = tau] - zh_sigma_k [rho_k = tau])
-#pragma unroll
-    for (int tau = 0; tau < 4; ++tau) {
-      double c[2] = {0.0, 0.0};
-#pragma unroll
-      for (int o = 0; o < 4; ++o) {
-        if (o == tau) continue;
-        int const r = o < tau ? o : tau, g = o < tau ? tau : o, k = r == 0 ? g - 1 : (r == 1 ? g + 1 : 5);
-#pragma unroll
-        for (int l = 0; l < 2; ++l) c[l] = fma(flip_sign(zh[o], tau < o ? 1u : 0u), e3[l][k], c[l]);
-      }
-      out[(size_t)(mu * (kBtN / 2) + 8 * (6 + tau) + 2 * nu + (lam >> 1)) * kSites] = make_double2(c[0], c[1]);
+  for (int task = warp; task < 32; task += 4) {
+    switch (task) {
+#define HG_COEF_T(T) case T: coef_task<T>(sm, lane, zh, out); break;
+#define HG_COEF_T4(T) HG_COEF_T(T) HG_COEF_T(T + 1) HG_COEF_T(T + 2) HG_COEF_T(T + 3)
+      HG_COEF_T4(0) HG_COEF_T4(4) HG_COEF_T4(8) HG_COEF_T4(12)
+      HG_COEF_T4(16) HG_COEF_T4(20) HG_COEF_T4(24) HG_COEF_T4(28)
+#undef HG_COEF_T4
+#undef HG_COEF_T
     }
   }
 }
@@ -477,7 +513,7 @@ __device__ __forceinline__ void coef_cta(CoefSmem& sm, const WArgs& wa, const Qe
 // longest) and D formation (integer pipe) share the SMs. ncoef: 0 where the caller
 // has coefficients; w: weights, or null to evaluate them here (exact mode). A
 // weights kernel and one kernel for each took 98 + 118 + 170 us per 8,192 sites,
-// this 282.
+// this 282, and 230 with the vanishing terms left out at compile time.
 __global__ void __launch_bounds__(kDThreads, 4)
 site_kernel(const double* __restrict__ y, WArgs wa, QedF32 qf, Geometry geo, int f0, int nf, ll s_begin, int ncoef,
             const int* __restrict__ rowexp, const double* __restrict__ w, uint4* __restrict__ words, int* __restrict__ esc,
