@@ -14,7 +14,8 @@
 // takes over at the end of the run: the ten results from S and T = sum zh_3 x
 // product = zh_3(first) S + (n S - W), those into the compensated sums every
 // kFlushTiles tiles. Measured (both flavours, one pair): with FP64 products 42 ms
-// at 663,552 sites and 0.54 ms at 8,192, so 16.7 and 0.25.
+// at 663,552 sites and 0.54 ms at 8,192, so 13.4 and 0.24 (with two stages and three
+// CTAs per SM 16.7 and 0.25: the CTAs hide each other's copies and barriers).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -33,30 +34,30 @@ constexpr int kRow = kTS * 24 + 2;     // staged row: 16 bytes of padding agains
 constexpr int kFlushTiles = 4;         // tiles per addition into the compensated sums
 constexpr int kThreads = 144;
 struct __align__(128) Smem {
-  double stage[2][24][kRow];           // rows [src | y][12]; a tile at work holds limbs (hi, lo) instead
+  double stage[24][kRow];           // rows [src | y][12]; a tile at work holds limbs (hi, lo) instead
   int zh[2][kTS][4];
   int em[24];                          // the rows' exponents (exp_of)
 };
 
-__global__ void __launch_bounds__(kThreads, 3)
+__global__ void __launch_bounds__(kThreads, 4)
 p1f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0, double* __restrict__ partials,
              int* __restrict__ err) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
-  __shared__ __align__(8) uint64_t s_bar[2];
+  __shared__ __align__(8) uint64_t s_bar;
   __shared__ int s_fail;
   int const t = threadIdx.x, pi = blockIdx.y, fl = blockIdx.z, nf = gridDim.z;
   const double* __restrict__ src = batch.p[pi].src;
   int const gsx[4] = {batch.p[pi].gsx[0], batch.p[pi].gsx[1], batch.p[pi].gsx[2], batch.p[pi].gsx[3]};
   int const ia = t / 12, ib = t % 12;
   // src flavour f0 + fl, y flavour 1 - (f0 + fl)
-  auto issue = [&](long long tile, int st) {
+  auto issue = [&](long long tile) {
     long long const s0 = tile * kTS;
     uint32_t const bytes = (uint32_t)min((long long)kTS, geo.V - s0) * 192u;
-    mbar_arrive_expect_tx(&s_bar[st], bytes * 24);
+    mbar_arrive_expect_tx(&s_bar, bytes * 24);
     for (int row = 0; row < 24; ++row) {
       int const i = row % 12, ff = row < 12 ? f0 + fl : 1 - f0 - fl;
-      bulk_g2s(sm.stage[st][row], (row < 12 ? src : y) + ((size_t)(ff * 12 + i) * geo.V + s0) * 24, bytes, &s_bar[st]);
+      bulk_g2s(sm.stage[row], (row < 12 ? src : y) + ((size_t)(ff * 12 + i) * geo.V + s0) * 24, bytes, &s_bar);
     }
   };
   auto zh_fill = [&](long long tile, int buf) {
@@ -68,8 +69,7 @@ p1f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0
     }
   };
   if (t == 0) {
-    mbar_init(&s_bar[0], 1);
-    mbar_init(&s_bar[1], 1);
+    mbar_init(&s_bar, 1);
     fence_mbar_init();
     s_fail = 0;
   }
@@ -102,7 +102,7 @@ p1f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0
   long long const ntiles = (geo.V + kTS - 1) / kTS;
   long long tile = blockIdx.x;
   if (tile < ntiles) {
-    if (t == 0) issue(tile, 0);
+    if (t == 0) issue(tile);
     zh_fill(tile, 0);
   }
   __syncthreads();
@@ -113,18 +113,13 @@ p1f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0
     long long const s0 = tile * kTS;
     int const nvalid = (int)min((long long)kTS, geo.V - s0);
     more = tile + gridDim.x < ntiles;
-    // the next tile into the other stage (its readers passed the last barrier)
-    if (t == 0 && more) {
-      fence_proxy_async_smem();
-      issue(tile + gridDim.x, st ^ 1);
-    }
-    if (!mbar_wait(&s_bar[st], (uint32_t)((it >> 1) & 1))) s_fail = 1;
+    if (!mbar_wait(&s_bar, (uint32_t)(it & 1))) s_fail = 1;
     __syncthreads();
     if (s_fail) break;
     {
       // the rows' exponents, then limbs in place: six threads per row
       int const row = t / 6, nval = nvalid * 24;
-      double* const p = sm.stage[st][row];
+      double* const p = sm.stage[row];
       int m = kZeroExp;
 #pragma unroll 8
       for (int i = t % 6; i < nval; i += 6) m = max(m, exp_of(p[i], 0));
@@ -140,8 +135,8 @@ p1f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0
     }
     __syncthreads();
     {
-      const double* A_base = sm.stage[st][ia];
-      const double* B_base = sm.stage[st][12 + ib];
+      const double* A_base = sm.stage[ia];
+      const double* B_base = sm.stage[12 + ib];
       const int (*zhs)[4] = sm.zh[st];
       // a product's unit 2^56 2^(em - 1077) 2^(em' - 1077)
       int const ea = sm.em[ia], eb = sm.em[12 + ib];
@@ -251,6 +246,11 @@ p1f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0
     }
     if (more) zh_fill(tile + gridDim.x, st ^ 1);
     __syncthreads();  // the stage, zh[st] and em are rewritten after this
+    // (one stage: the CTAs of an SM hide each other's copies)
+    if (t == 0 && more) {
+      fence_proxy_async_smem();
+      issue(tile + gridDim.x);
+    }
     if (t < 24) sm.em[t] = kZeroExp;
   }
   flush();
@@ -259,8 +259,7 @@ p1f64_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0
     // memory outlive it (bounded, as everything else)
     if (t == 0) {
       if (err) atomicExch(err, kErrWaitTimeout);
-      mbar_wait(&s_bar[it & 1], (uint32_t)((it >> 1) & 1));
-      if (more) mbar_wait(&s_bar[(it + 1) & 1], (uint32_t)(((it + 1) >> 1) & 1));
+      mbar_wait(&s_bar, (uint32_t)(it & 1));
     }
     return;
   }
