@@ -58,3 +58,56 @@ def test_zero_and_not_finite(value):
     else:
         y[7 * 24 + 5] = value  # flavour 0 of y: both passes of both flavours' sums read it
         assert not np.any(np.isfinite(run(lat, x, y, gsx, yv)))
+
+
+@pytest.mark.parametrize("lat", [(4, 4, 4, 7), (4, 8, 4, 4), (5, 7, 5, 3)])
+def test_several_pairs_in_a_batch(lat):
+    """448, 512 and 525 sites: both sides of the volume from which a batch of pairs
+    goes through digit products; repeated calls are bit-identical."""
+    import hlbl_gb300 as hg
+
+    n = 3
+    y, xs = S.gaussian_block(lat, 81), [S.random_block(lat, 82 + i) for i in range(n)]
+    gsxs, yvs = [(i, 1, 2, 0) for i in range(n)], [(1, i, -1, 2) for i in range(n)]
+    with hg.Contractor(lat) as c:
+        out = torch.zeros(2, n, 2, dtype=torch.float64, device="cuda")
+        d_y, d_xs = dev(y), [dev(x) for x in xs]
+        for rep in range(2):
+            c.kernel_sums_batched(d_y, d_xs, gsxs, yvs, 0.4, out[rep], hg.FP64)
+        torch.cuda.synchronize()
+        c.check()
+        out = out.cpu().numpy()
+    assert np.array_equal(out[0], out[1])
+    for i in range(n):
+        assert S.pair_rel_err(out[0, i], S.oracle_kernel_sum(xs[i], y, gsxs[i], yvs[i], 0.4, lat)) <= TOL64
+
+
+def test_capture_without_the_work_buffer():
+    """A capture on a context that has no work buffer yet takes the kernel that
+    needs none; afterwards the eager call and a new capture take digit products."""
+    import hlbl_gb300 as hg
+
+    lat, gsx, yv = (3, 4, 5, 6), (2, 1, 0, 3), (1, 2, -2, 1)
+    x, y = S.gaussian_block(lat, 91), S.gaussian_block(lat, 92)
+    want = S.oracle_kernel_sum(x, y, gsx, yv, 0.4, lat)
+    with hg.Contractor(lat) as c:
+        d_x, d_y = dev(x), dev(y)
+        out = torch.zeros(3, 2, dtype=torch.float64, device="cuda")
+        c.reserve(1)
+        graphs = []
+        for i in (0, 2):
+            c.graph_begin()
+            c.kernel_sum_async(d_x, d_y, gsx, yv, 0.4, out[i], hg.FP64)
+            graphs.append(c.graph_end())
+            if i == 0:
+                c.kernel_sum_async(d_x, d_y, gsx, yv, 0.4, out[1], hg.FP64)
+        for g in graphs:
+            g.launch()
+        torch.cuda.synchronize()
+        c.check()
+        got = out.cpu().numpy()
+        for g in graphs:
+            g.close()
+    for i in range(3):
+        assert S.pair_rel_err(got[i], want) <= TOL64
+    assert np.array_equal(got[1], got[2])
