@@ -386,11 +386,12 @@ int wait_staged(hlbl_ctx* c) {
 // work buffer exists or can be had (not during a capture; p2_f64.cu needs
 // none). p2_f64.cu takes all pairs of a batch in one launch, p2_dig.cu a handful
 // of launches for each pair: whole kernel sums with p2_f64.cu and p2_dig.cu, in us,
-//   128 sites: 399, 343 (one pair), 413, 748 (four); 256: 403, 347; 587, 750;
-//   512: 407, 351; 994, 830; 3320, 2893 (16 pairs); 2048: 997, 551; 3068, 1678.
-constexpr long long kDigMinSites = 128, kDigMinSitesBatch = 512;
+//   one pair:   4 sites 292, 199; 64: 327, 209; 128: 347, 210; 512: 354, 219; 2048: 964, 376
+//   four pairs: 128 sites 361, 748 (p2_dig.cu's first form); 512: 929, 756; 2048: 2929, 1263
+//   sixteen:    512 sites 2974, 2823; 1024: 5562, 3368
+constexpr long long kDigMinSitesBatch = 512;
 bool dig_ready(hlbl_ctx* c, const Geometry& geo, int npairs) {
-  if (geo.V < (npairs == 1 ? kDigMinSites : kDigMinSitesBatch)) return false;
+  if (npairs > 1 && geo.V < kDigMinSitesBatch) return false;
   size_t const need = p2dig_ws_bytes(geo.V, c->nsm);
   if (need <= c->dig_cap) return true;
   if (c->capturing) return false;

@@ -1,5 +1,6 @@
 // p2_f64.cu -- the FP64 pass 2 (ker_4pt_contraction, cuda_lattice.cu:277-484)
-// in the block-diagonal form of quat_basis.cuh.
+// in the block-diagonal form of quat_basis.cuh: for several pairs on lattices too
+// small for the digit products of p2_dig.cu, and where their work buffer cannot be had.
 //
 // What bounds it: the FP64 pipe (two lanes per SM and cycle here), so the
 // kernel is laid out for few FP64 instructions and nothing else. Per site and

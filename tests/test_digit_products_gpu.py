@@ -1,6 +1,6 @@
 """The FP64 pass 2 by digit products (p2_dig.cu) where it can go wrong: around
-the volume from which it is taken, ragged tiles of 32 and groups of 4 sites, more
-sites than a batch, one and two flavours, blocks of widely different scale (per
+the volume from which a batch of pairs takes it, ragged tiles of 32 and groups of 4
+sites, more sites than a batch, one and two flavours, blocks of widely different scale (per
 site, per row and per block), zero blocks and values that are not finite.
 Against the CPU oracle at the FP64 bar, 1e-12 of the pair's sum. Needs a GPU."""
 import numpy as np
@@ -111,3 +111,29 @@ def test_capture_without_the_work_buffer():
     for i in range(3):
         assert S.pair_rel_err(got[i], want) <= TOL64
     assert np.array_equal(got[1], got[2])
+
+
+def test_launcher_in_a_capture_without_the_work_buffer():
+    """There the launcher of pass 2 takes the kernels that need no buffer, also
+    with sums that are not the gamma images of one dz."""
+    import hlbl_gb300 as hg
+
+    lat, gsx, yv, f = (3, 4, 5, 6), (2, 1, 0, 3), (1, 2, -2, 1), 1
+    x, y = S.gaussian_block(lat, 93), S.gaussian_block(lat, 94)
+    rng = np.random.default_rng(9)
+    images = S.oracle_gammas(*S.oracle_dz(x, y, f, gsx, lat))
+    z = (0, 0, 0, 0)
+    for gu, gs in (images, (rng.normal(size=6912), rng.normal(size=4608))):
+        want = S.oracle_4pt(gu, gs, x, y, f, gsx, 0.4, yv, lat)
+        with hg.Contractor(lat) as c:
+            d_x, d_y, d_gu, d_gs = dev(x), dev(y), dev(gu), dev(gs)
+            ks = torch.zeros(1, dtype=torch.float64, device="cuda")
+            c.reserve(1)
+            c.graph_begin()
+            c.cu_4pt_contraction(ks, d_gu, d_gs, d_x, d_y, f, z, gsx, 0.4, yv, lat, lat)
+            g = c.graph_end()
+            g.launch()
+            torch.cuda.synchronize()
+            c.check()
+            g.close()
+        assert abs(float(ks[0]) - want) <= TOL64 * abs(want)

@@ -1,8 +1,8 @@
-"""The FP64 passes at the edges of their tiles (4 sites in pass 2, 8 in pass 1,
-runs along z that cross them, more tiles than thread blocks, the flush of the
-compensated sums), and the launcher of pass 2 on sums that are not the gamma
-images of one dz, which take the general kernel. Against the CPU oracle at the
-FP64 bar, 1e-12 of the pair's (flavour's) sum. Needs a GPU."""
+"""The FP64 passes at the edges of their tiles (8 sites in pass 1, 4 and 32 in
+pass 2, runs along z that cross them, more tiles than thread blocks, the flush of
+the compensated sums), and the launcher of pass 2 on sums that are not the gamma
+images of one dz. Against the CPU oracle at the FP64 bar, 1e-12 of the pair's
+(flavour's) sum. Needs a GPU."""
 import numpy as np
 import pytest
 
