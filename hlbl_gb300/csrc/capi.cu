@@ -282,6 +282,7 @@ struct hlbl_ctx {
   double* d_dzq = nullptr;    // FP64 pass 2: dz in block-diagonal form, [kMaxBatch][2][p2f64_dzq_len]
   void* d_dig = nullptr;      // FP64 pass 2: work buffer of p2_dig.cu
   size_t dig_cap = 0;         // its bytes
+  void* d_dig_first = nullptr;  // the smaller one before it, if any
   int* d_bad = nullptr;       // hlbl_cu_4pt_contraction: sums that are not the gamma images of one dz
   double* d_w = nullptr;      // QED weights [V][3][6]
   long long w_cap = 0;        // sites d_w holds
@@ -392,17 +393,20 @@ int wait_staged(hlbl_ctx* c) {
 constexpr long long kDigMinSitesBatch = 512;
 bool dig_ready(hlbl_ctx* c, const Geometry& geo, int npairs) {
   if (npairs > 1 && geo.V < kDigMinSitesBatch) return false;
-  size_t const need = p2dig_ws_bytes(geo.V, c->nsm);
-  if (need <= c->dig_cap) return true;
+  if (p2dig_ws_bytes(geo.V, c->nsm) <= c->dig_cap) return true;
   if (c->capturing) return false;
-  cudaStreamSynchronize(c->stream);
-  cudaFree(c->d_dig);
-  c->d_dig = nullptr;
-  c->dig_cap = 0;
-  if (cudaMalloc(&c->d_dig, need) != cudaSuccess) {
+  // The context's own geometry, or, where a launcher's is larger, the size that
+  // serves any: it grows at most once, and the first buffer stays, as a graph
+  // captured before may use it.
+  bool const any = c->d_dig != nullptr || geo.V > c->geo.V;
+  size_t const need = p2dig_ws_bytes(any ? 1LL << 40 : c->geo.V, c->nsm);
+  void* p = nullptr;
+  if (cudaMalloc(&p, need) != cudaSuccess) {
     cudaGetLastError();  // not an error of the call
     return false;
   }
+  c->d_dig_first = c->d_dig;
+  c->d_dig = p;
   c->dig_cap = need;
   return true;
 }
@@ -757,6 +761,7 @@ void hlbl_ctx_destroy(hlbl_ctx* c) {
   cudaFree(c->d_bt);
   cudaFree(c->d_dzq);
   cudaFree(c->d_dig);
+  cudaFree(c->d_dig_first);
   cudaFree(c->d_bad);
   cudaFree(c->d_btu);
   cudaFree(c->d_bscale);

@@ -137,3 +137,33 @@ def test_launcher_in_a_capture_without_the_work_buffer():
             c.check()
             g.close()
         assert abs(float(ks[0]) - want) <= TOL64 * abs(want)
+
+
+def test_graph_outlives_a_larger_launcher_geometry():
+    """A launcher on a larger lattice than the context's makes the work buffer grow;
+    a graph captured before keeps its own and gives the same sums."""
+    import hlbl_gb300 as hg
+
+    lat, gsx, yv = (3, 4, 5, 6), (2, 1, 0, 3), (1, 2, -2, 1)
+    big, f, z = (7, 9, 8, 5), 0, (0, 0, 0, 0)
+    x, y = S.gaussian_block(lat, 95), S.gaussian_block(lat, 96)
+    bx, by = S.gaussian_block(big, 97), S.gaussian_block(big, 98)
+    gu, gs = S.oracle_gammas(*S.oracle_dz(bx, by, f, gsx, big))
+    with hg.Contractor(lat) as c:
+        d_x, d_y, d_bx, d_by, d_gu, d_gs = (dev(a) for a in (x, y, bx, by, gu, gs))
+        out = torch.zeros(2, 2, dtype=torch.float64, device="cuda")
+        ks = torch.zeros(1, dtype=torch.float64, device="cuda")
+        c.kernel_sum_async(d_x, d_y, gsx, yv, 0.4, out[0], hg.FP64)
+        c.graph_begin()
+        c.kernel_sum_async(d_x, d_y, gsx, yv, 0.4, out[1], hg.FP64)
+        g = c.graph_end()
+        c.cu_4pt_contraction(ks, d_gu, d_gs, d_bx, d_by, f, z, gsx, 0.4, yv, big, big)
+        g.launch()
+        torch.cuda.synchronize()
+        c.check()
+        got, launched = out.cpu().numpy(), float(ks[0])
+        g.close()
+    assert np.array_equal(got[0], got[1])
+    assert S.pair_rel_err(got[0], S.oracle_kernel_sum(x, y, gsx, yv, 0.4, lat)) <= TOL64
+    want = S.oracle_4pt(gu, gs, bx, by, f, gsx, 0.4, yv, big)
+    assert abs(launched - want) <= TOL64 * abs(want)
