@@ -12,6 +12,7 @@
 
 #include <type_traits>
 
+#include "fixed_point.cuh"
 #include "hlbl_device.cuh"
 #include "qed_f32.cuh"
 
@@ -282,13 +283,15 @@ p1_kernel(const double* __restrict__ y, PairBatch batch, Geometry geo, int f0,
   }
 }
 
-// Fixed-order, compensated (Neumaier) FP64 sum over the CTAs' partials.
+// FP64 sum over the CTAs' partials, exact in 128-bit integers of the exponent of the
+// output's largest partial (113 bits below it), rounded once at the end.
 // dz[fl][i] = sum_cta partials[cta][fl][i]; if add_to != null also
 // add_to[fl][i] += dz (the reference's accumulate-into-caller semantics).
-// A CTA takes 16 outputs (180 CTAs per flavour and pair, so that they spread
-// evenly over the SMs: the kernel is bound by the FP64 pipe, 5760 compensated
-// additions per partial); its 16 half warps each sum every 16th CTA's partials
-// (four loads in flight), then a tree adds the 16 sums.
+// A CTA takes 16 outputs; its 16 half warps each take every 16th CTA's partials (four
+// loads in flight), first their exponents, then their sum, and a tree adds the 16 sums.
+// On the integer pipe, as the compensated FP64 additions before it (four on the slow
+// pipe per partial) took 26 us for 57 partials of four pairs and 31 us for 304 of one
+// FP64 pair, and this 12 and 14. At most 2^13 partials (grids are below 2^11).
 constexpr int kRedOut = 16, kRedGrp = 16;
 static __global__ void __launch_bounds__(kRedOut * kRedGrp)
     p1_reduce_kernel(const double* __restrict__ partials, int ncta, int nf, double* __restrict__ dz,
@@ -296,36 +299,54 @@ static __global__ void __launch_bounds__(kRedOut * kRedGrp)
   int const fl = blockIdx.y, pi = blockIdx.z;
   int const o = threadIdx.x % kRedOut, grp = threadIdx.x / kRedOut;
   int const i = blockIdx.x * kRedOut + o;
-  __shared__ double rs[kRedGrp][kRedOut], rc[kRedGrp][kRedOut];
-  partials += (size_t)pi * ncta * nf * kDzLen;
-  Neu a;
-  if (i < kDzLen && fl < nf) {
-    const double* p = partials + (size_t)fl * kDzLen + i;
-    size_t const step = (size_t)nf * kDzLen;
-    int b = grp;
-    for (; b + 3 * kRedGrp < ncta; b += 4 * kRedGrp) {
-      double v[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = p[(size_t)(b + u * kRedGrp) * step];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) a.add(v[u]);
+  __shared__ unsigned long long rs[kRedGrp][kRedOut][2];
+  __shared__ int s_em[kRedOut];
+  bool const mine = i < kDzLen && fl < nf;
+  size_t const step = (size_t)nf * kDzLen;
+  const double* p = partials + (size_t)pi * ncta * step + (size_t)fl * kDzLen + i;
+  if (grp == 0) s_em[o] = kZeroExp;
+  __syncthreads();
+  int m = kZeroExp;
+  if (mine) {
+#pragma unroll 4
+    for (int b = grp; b < ncta; b += kRedGrp) m = max(m, exp_of(p[(size_t)b * step], 0));
+  }
+  atomicMax(&s_em[o], m);
+  __syncthreads();
+  m = s_em[o];
+  __int128 acc = 0;  // units of 2^(m - 1075 - 60); a partial is below 2^113 of them
+  if (mine) {
+#pragma unroll 4
+    for (int b = grp; b < ncta; b += kRedGrp) {
+      unsigned long long const v = (unsigned long long)__double_as_longlong(p[(size_t)b * step]);
+      int const f = (int)((v >> 52) & 0x7FFu);
+      unsigned long long const q = (v & 0xFFFFFFFFFFFFFull) | (f ? 1ull << 52 : 0ull);
+      int const sh = 60 - (m - (f ? f : 1));
+      unsigned long long lo, hi = 0;
+      if (sh >= 0) {
+        lo = q << sh;
+        hi = sh ? q >> (64 - sh) : 0;
+      } else {
+        lo = sh > -64 ? q >> -sh : 0;
+      }
+      __int128 const x = (__int128)(((unsigned __int128)hi << 64) | lo);
+      acc += v >> 63 ? -x : x;
     }
-    for (; b < ncta; b += kRedGrp) a.add(p[(size_t)b * step]);
   }
 #pragma unroll
   for (int h = kRedGrp / 2; h > 0; h >>= 1) {
     if (grp >= h && grp < 2 * h) {
-      rs[grp][o] = a.s;
-      rc[grp][o] = a.c;
+      rs[grp][o][0] = (unsigned long long)acc;
+      rs[grp][o][1] = (unsigned long long)((unsigned __int128)acc >> 64);
     }
     __syncthreads();
-    if (grp < h) {
-      a.add(rs[grp + h][o]);
-      a.c += rc[grp + h][o];
-    }
+    if (grp < h) acc += (__int128)(((unsigned __int128)rs[grp + h][o][1] << 64) | rs[grp + h][o][0]);
   }
-  if (grp != 0 || i >= kDzLen || fl >= nf) return;
-  double const s = a.get();
+  if (grp != 0 || !mine) return;
+  // (an infinite or NaN partial: NaN)
+  double const s = m == kNoScale ? __longlong_as_double(0x7FF8000000000000ll)
+                                 : ldexp(fma((double)(long long)(acc >> 64), 18446744073709551616.0,
+                                             (double)(unsigned long long)acc), m - 1075 - 60);
   dz += (size_t)pi * nf * kDzLen;
   dz[fl * kDzLen + i] = s;
   if (add_dzu != nullptr) {
